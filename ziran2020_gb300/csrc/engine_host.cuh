@@ -231,7 +231,7 @@ public:
             dev_bytes_ -= (int64_t)max_add;
         }
         // keys, and a first binning pass that sizes the grid (every group activates at most 8 blocks)
-        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_);
+        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
         ZR_CUDA(sort_keys((int64_t)N_));
         ZR_CUDA(group_heads((int64_t)N_));
         DevStatus hs;
@@ -326,7 +326,7 @@ public:
             ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
             if (cg_) ZR_CUDA(cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_));
             ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
-            k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_);
+            k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
             ZR_CUDA(cudaStreamSynchronize(stream_));
             const uint32_t f = hst_->flags;
             if ((f & FLAG_SORT) && !(f & (FLAG_CFL | FLAG_NONFINITE | FLAG_OUT_OF_DOMAIN | FLAG_TIMEOUT | FLAG_CHECK | FLAG_CAPACITY))) {
@@ -562,7 +562,7 @@ public:
             if ((e = cudaStreamWaitEvent(stream_, io_ev_[b], 0)) != cudaSuccess) break;
             if ((rc = fill_inv(s)) || (rc = launch_rows<ROWS_IMPORT>(s, rf, io_in_[b], nullptr, f32))) break;
             if ((e = cudaEventRecord(io_ev_[2 + b], stream_)) != cudaSuccess) break;
-            k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_); // raises FLAG_OUT_OF_DOMAIN
+            k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr); // raises FLAG_OUT_OF_DOMAIN
             forget_drive(s);
             if ((rc = refresh_drive())) break;
             if (i + 2 < nsteps && (e = issue_in(i + 2)) != cudaSuccess) break;
@@ -1225,12 +1225,18 @@ private:
     int rekey()
     {
         sorted_storage_ = false; // new positions: the storage order may no longer follow the cells
-        // the sort base (keys_sorted_) stays a sorted array of the same keys' layout, which is all the incremental
-        // sort needs to be correct: particles whose key matches it at their slot form a sorted subsequence
+        // The sort base (keys_sorted_) stays a sorted array of the same keys' layout, which is all the incremental sort
+        // needs to be correct: particles whose key matches it at their slot form a sorted subsequence. When more
+        // particles left their slot's key than the mover list holds, the next substep sorts in full: found out in that
+        // substep instead, the overflow aborts it, the launches already queued behind it run empty, and the list is grown
+        // for one substep and shrunk after the run, with the graphs captured again both times (a 50-substep job on 32,768
+        // particles: 4.9 ms so, 4.0 ms on the device; 426k particles, 20 substeps: 3.9 ms against 3.0 ms).
+        const bool based = inc_sort_usable() && !sort_base_stale_;
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
-        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_);
+        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, based ? (const uint32_t*)keys_sorted_ : nullptr);
         ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
+        if (based && (int64_t)hst_->max_movers > mcap_) sort_base_stale_ = true;
         if (hst_->flags & FLAG_OUT_OF_DOMAIN) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
         return 0;
     }
@@ -1657,7 +1663,7 @@ private:
             if (cg_) ZR_CUDA(cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_));
         }
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
-        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_);
+        k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
         return 0;

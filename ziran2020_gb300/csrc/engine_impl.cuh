@@ -156,12 +156,15 @@ __device__ inline bool aborted_cta(const DevStatus* st)
 
 // ---------------------------------------------------------------------------------------------------
 // keys of the current particle positions (used after a load or a host upload; afterwards G2P writes
-// the keys of the next substep). Also checks that every base node lies in its scene's domain.
+// the keys of the next substep). Also checks that every base node lies in its scene's domain. With a sort base (the
+// 32-bit keys the storage order was sorted by) the particles whose key differs from it are counted into max_movers.
 // ---------------------------------------------------------------------------------------------------
 template <class T>
-__global__ void k_keys(Pool<T> p, const SceneParams<T>* scenes, int n_scenes, uint64_t* keys, uint32_t n_total, KeyLayout kl, DevStatus* st)
+__global__ void k_keys(Pool<T> p, const SceneParams<T>* scenes, int n_scenes, uint64_t* keys, uint32_t n_total, KeyLayout kl, DevStatus* st,
+    const uint32_t* base)
 {
     using L = typename LayoutOf<T>::type;
+    uint32_t movers = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_total; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = n_scenes - 1; // scene owning storage slot i
         while (lo < hi) {
@@ -181,8 +184,13 @@ __global__ void k_keys(Pool<T> p, const SceneParams<T>* scenes, int n_scenes, ui
             raise_flag(st, FLAG_OUT_OF_DOMAIN);
             b[0] = b[1] = b[2] = 0;
         }
-        kl.put(keys, i, ((uint64_t)lo << (kl.cp + kl.ib)) | ((L::offset(b[0], b[1], b[2]) >> L::data_bits) << kl.ib));
+        const uint64_t k = ((uint64_t)lo << (kl.cp + kl.ib)) | ((L::offset(b[0], b[1], b[2]) >> L::data_bits) << kl.ib);
+        kl.put(keys, i, k);
+        if (base) movers += (uint32_t)k != base[i] ? 1u : 0u;
     }
+    if (!base) return;
+    for (int o = 16; o > 0; o >>= 1) movers += __shfl_down_sync(0xffffffffu, movers, o);
+    if ((threadIdx.x & 31) == 0 && movers) atomicAdd(&st->max_movers, movers);
 }
 
 // The hot-path keys hold (scene, page, cell) only, so the radix sort needs 4 passes instead of 7; a
