@@ -139,7 +139,7 @@ public:
             }
             ZR_CUDA(cudaStreamSynchronize(stream_));
             void* olds[] = { pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, sort_tmp_, pay_,
-                sort_aux_, inc_move_, inc_bkey_, inc_bidx_ };
+                sort_aux_, inc_bkey_, inc_bidx_ };
             for (void* p : olds)
                 if (p) cudaFree(p);
             pool_[0] = grown_pool[0];
@@ -149,16 +149,15 @@ public:
             cap_ = (uint64_t)cap;
             pay_ = nullptr;
             sort_aux_ = nullptr;
-            inc_move_ = inc_bkey_ = inc_bidx_ = nullptr;
+            inc_bkey_ = inc_bidx_ = nullptr;
             // P2G payload: NPAY fields of sorted particles at q + q/8, plus the copy granularity at the end
             pstride_ = (int64_t)((pay_pos((uint64_t)cap) + 64 + 63) & ~(uint64_t)63);
             if (alloc((void**)&keys_in_, 8 * cap) || alloc((void**)&keys_sorted_, 8 * cap) || alloc((void**)&iota_, 4 * cap)
                 || alloc((void**)&vals_sorted_, 4 * cap) || alloc((void**)&g_start_, 4 * cap) || alloc((void**)&pay_, sizeof(T) * NPAY * (size_t)pstride_)
-                || alloc((void**)&sort_aux_, sort_aux_bytes(cap)) || alloc((void**)&inc_move_, 4 * cap)
-                || alloc((void**)&inc_bkey_, 4 * bucket_slots(cap)) || alloc((void**)&inc_bidx_, 4 * bucket_slots(cap)))
+                || alloc((void**)&sort_aux_, sort_aux_bytes(cap)) || alloc((void**)&inc_bkey_, 4 * bucket_slots(cap)) || alloc((void**)&inc_bidx_, 4 * bucket_slots(cap)))
                 return ZR_ERR_CUDA_;
-            mcap_ = std::min<int64_t>(cap, std::max<int64_t>(MCAP_MIN, cap / 32));
             ZR_CUDA(cudaMemsetAsync(pay_, 0, sizeof(T) * NPAY * (size_t)pstride_, stream_));
+            ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes(cap), stream_));
             k_iota<T><<<nsm_ * 4, 256, 0, stream_>>>(iota_, (uint32_t)cap);
             size_t sb = 0, sb32 = 0;
             ZR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sb, keys_in_, keys_sorted_, iota_, vals_sorted_, cap, 0, 64, stream_));
@@ -245,8 +244,7 @@ public:
             if (rc) return rc;
         }
         else {
-            ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_));
-            ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
+            ZR_CUDA(clean_substep());
             int rc = ensure_cg();
             if (rc) return rc;
         }
@@ -307,13 +305,6 @@ public:
                 done += todo;
                 sorted_storage_ = true;
                 sort_base_stale_ = false;
-                // the mover buffer follows the movers seen: shrink to 3x the most seen when it is 8x too large
-                // (graphs are re-captured); a substep with more movers than it holds is repeated after growing it
-                const int64_t mm = (int64_t)hst_->max_movers;
-                if (inc_sort_usable() && todo >= 8 && mm > 0 && 8 * mm < mcap_ && mcap_ > MCAP_MIN) {
-                    mcap_ = std::min<int64_t>((int64_t)cap_, std::max<int64_t>(MCAP_MIN, 3 * mm));
-                    drop_graphs();
-                }
                 break;
             }
             sort_base_stale_ = true; // the aborted substep's sort overwrote the base
@@ -322,21 +313,14 @@ public:
             cur_ = (cur0 + k) & 1;
             if (k > 0) sorted_storage_ = true;
             // the aborted substep may have left partial grid sums, hash entries or next keys behind
-            ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_));
-            ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
-            if (cg_) ZR_CUDA(cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_));
+            ZR_CUDA(clean_substep());
             ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
             k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
             ZR_CUDA(cudaStreamSynchronize(stream_));
             const uint32_t f = hst_->flags;
             if ((f & FLAG_SORT) && !(f & (FLAG_CFL | FLAG_NONFINITE | FLAG_OUT_OF_DOMAIN | FLAG_TIMEOUT | FLAG_CHECK | FLAG_CAPACITY))) {
-                // more movers than the list holds (grow it), or a bucket beyond the merge's shared memory: the
-                // substep is repeated with a full sort (it cannot raise FLAG_SORT, so every retry makes progress)
-                const int64_t mm = (int64_t)hst_->max_movers;
-                if (mm > mcap_ && mcap_ < (int64_t)cap_) {
-                    mcap_ = std::min<int64_t>((int64_t)cap_, std::max<int64_t>(2 * mcap_, mm + mm / 2));
-                    drop_graphs();
-                }
+                // a bucket beyond the merge's shared memory: the substep is repeated with a full sort (it cannot raise
+                // FLAG_SORT, so every retry makes progress)
                 continue;
             }
             if ((f & FLAG_CAPACITY) && !(f & (FLAG_CFL | FLAG_NONFINITE | FLAG_OUT_OF_DOMAIN | FLAG_TIMEOUT | FLAG_CHECK)) && grow_rounds < 6) {
@@ -589,9 +573,7 @@ public:
         cur_ = (cur1 + k - 1) & 1;
         sort_base_stale_ = true;
         sorted_storage_ = false;
-        ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_));
-        ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
-        if (cg_) ZR_CUDA(cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_));
+        ZR_CUDA(clean_substep());
         ZR_CUDA(cudaStreamSynchronize(stream_));
         stream_reruns_ += nsteps - k;
         for (int i = k; i < nsteps; i++)
@@ -715,8 +697,7 @@ public:
         ZR_CUDA(cudaMemcpyAsync(d_scenes_, ck_scenes_, sc_b, cudaMemcpyDeviceToDevice, stream_));
         h_scenes_ = ck_host_scenes_;
         // a clean grid and the keys of the restored positions
-        ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_));
-        ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
+        ZR_CUDA(clean_substep());
         return rekey();
     }
 
@@ -849,6 +830,7 @@ private:
     uint64_t *keys_in_ = nullptr, *keys_sorted_ = nullptr;
     uint32_t *iota_ = nullptr, *vals_sorted_ = nullptr, *g_start_ = nullptr;
     int32_t* g_nbr_ = nullptr;
+    uint32_t *g_stop_ = nullptr, *g_end_ = nullptr;
     uint64_t* b_key_ = nullptr;
     T *acc_ = nullptr, *vel_ = nullptr;
     uint64_t* h_keys_ = nullptr;
@@ -893,12 +875,10 @@ private:
     bool sort_base_stale_ = true;
     bool inc_sort_on_ = true; // ZR_SORT=full turns the incremental sort off
     bool prefetch_ = true; // P2G's L2 prefetch of the groups ahead (ZR_PREFETCH=0 turns it off)
-    static constexpr int64_t MCAP_MIN = 4096;
-    // the sort's tile arrays (stayer bits, per-tile counts and keys, bucket counts, group-head look-back words);
-    // the movers' list, buckets and tickets, and their keys and storage indices grouped by bucket
+    // the sort's tile arrays (stayer bits, per-tile counts and keys, bucket counts, group-head look-back words), and
+    // the movers' keys and storage indices by bucket (fixed slots)
     unsigned char* sort_aux_ = nullptr;
-    uint32_t *inc_move_ = nullptr, *inc_bkey_ = nullptr, *inc_bidx_ = nullptr; // mover list; movers by bucket (fixed slots)
-    int64_t mcap_ = 0; // movers the incremental sort takes per substep
+    uint32_t *inc_bkey_ = nullptr, *inc_bidx_ = nullptr;
     void *ck_pool_ = nullptr, *ck_pid_ = nullptr, *ck_scenes_ = nullptr; // device checkpoint
     uint64_t ck_cap_ = 0;
     size_t ck_scenes_n_ = 0;
@@ -930,51 +910,39 @@ private:
     static int64_t sort_tiles(int64_t n) { return std::max<int64_t>(1, (n + SORT_TILE - 1) / SORT_TILE); }
     // movers' fixed bucket slots: SORT_MAXM per tile
     static int64_t bucket_slots(int64_t cap) { return sort_tiles(cap) * SORT_MAXM; }
-    // sort_aux_: [zeroed every substep: movers found (i64), unused (3 x i64), b_cnt, b_max (tiles u32 each)]
-    // [stay bits: ceil(cap/32) u32][t_stay, t_first, t_last, t_base, t_heads: tiles u32 each][look-back: tiles + 1 u64]
-    static size_t sort_zero_bytes(int64_t cap) { return 32 + 8 * (size_t)sort_tiles(cap); }
-    static size_t sort_aux_words(int64_t cap) { return sort_zero_bytes(cap) / 4 + (size_t)((cap + 31) / 32) + 5 * (size_t)sort_tiles(cap) + 1; }
+    // sort_aux_: [zero at the start of a substep: b_cnt, b_max (tiles u32 each)]
+    // [stay bits: ceil(cap/32) u32][t_first, t_stay, t_last: tiles u32 each][look-back: tiles + 1 u64]
+    static size_t sort_zero_bytes(int64_t cap) { return 8 * (size_t)sort_tiles(cap); }
+    static size_t sort_aux_words(int64_t cap) { return sort_zero_bytes(cap) / 4 + (size_t)((cap + 31) / 32) + 3 * (size_t)sort_tiles(cap) + 1; }
     static size_t sort_aux_bytes(int64_t cap) { return 4 * sort_aux_words(cap) + 8 * ((size_t)sort_tiles(cap) + 2); }
     uint64_t* lookback_words() const
     {
         const size_t off = (4 * sort_aux_words((int64_t)cap_) + 7) & ~(size_t)7;
         return reinterpret_cast<uint64_t*>(sort_aux_ + off);
     }
-    bool inc_sort_usable() const { return inc_sort_on_ && !kl_.wide && kl_.total() <= 31 && inc_move_; }
+    uint32_t* tile_first() const { return reinterpret_cast<uint32_t*>(sort_aux_) + sort_zero_bytes((int64_t)cap_) / 4 + (cap_ + 31) / 32; }
+    bool inc_sort_usable() const { return inc_sort_on_ && !kl_.wide && kl_.total() <= 31; }
 
-    // The sorted keys and storage indices of keys_in_ from the previous substep's sorted keys (keys_sorted_), by
-    // the hand-written kernels of the incremental sort (stayers in place, movers bucketed by stayer tile and merged),
-    // then the group heads placed and their blocks activated (k_heads_activate).
-    // ev_sorted (may be null) is recorded between the merge and the head placement.
-    cudaError_t sort_and_activate_incremental(int64_t n, const StepArgs<T>& a, cudaEvent_t ev_sorted)
+    // The sorted keys and storage indices of keys_in_ from the previous substep's sorted keys (keys_sorted_), the groups
+    // and their blocks, by the hand-written kernels of the incremental sort (stayers in place, movers bucketed by stayer
+    // tile and merged).
+    cudaError_t bin_incremental(int64_t n, const StepArgs<T>& a)
     {
-        const uint32_t* nk = (const uint32_t*)keys_in_;
-        const uint32_t* ok = (const uint32_t*)keys_sorted_;
         SortBufs sb;
         const int64_t tiles = sort_tiles(n), tcap = sort_tiles((int64_t)cap_);
-        sb.cnt = reinterpret_cast<int64_t*>(sort_aux_);
-        sb.b_cnt = reinterpret_cast<uint32_t*>(sort_aux_ + 32);
+        sb.b_cnt = reinterpret_cast<uint32_t*>(sort_aux_);
         sb.b_max = sb.b_cnt + tcap;
         sb.stay_bits = sb.b_max + tcap;
-        sb.t_stay = sb.stay_bits + (cap_ + 31) / 32;
-        sb.t_first = sb.t_stay + tcap;
-        sb.t_last = sb.t_first + tcap;
-        sb.t_base = sb.t_last + tcap;
-        sb.t_heads = sb.t_base + tcap;
-        sb.m_idx = inc_move_;
+        sb.t_first = tile_first();
+        sb.t_stay = sb.t_first + tcap;
+        sb.t_last = sb.t_stay + tcap;
         sb.b_key = inc_bkey_;
         sb.b_idx = inc_bidx_;
-        sb.mcap = mcap_;
         sb.n = n;
         sb.tiles = (int)tiles;
-        cudaError_t e = cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_);
-        if (e != cudaSuccess) return e;
-        const int mgrid = (int)std::max<int64_t>(1, std::min<int64_t>(nsm_ * 4, (mcap_ + SORT_NT - 1) / SORT_NT));
-        k_sort_tiles<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, ok, sb, st_);
-        k_sort_bucket<<<mgrid, SORT_NT, 0, stream_>>>(nk, sb, st_);
-        k_sort_merge<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, sb, (uint32_t*)keys_sorted_, vals_sorted_, kl_, st_);
-        if (ev_sorted && (e = cudaEventRecord(ev_sorted, stream_)) != cudaSuccess) return e;
-        k_heads_activate<T><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(a, sb, g_start_, (uint32_t)cap_);
+        const uint32_t* nk = (const uint32_t*)keys_in_;
+        k_sort_tiles<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, (const uint32_t*)keys_sorted_, sb, st_);
+        k_sort_merge<T><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(a, nk, sb, (uint32_t*)keys_sorted_, vals_sorted_);
         return cudaGetLastError();
     }
 
@@ -986,7 +954,7 @@ private:
         cudaError_t e = cudaMemsetAsync(lb, 0, 8 * ((size_t)tiles + 1), stream_);
         if (e != cudaSuccess) return e;
         k_group_heads<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(keys_sorted_, n, kl_, lb, reinterpret_cast<uint32_t*>(lb + tiles), g_start_,
-            (uint32_t)cap_, st_);
+            (uint32_t)cap_, tile_first(), st_);
         return cudaGetLastError();
     }
 
@@ -1192,9 +1160,14 @@ private:
         dfree(p);
         p = h_vals_;
         dfree(p);
+        p = g_stop_;
+        dfree(p);
+        p = g_end_;
+        dfree(p);
         p = cg_;
         dfree(p);
         cg_ = nullptr;
+        g_stop_ = g_end_ = nullptr;
         g_nbr_ = nullptr;
         b_key_ = nullptr;
         acc_ = vel_ = nullptr;
@@ -1205,12 +1178,24 @@ private:
         while (hs < 4 * cap) hs <<= 1;
         h_mask_ = hs - 1;
         if (alloc((void**)&g_nbr_, 32 * (size_t)cap) || alloc((void**)&b_key_, 8 * (size_t)cap) || alloc((void**)&acc_, sizeof(T) * (size_t)cap * NACC * L::nodes)
-            || alloc((void**)&vel_, sizeof(T) * (size_t)cap * NVEL * L::nodes) || alloc((void**)&h_keys_, 8 * (size_t)hs) || alloc((void**)&h_vals_, 4 * (size_t)hs))
+            || alloc((void**)&vel_, sizeof(T) * (size_t)cap * NVEL * L::nodes) || alloc((void**)&h_keys_, 8 * (size_t)hs) || alloc((void**)&h_vals_, 4 * (size_t)hs)
+            || alloc((void**)&g_stop_, 4 * (size_t)cap) || alloc((void**)&g_end_, 4 * (size_t)hs))
             return ZR_ERR_CUDA_;
         ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)cap * NACC * L::nodes, stream_));
         ZR_CUDA(cudaMemsetAsync(vel_, 0, sizeof(T) * (size_t)cap * NVEL * L::nodes, stream_));
         ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)hs, stream_));
         return ensure_cg();
+    }
+
+    // what a substep finds zero or empty and an aborted one may leave otherwise: the grid sums, the block hash, the
+    // damage solve's vectors and the sort's counters
+    cudaError_t clean_substep()
+    {
+        cudaError_t e = cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_);
+        if (e == cudaSuccess) e = cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_);
+        if (e == cudaSuccess && cg_) e = cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_);
+        if (e == cudaSuccess) e = cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_);
+        return e;
     }
 
     int ensure_stage(size_t bytes)
@@ -1226,17 +1211,16 @@ private:
     {
         sorted_storage_ = false; // new positions: the storage order may no longer follow the cells
         // The sort base (keys_sorted_) stays a sorted array of the same keys' layout, which is all the incremental sort
-        // needs to be correct: particles whose key matches it at their slot form a sorted subsequence. When more
-        // particles left their slot's key than the mover list holds, the next substep sorts in full: found out in that
-        // substep instead, the overflow aborts it, the launches already queued behind it run empty, and the list is grown
-        // for one substep and shrunk after the run, with the graphs captured again both times (a 50-substep job on 32,768
-        // particles: 4.9 ms so, 4.0 ms on the device; 426k particles, 20 substeps: 3.9 ms against 3.0 ms).
+        // needs to be correct: particles whose key matches it at their slot form a sorted subsequence. When more than a
+        // quarter of the particles left their slot's key, the next substep sorts in full: a tile's bucket takes half as many
+        // movers as the tile has particles, and an overflow found out in that substep aborts it and the launches already
+        // queued behind it run empty.
         const bool based = inc_sort_usable() && !sort_base_stale_;
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, based ? (const uint32_t*)keys_sorted_ : nullptr);
         ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
-        if (based && (int64_t)hst_->max_movers > mcap_) sort_base_stale_ = true;
+        if (based && (uint64_t)hst_->max_movers * 4 > (uint64_t)N_) sort_base_stale_ = true;
         if (hst_->flags & FLAG_OUT_OF_DOMAIN) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
         return 0;
     }
@@ -1266,6 +1250,8 @@ private:
         a.pin = pool(parity);
         a.pout = pool(parity ^ 1);
         a.g_start = g_start_;
+        a.g_stop = g_stop_;
+        a.g_end = g_end_;
         a.g_nbr = g_nbr_;
         a.pay = pay_;
         a.pstride = pstride_;
@@ -1279,6 +1265,8 @@ private:
         a.h_mask = h_mask_;
         a.scenes = d_scenes_;
         a.grid_mass = grid_mass_;
+        a.sort_zero = reinterpret_cast<uint32_t*>(sort_aux_);
+        a.sort_zero_n = (uint32_t)(sort_zero_bytes((int64_t)cap_) / 4);
         a.st = st_;
         a.n_total = N_;
         a.b_cap = b_cap_;
@@ -1301,8 +1289,10 @@ private:
             ZR_CUDA(group_heads(n));
             k_activate<T><<<nsm_ * 4, 256, 0, stream_>>>(a);
         }
-        else // its last kernel places the group heads and activates their blocks (after ev[1]: the activate phase)
-            ZR_CUDA(sort_and_activate_incremental(n, a, ev ? ev[1] : nullptr));
+        else {
+            ZR_CUDA(bin_incremental(n, a));
+            if (ev) ZR_CUDA(cudaEventRecord(ev[1], stream_)); // the merge also activates the blocks: both in the first phase
+        }
         if (sched_.fused == 0 || sched_.fused == 3) // these P2G forms read grid slots; the fused one translates its groups' entries
             k_nbr<T><<<nsm_ * 4, 256, 0, stream_>>>(a);
         if (ev) ZR_CUDA(cudaEventRecord(ev[2], stream_));
@@ -1349,7 +1339,6 @@ private:
         case 3: launch_g2p<3>(a, gi); break;
         default: launch_g2p<0>(a, gi);
         }
-        k_step_end<T><<<1, 256, 0, stream_>>>(d_scenes_, n_scenes(), st_);
         if (ev) ZR_CUDA(cudaEventRecord(ev[5], stream_));
         ZR_CUDA(cudaGetLastError());
         return 0;
@@ -1658,9 +1647,7 @@ private:
         // roll back: scene clocks, a clean grid after an aborted trial, the keys of the current buffer
         ZR_CUDA(cudaMemcpyAsync(d_scenes_, scenes_backup_, sizeof(SceneParams<T>) * h_scenes_.size(), cudaMemcpyDeviceToDevice, stream_));
         if (aborted_out) {
-            ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_));
-            ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_));
-            if (cg_) ZR_CUDA(cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_));
+            ZR_CUDA(clean_substep());
         }
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
@@ -1796,7 +1783,7 @@ private:
         free_io();
         void* ps[] = { pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, g_nbr_, b_key_, acc_, vel_, h_keys_, h_vals_,
             d_scenes_, grid_mass_, st_, sort_tmp_, stage_, pay_, scenes_backup_, ck_pool_, ck_pid_, ck_scenes_, cg_, cgs_,
-            sort_aux_, inc_move_, inc_bkey_, inc_bidx_, inv_ };
+            sort_aux_, inc_bkey_, inc_bidx_, inv_, g_stop_, g_end_ };
         for (void* p : ps)
             if (p) cudaFree(p);
         pool_[0] = pool_[1] = nullptr;
@@ -1819,8 +1806,8 @@ private:
         cgs_ = nullptr;
         implicit_ = false;
         sort_aux_ = nullptr;
-        inc_move_ = inc_bkey_ = inc_bidx_ = nullptr;
-        mcap_ = 0;
+        inc_bkey_ = inc_bidx_ = nullptr;
+        g_stop_ = g_end_ = nullptr;
         inv_ = nullptr;
         inv_cap_ = 0;
         sort_base_stale_ = true;

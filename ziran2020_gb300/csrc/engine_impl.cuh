@@ -3,10 +3,11 @@
 //
 // One substep (MpmSimulationBase::advanceOneTimeStep, MpmSimulationBase.cpp:262-357, with the
 // AnisoFractureSimulation particlesToGrid override, AnisoFractureSimulation.h:129-141):
-//   1. sort      CUB radix sort of the 64-bit particle keys written by the previous G2P (or k_keys)
-//   2. groups    CUB select of the first sorted index of every (scene, SPGrid page)
+//   1. sort      the particle keys written by the previous G2P (or k_keys) merged into the previous order
+//                (incremental sort; a radix sort after loads and aborts)
+//   2. groups    the sorted range of every (scene, SPGrid page)
 //   3. activate  every group inserts its page and the 7 pages at +1 block into a hash table; new
-//                entries get a grid slot (MpmGrid::pollute, MpmGrid.h:153-193)
+//                entries get a grid slot (MpmGrid::pollute, MpmGrid.h:153-193); in one kernel with the merge
 //   4. p2g       one CTA per group: stress V0*tau(F, g(d)) + APIC scatter of m, m v + m C (x_i - x_p),
 //                -V0 tau grad w and the phase-field pair (d w, w) into a shared node tile, then
 //                vector atomics into the 8 neighbouring grid blocks (MpmSimulationBase.cpp:669-855,
@@ -19,7 +20,7 @@
 //                domain checks, next key; writes the particle to its sorted slot of the other buffer
 //                (MpmSimulationBase.cpp:1269-1515, FBasedMpmForceHelper.cpp:95-108,
 //                AnisoFractureSimulation.h:182-283)
-//   7. end       time += dt per scene, substep counter
+//   7. end       time += dt per scene, substep counter (by the last CTA of G2P)
 #pragma once
 #include "common.cuh"
 #include "engine.h"
@@ -92,8 +93,10 @@ struct StepArgs {
     const uint32_t* vals_sorted;
     uint64_t* keys_next;
     Pool<T> pin, pout;
-    const uint32_t* g_start;
-    int32_t* g_nbr;
+    uint32_t* g_start; // per group: first sorted index
+    uint32_t* g_stop; // per group: one past its last sorted index (from P2G's set-up or k_nbr on)
+    uint32_t* g_end; // the same per hash position of the group's own block (from activation on)
+    int32_t* g_nbr; // per group: hash positions (from activation on), then grid slots, of its block and the +1 neighbours
     T* pay; // P2G payload, NPAY fields of pstride elements (also the implicit damage solve's particle scratch)
     int64_t pstride;
     T* cg; // implicit damage solve: CG_NF node vectors of b_cap * nodes
@@ -106,6 +109,8 @@ struct StepArgs {
     uint32_t h_mask;
     SceneParams<T>* scenes;
     double* grid_mass; // per scene, refreshed every substep
+    uint32_t* sort_zero; // the incremental sort's counters, zero at the start of a substep
+    uint32_t sort_zero_n; // words
     DevStatus* st;
     uint32_t n_total;
     uint32_t b_cap;
@@ -235,56 +240,54 @@ struct GroupHead {
 // particles whose cell did not change ("stayers") are already sorted; only the particles that changed cell
 // ("movers", ~2% per substep at the slab's speeds) need placing.
 //
-// Storage is cut into tiles of SORT_TILE indices. B[j] = the smallest stayer key in tiles >= j (non-decreasing;
-// "no key" past the last stayer). Mover key k belongs to bucket b(k) = the largest j with B[j] <= k (0 when there is
-// none): every element of bucket j (its movers) and tile j (its stayers) lies in [B[j], B[j+1]] and comes after
-// every element of lower tiles and buckets, so tile j's merged output starts at
-// (stayers in tiles < j) + (movers in buckets < j). Inside it, in the order (key, stayers first, storage index), a
-// stayer goes to its rank among the tile's stayers plus the bucket's movers with a smaller key, a mover to its rank
-// in the bucket plus the tile's stayers with a key not above its own. The order is fully determined by the keys
-// and storage indices (no dependence on the order in which movers were found).
+// Storage is cut into tiles of SORT_TILE indices. B[j] = the first old key of tile j (the old keys ascend with the
+// storage index). Mover key k belongs to bucket b(k) = the largest j with B[j] <= k (0 when there is none): every
+// element of bucket j (its movers) and tile j (its stayers) lies in [B[j], B[j+1]] and comes after every element of
+// lower tiles and buckets, so tile j's merged output starts at (stayers in tiles < j) + (movers in buckets < j). Inside
+// it, in the order (key, stayers first, storage index), a stayer goes to its rank among the tile's stayers plus the
+// bucket's movers with a smaller key, a mover to its rank in the bucket plus the tile's stayers with a key not above its
+// own. The order is fully determined by the keys and storage indices (no dependence on the order in which movers were
+// found).
 //
-//   k_sort_tiles      per tile: stayer count, first and last stayer key; movers appended to a list (one atomic per
-//                     tile)
-//   k_sort_bucket     per mover: bucket (binary search over B, read from the tiles' first stayer keys), a ticket
+//   k_sort_tiles      per tile: stayer count and last stayer key; per mover its bucket (binary search over B), a ticket
 //                     within it, the bucket's largest key, and (key, storage index) into the bucket's fixed slots
 //   k_sort_merge      per tile: where its output starts and the key just before it (sums and maxima over the lower
 //                     tiles and buckets, by the CTA itself), then the tile's stayers and its bucket's movers (sorted
-//                     in shared memory) to their places; the group heads in the tile's output counted
-//   k_heads_activate  per tile: the group heads of its output written to g_start after the lower tiles' heads, and
-//                     their blocks and +1 neighbours activated in the grid hash
+//                     in shared memory) to their places; the groups that start in the tile's output take group
+//                     numbers, and their blocks and +1 neighbours are activated in the grid hash
 //
-// More movers than the list holds, or a bucket larger than SORT_MAXM, raises FLAG_SORT: the host repeats the
-// substep with a full radix sort (and grows the list).
+// Both kernels are chains of dependent memory round trips (about 0.7 us each) with little work behind them, so what they
+// cost is the length of the chain. B comes from the old keys, known before the pass (B from the stayers put a second
+// kernel between finding the movers and placing them), and groups are numbered as tiles finish (numbers in key order put
+// a third kernel behind the merge, for the head counts of the lower tiles): as five nodes (a memset
+// and four kernels) the substep took 57.0 us on 32,768 particles and 125.6 us on 425,984, with two 49.3 and 118.8 us.
+//
+// A bucket larger than SORT_MAXM raises FLAG_SORT: the host repeats the substep with a full radix sort.
 // ---------------------------------------------------------------------------------------------------
 constexpr int SORT_NT = 256, SORT_PER = 8, SORT_TILE = SORT_NT * SORT_PER, SORT_MAXM = 1024;
 constexpr uint32_t SORT_NOKEY = 0xffffffffu; // keys of the incremental sort hold at most 31 bits
 
 struct SortBufs {
-    int64_t* cnt; // [0] movers found (zeroed per substep)
-    uint32_t* b_cnt; // [tiles] movers per bucket (zeroed per substep)
-    uint32_t* b_max; // [tiles] largest mover key per bucket (zeroed per substep)
+    uint32_t* b_cnt; // [tiles] movers per bucket (zero at the start of a substep; k_grid clears it for the next one)
+    uint32_t* b_max; // [tiles] largest mover key per bucket (likewise)
     uint32_t* stay_bits; // [ceil(n / 32)] bit i % 32 of word i / 32: storage index i keeps its key
+    uint32_t* t_first; // [tiles] first old key per tile: B (k_group_heads or the previous merge wrote it)
     uint32_t* t_stay; // [tiles] stayers per tile
-    uint32_t* t_first; // [tiles] first stayer key per tile (SORT_NOKEY: none)
     uint32_t* t_last; // [tiles] last stayer key per tile (SORT_NOKEY: none)
-    uint32_t* t_base; // [tiles] sorted position of the tile's first output (the merge writes it)
-    uint32_t* t_heads; // [tiles] group heads in the tile's output (the merge counts them)
-    uint32_t* m_idx; // [mcap] movers' storage indices (list order)
     uint32_t* b_key; // [tiles * SORT_MAXM] movers' keys: bucket j's at j * SORT_MAXM + ticket
     uint32_t* b_idx; // [tiles * SORT_MAXM] movers' storage indices, likewise
-    int64_t mcap;
     int64_t n;
     int tiles;
 };
+constexpr int SORT_FIRST = 4096; // tiles whose first keys a CTA copies to shared memory for its searches
 
-static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, const uint32_t* kold, SortBufs sb, DevStatus* st)
+static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, const uint32_t* kold, SortBufs sb, const DevStatus* st)
 {
-    __shared__ uint32_t s_cnt[SORT_NT / 32], s_first[SORT_NT / 32], s_last[SORT_NT / 32], s_moff[SORT_NT / 32][SORT_PER];
-    __shared__ uint64_t s_base;
-    const int j = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ uint32_t s_first[SORT_FIRST];
+    __shared__ uint32_t s_cnt[SORT_NT / 32], s_last[SORT_NT / 32];
+    const int j = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, T = sb.tiles;
     const int64_t t0 = (int64_t)j * SORT_TILE;
-    uint32_t nst = 0, first = SORT_NOKEY, last = SORT_NOKEY;
+    uint32_t nst = 0, last = SORT_NOKEY;
     unsigned moves = 0; // bit r: this thread's item of round r moved
     // items in storage order; a warp takes 256 consecutive ones, 32 at a time; every load issued first
     uint32_t kn[SORT_PER], ko[SORT_PER];
@@ -294,88 +297,43 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* k
         kn[r] = i < sb.n ? knew[i] : 0u;
         ko[r] = i < sb.n ? kold[i] : 1u;
     }
+    const bool ab = aborted(st);
+    if (T <= SORT_FIRST)
+        for (int q = threadIdx.x; q < T; q += SORT_NT) s_first[q] = sb.t_first[q];
+    const uint32_t* B = T <= SORT_FIRST ? s_first : sb.t_first;
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
         const int64_t i = t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane;
-        const bool valid = i < sb.n, stay = valid && kn[r] == ko[r], move = valid && !stay;
-        const unsigned bs = __ballot_sync(0xffffffffu, stay), bm = __ballot_sync(0xffffffffu, move);
+        const bool valid = i < sb.n, stay = valid && kn[r] == ko[r];
+        const unsigned bs = __ballot_sync(0xffffffffu, stay);
         if (lane == 0 && valid) sb.stay_bits[i >> 5] = bs; // the merge reads these: it overwrites the old keys
-        if (bs) {
-            if (first == SORT_NOKEY) first = __shfl_sync(0xffffffffu, kn[r], __ffs(bs) - 1);
-            last = __shfl_sync(0xffffffffu, kn[r], 31 - __clz(bs));
-        }
+        if (bs) last = __shfl_sync(0xffffffffu, kn[r], 31 - __clz(bs));
         nst += __popc(bs);
-        if (move) moves |= 1u << r;
-        if (lane == 0) s_moff[w][r] = __popc(bm);
+        if (valid && !stay) moves |= 1u << r;
     }
     if (lane == 0) {
         s_cnt[w] = nst;
-        s_first[w] = first;
         s_last[w] = last;
     }
     __syncthreads();
-    if (w == 0) {
-        // the tile's movers in storage order (warp-major, then round): 64 counts, two per lane, one warp scan
-        static_assert(SORT_PER * (SORT_NT / 32) == 64, "two counts per lane");
-        uint32_t* mo = &s_moff[0][0];
-        const uint32_t a0 = mo[2 * lane], a1 = mo[2 * lane + 1];
-        uint32_t x = a0 + a1;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+    if (threadIdx.x == 0) {
+        uint32_t c = 0, l = SORT_NOKEY;
+        for (int q = 0; q < SORT_NT / 32; q++) {
+            c += s_cnt[q];
+            if (s_last[q] != SORT_NOKEY) l = s_last[q];
         }
-        mo[2 * lane] = x - a0 - a1;
-        mo[2 * lane + 1] = x - a1;
-        const uint32_t m = __shfl_sync(0xffffffffu, x, 31);
-        if (lane == 0) {
-            uint32_t c = 0, f = SORT_NOKEY, l = SORT_NOKEY;
-            for (int q = 0; q < SORT_NT / 32; q++) {
-                c += s_cnt[q];
-                if (f == SORT_NOKEY) f = s_first[q];
-                if (s_last[q] != SORT_NOKEY) l = s_last[q];
-            }
-            sb.t_stay[j] = c;
-            sb.t_first[j] = f;
-            sb.t_last[j] = l;
-            s_base = m ? (uint64_t)atomicAdd((unsigned long long*)&sb.cnt[0], (unsigned long long)m) : 0ull; // one atomic per tile
-        }
+        sb.t_stay[j] = c;
+        sb.t_last[j] = l;
     }
-    __syncthreads();
-    const uint64_t base = s_base;
+    if (ab || !moves) return; // (an aborted substep's tickets would not be cleared)
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
-        const unsigned bm = __ballot_sync(0xffffffffu, (moves >> r) & 1u);
-        if ((moves >> r) & 1u) {
-            const uint64_t pos = base + s_moff[w][r] + __popc(bm & ((1u << lane) - 1u));
-            if (pos < (uint64_t)sb.mcap) sb.m_idx[pos] = (uint32_t)(t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane);
-        }
-    }
-    (void)st;
-}
-
-static __global__ void __launch_bounds__(SORT_NT) k_sort_bucket(const uint32_t* knew, SortBufs sb, DevStatus* st)
-{
-    const int64_t Mall = sb.cnt[0];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicMax(&st->max_movers, (uint32_t)(Mall < 0xffffffffLL ? Mall : 0xffffffffLL));
-        if (Mall > sb.mcap) raise_flag(st, FLAG_SORT);
-    }
-    const int64_t M = min(Mall, sb.mcap);
-    const int T = sb.tiles;
-    // B[q] = the first stayer key at or after tile q: a tile without a stayer takes the next tile's (emptying a tile
-    // takes 2048 listed movers, so these walks are short); non-decreasing, as the stayers keep their order
-    auto B = [&](int q) {
-        uint32_t v = sb.t_first[q];
-        while (v == SORT_NOKEY && ++q < T) v = sb.t_first[q];
-        return v;
-    };
-    for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < M; m += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t i = sb.m_idx[m];
-        const uint32_t k = i < (uint64_t)sb.n ? knew[i] : SORT_NOKEY;
-        int lo = 0, hi = T; // first j with B[j] > k
+        if (!((moves >> r) & 1u)) continue;
+        const uint32_t k = kn[r];
+        int lo = 0, hi = T; // first q with B[q] > k
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (B(mid) <= k) lo = mid + 1;
+            if (B[mid] <= k) lo = mid + 1;
             else hi = mid;
         }
         const uint32_t b = lo > 0 ? (uint32_t)(lo - 1) : 0u;
@@ -383,30 +341,92 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_bucket(const uint32_t* 
         atomicMax(&sb.b_max[b], k);
         if (t < (uint32_t)SORT_MAXM) { // a fuller bucket makes the merge raise FLAG_SORT
             sb.b_key[(size_t)b * SORT_MAXM + t] = k;
-            sb.b_idx[(size_t)b * SORT_MAXM + t] = i;
+            sb.b_idx[(size_t)b * SORT_MAXM + t] = (uint32_t)(t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane);
         }
     }
 }
 
-static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* knew, SortBufs sb, uint32_t* out_keys, uint32_t* out_vals, KeyLayout kl,
-    DevStatus* st)
+// Block dl (x*4 + y*2 + z, at +1 block) of the group with key key0, into the block hash; a block seen for the first time
+// takes the next grid slot (one slot counter atomic per group of converged lanes). Returns the block's hash position,
+// whether this thread inserted the block or found it (-1: the probe failed and raised FLAG_CAPACITY). The slot behind it
+// is written by the inserting thread, so it is read (nbr_slot) only by a later kernel.
+template <class T>
+__device__ __forceinline__ int32_t activate_block(const StepArgs<T>& a, uint64_t key0, uint32_t dl)
 {
-    __shared__ uint32_t s_key[SORT_TILE], s_idx[SORT_TILE]; // the tile's stayers in storage (= key) order
-    __shared__ uint32_t m_key[SORT_MAXM], m_idx[SORT_MAXM], m_key2[SORT_MAXM], m_idx2[SORT_MAXM];
-    __shared__ uint32_t o_key[SORT_TILE + SORT_MAXM]; // the tile's output in order
-    __shared__ uint32_t s_heads;
-    __shared__ uint32_t s_wcnt[SORT_PER][SORT_NT / 32];
-    __shared__ uint32_t s_red[2][SORT_NT / 32];
-    __shared__ int s_ns;
-    const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int64_t M = sb.cnt[0];
-    if (M > sb.mcap) return; // FLAG_SORT raised: the substep is repeated with a full sort
-    const uint32_t bc = sb.b_cnt[j];
-    if (bc > (uint32_t)SORT_MAXM) {
-        if (tid == 0) raise_flag(st, FLAG_SORT);
-        return;
+    using L = typename LayoutOf<T>::type;
+    const uint64_t scene = a.kl.scene(key0);
+    uint32_t bi, bj, bk;
+    L::block_of_page(a.kl.page(key0), bi, bj, bk);
+    const uint64_t hk = (scene << 40) | L::page_of_block(bi + (dl >> 2), bj + ((dl >> 1) & 1), bk + (dl & 1));
+    uint32_t h = (uint32_t)hash64(hk) & a.h_mask;
+    bool done = false, fresh = false;
+    for (int p = 0; p < HASH_PROBES && !done; p++) {
+        const unsigned long long prev = atomicCAS((unsigned long long*)&a.h_keys[h], (unsigned long long)HASH_EMPTY, (unsigned long long)hk);
+        if (prev == HASH_EMPTY)
+            done = fresh = true;
+        else if (prev == hk)
+            done = true;
+        else
+            h = (h + 1) & a.h_mask;
     }
-    const int nm = (int)bc;
+    if (!done) raise_flag(a.st, FLAG_CAPACITY);
+    const unsigned am = __activemask();
+    const unsigned nw = __ballot_sync(am, fresh);
+    if (nw) {
+        const int lane = threadIdx.x & 31, leader = __ffs(nw) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(&a.st->n_blocks, (uint32_t)__popc(nw));
+        base = __shfl_sync(am, base, leader);
+        if (fresh) {
+            const uint32_t slot = base + (uint32_t)__popc(nw & ((1u << lane) - 1u));
+            if (slot >= a.b_cap) {
+                raise_flag(a.st, FLAG_CAPACITY);
+                a.h_vals[h] = -1;
+            }
+            else {
+                a.h_vals[h] = (int32_t)slot;
+                a.b_key[slot] = hk;
+            }
+        }
+    }
+    return done ? (int32_t)h : -1;
+}
+
+// The shared buffers of k_sort_merge's two parts overlap.
+union MergeShared {
+    struct {
+        uint32_t s_key[SORT_TILE], s_idx[SORT_TILE]; // the tile's stayers in storage (= key) order
+        uint32_t m_key[SORT_MAXM], m_idx[SORT_MAXM], m_key2[SORT_MAXM], m_idx2[SORT_MAXM];
+    } m;
+    uint32_t pos[SORT_TILE + SORT_MAXM]; // output positions of the tile's group heads, in order
+};
+
+template <class T>
+__global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uint32_t* knew, SortBufs sb, uint32_t* out_keys, uint32_t* out_vals)
+{
+    constexpr int RMAX = (SORT_TILE + SORT_MAXM) / SORT_NT; // rounds over a tile's output
+    __shared__ MergeShared sh;
+    __shared__ uint32_t o_key[SORT_TILE + SORT_MAXM]; // the tile's output in order
+    __shared__ uint32_t s_wcnt[RMAX][SORT_NT / 32];
+    __shared__ uint32_t s_red[2][SORT_NT / 32];
+    __shared__ uint32_t s_ns, s_nh, s_g0;
+    uint32_t *s_key = sh.m.s_key, *s_idx = sh.m.s_idx, *m_key = sh.m.m_key, *m_idx = sh.m.m_idx, *m_key2 = sh.m.m_key2, *m_idx2 = sh.m.m_idx2;
+    const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    DevStatus* st = a.st;
+    const KeyLayout kl = a.kl;
+    if (blockIdx.x == 0) // the per-scene grid mass k_grid accumulates
+        for (int s = tid; s < a.n_scenes; s += SORT_NT) a.grid_mass[s] = 0;
+    // the tile's new keys and stay bits: issued ahead of everything that is tested. Item (r, w, lane) = t0 + r*256 + w*32 + lane
+    const int64_t t0 = (int64_t)j * SORT_TILE;
+    uint32_t keys[SORT_PER];
+    unsigned mine = 0; // bit r: this thread's item of round r stays
+#pragma unroll
+    for (int r = 0; r < SORT_PER; r++) {
+        const int64_t i = t0 + r * SORT_NT + tid;
+        keys[r] = i < sb.n ? knew[i] : 0u;
+        if (i < sb.n && ((sb.stay_bits[i >> 5] >> lane) & 1u)) mine |= 1u << r; // i % 32 == lane: rounds and warps start at multiples of 32
+    }
+    const uint32_t bc = sb.b_cnt[j];
     // the lower tiles and buckets: their element count (where this tile's output starts) and their largest key (the
     // key just before the output: stayer and bucket key ranges ascend with the tile). pk holds key + 1, 0 for none.
     uint32_t below = 0, pk = 0;
@@ -417,6 +437,16 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
         if (l != SORT_NOKEY) pk = max(pk, l + 1);
         if (c) pk = max(pk, mk + 1);
     }
+    if (aborted_cta(st)) return;
+    if (bc > (uint32_t)SORT_MAXM) { // the whole CTA: the substep is repeated with a full sort
+        if (tid == 0) raise_flag(st, FLAG_SORT);
+        return;
+    }
+    const int nm = (int)bc;
+    for (int q = tid; q < nm; q += SORT_NT) {
+        m_key[q] = sb.b_key[(size_t)j * SORT_MAXM + q];
+        m_idx[q] = sb.b_idx[(size_t)j * SORT_MAXM + q];
+    }
     for (int o = 16; o > 0; o >>= 1) {
         below += __shfl_down_sync(0xffffffffu, below, o);
         pk = max(pk, __shfl_down_sync(0xffffffffu, pk, o));
@@ -425,42 +455,30 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
         s_red[0][w] = below;
         s_red[1][w] = pk;
     }
-    // the tile's stayers, compacted in storage order: item (r, w, lane) = t0 + r*256 + w*32 + lane
-    const int64_t t0 = (int64_t)j * SORT_TILE;
-    unsigned mine = 0; // bit r: this thread's item of round r stays
-    uint32_t keys[SORT_PER];
+    // the tile's stayers, compacted in storage order
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
-        const int64_t i = t0 + r * SORT_NT + tid;
-        keys[r] = 0;
-        bool stay = false;
-        if (i < sb.n) {
-            keys[r] = knew[i];
-            stay = (sb.stay_bits[i >> 5] >> lane) & 1u; // i % 32 == lane: rounds and warps start at multiples of 32
-        }
-        const unsigned b = __ballot_sync(0xffffffffu, stay);
-        if (stay) mine |= 1u << r;
+        const unsigned b = __ballot_sync(0xffffffffu, (mine >> r) & 1u);
         if (lane == 0) s_wcnt[r][w] = __popc(b);
     }
-    for (int q = tid; q < nm; q += SORT_NT) {
-        m_key[q] = sb.b_key[(size_t)j * SORT_MAXM + q];
-        m_idx[q] = sb.b_idx[(size_t)j * SORT_MAXM + q];
-    }
-    __syncthreads();
-    if (w == 0) { // exclusive offsets of the 64 (round, warp) groups in storage order: two per lane, one warp scan
-        static_assert(SORT_PER * (SORT_NT / 32) == 64, "two groups per lane");
+    // exclusive offsets of the (round, warp) counts in order by the first warp, the total into *total: 8 per round
+    auto scan_counts = [&](int rounds, uint32_t* total) {
         uint32_t* c = &s_wcnt[0][0];
-        const uint32_t a0 = c[2 * lane], a1 = c[2 * lane + 1];
-        uint32_t x = a0 + a1;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+        uint32_t carry = 0;
+        for (int q0 = 0; q0 < rounds * (SORT_NT / 32); q0 += 32) {
+            const uint32_t v = q0 + lane < rounds * (SORT_NT / 32) ? c[q0 + lane] : 0u;
+            uint32_t x = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (q0 + lane < rounds * (SORT_NT / 32)) c[q0 + lane] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
         }
-        const uint32_t ex = x - a0 - a1;
-        c[2 * lane] = ex;
-        c[2 * lane + 1] = ex + a0;
-        if (lane == 31) s_ns = (int)x;
-    }
+        if (lane == 0) *total = carry;
+    };
+    __syncthreads();
+    if (w == 0) scan_counts(SORT_PER, &s_ns);
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
@@ -480,7 +498,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
         m_idx2[rank] = i;
     }
     __syncthreads();
-    const int ns = s_ns;
+    const int ns = (int)s_ns, cnt = ns + nm;
     uint32_t below_all = 0, pk_all = 0;
 #pragma unroll
     for (int q = 0; q < SORT_NT / 32; q++) {
@@ -488,7 +506,17 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
         pk_all = max(pk_all, s_red[1][q]);
     }
     const int64_t base = below_all; // elements of lower tiles and buckets
-    if (tid == 0) sb.t_base[j] = below_all;
+    if (base + cnt > sb.n) { // the counts cannot give this range (the whole CTA)
+        if (tid == 0) check_failed(st, 8);
+        return;
+    }
+    auto place = [&](int p, uint32_t k, uint32_t v) { // output p of the tile
+        const int64_t pos = base + p;
+        out_keys[pos] = k;
+        out_vals[pos] = v;
+        o_key[p] = k;
+        if (pos % SORT_TILE == 0) sb.t_first[pos / SORT_TILE] = k; // B of the next substep
+    };
     for (int t = tid; t < ns; t += SORT_NT) { // stayer: its rank + the bucket's movers with a smaller key
         const uint32_t k = s_key[t];
         int lo = 0, hi = nm;
@@ -497,14 +525,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
             if (m_key2[mid] < k) lo = mid + 1;
             else hi = mid;
         }
-        const int64_t pos = base + t + lo;
-        if (pos < 0 || pos >= sb.n) {
-            check_failed(st, 8);
-            continue;
-        }
-        out_keys[pos] = k;
-        out_vals[pos] = s_idx[t];
-        o_key[t + lo] = k;
+        place(t + lo, k, s_idx[t]);
     }
     for (int r = tid; r < nm; r += SORT_NT) { // mover: its rank + the tile's stayers with a key not above its own
         const uint32_t k = m_key2[r];
@@ -514,30 +535,62 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
             if (s_key[mid] <= k) lo = mid + 1;
             else hi = mid;
         }
-        const int64_t pos = base + r + lo;
-        if (pos < 0 || pos >= sb.n) {
-            check_failed(st, 8);
+        place(r + lo, k, m_idx2[r]);
+    }
+    __syncthreads();
+    // the groups that start in the tile's output: an output whose group differs from that of the key before it
+    const uint32_t pred = pk_all ? pk_all - 1 : SORT_NOKEY; // the key before the tile's output (SORT_NOKEY: none)
+    const int R = (cnt + SORT_NT - 1) / SORT_NT;
+    unsigned heads = 0;
+#pragma unroll
+    for (int r = 0; r < RMAX; r++) {
+        if (r >= R) break;
+        const int p = r * SORT_NT + tid;
+        bool head = false;
+        if (p < cnt) {
+            const uint32_t k = o_key[p], kp = p == 0 ? pred : o_key[p - 1];
+            head = (p == 0 && pred == SORT_NOKEY) || kl.group(k) != kl.group(kp);
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, head);
+        if (head) heads |= 1u << r;
+        if (lane == 0) s_wcnt[r][w] = __popc(b);
+    }
+    __syncthreads();
+    if (w == 0) {
+        scan_counts(R, &s_nh);
+        __syncwarp();
+        if (lane == 0) s_g0 = s_nh ? atomicAdd(&st->n_groups, s_nh) : 0u; // group numbers: as tiles come
+    }
+#pragma unroll
+    for (int r = 0; r < RMAX; r++) {
+        if (r >= R) break;
+        const unsigned b = __ballot_sync(0xffffffffu, (heads >> r) & 1u);
+        if (r == 0) __syncthreads(); // (after the first ballot: every warp takes part)
+        if ((heads >> r) & 1u) sh.pos[s_wcnt[r][w] + __popc(b & ((1u << lane) - 1u))] = (uint32_t)(r * SORT_NT + tid);
+    }
+    __syncthreads();
+    if (R == 0 && j + 1 < sb.tiles) return;
+    const uint32_t nh = s_nh, g0 = s_g0;
+    // per group: its 8 blocks, its first sorted index, and the end of the group before it (known by that group's own block)
+    for (uint32_t t = tid; t < nh * 9; t += SORT_NT) {
+        const uint32_t i = t / 9, q = t - 9 * i, p = sh.pos[i], g = g0 + i;
+        if (g >= a.b_cap || g >= (uint64_t)sb.n) { // more groups than grid blocks: the host grows the grid and repeats the substep
+            raise_flag(st, FLAG_CAPACITY);
             continue;
         }
-        out_keys[pos] = k;
-        out_vals[pos] = m_idx2[r];
-        o_key[r + lo] = k;
+        if (q == 8 && p == 0 && pred == SORT_NOKEY) continue; // nothing before the first group
+        const uint32_t k = q < 8 ? o_key[p] : (p == 0 ? pred : o_key[p - 1]);
+        const int32_t h = activate_block(a, (uint64_t)k, q & 7);
+        if (q < 8)
+            a.g_nbr[(size_t)g * 8 + q] = h;
+        else if (h >= 0)
+            a.g_end[h] = (uint32_t)(base + p);
+        if (q == 0) a.g_start[g] = (uint32_t)(base + p);
     }
-    // group heads in the tile's output (compared with the key before it): counted here, placed by k_heads_activate
-    if (tid == 0) s_heads = 0;
-    __syncthreads();
-    const uint32_t pred = pk_all ? pk_all - 1 : SORT_NOKEY;
-    uint32_t h = 0;
-    for (int p = tid; p < ns + nm; p += SORT_NT) {
-        const uint32_t k = o_key[p];
-        const bool first = p == 0 ? pred == SORT_NOKEY : false;
-        const uint32_t kp = p == 0 ? pred : o_key[p - 1];
-        h += (first || kl.group(k) != kl.group(kp)) ? 1u : 0u;
+    if (j + 1 == sb.tiles && tid == 0) { // the last group ends with the particles
+        const int32_t h = activate_block(a, (uint64_t)(cnt ? o_key[cnt - 1] : pred), 0);
+        if (h >= 0) a.g_end[h] = (uint32_t)sb.n;
     }
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_down_sync(0xffffffffu, h, o);
-    if (lane == 0 && h) atomicAdd(&s_heads, h);
-    __syncthreads();
-    if (tid == 0) sb.t_heads[j] = s_heads;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -549,7 +602,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_merge(const uint32_t* k
 constexpr uint64_t LB_AGG = 1ull << 62, LB_PREFIX = 2ull << 62, LB_VALUE = (1ull << 62) - 1;
 
 static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* keys, int64_t n, KeyLayout kl, uint64_t* status, uint32_t* counter,
-    uint32_t* g_start, uint32_t cap, DevStatus* st)
+    uint32_t* g_start, uint32_t cap, uint32_t* t_first, DevStatus* st)
 {
     __shared__ uint32_t s_w[SORT_PER][SORT_NT / 32];
     __shared__ int s_tile;
@@ -559,6 +612,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* 
     __syncthreads();
     const int j = s_tile;
     const int64_t t0 = (int64_t)j * SORT_TILE;
+    if (tid == 0) t_first[j] = (uint32_t)kl.at(keys, (uint32_t)t0); // B of the next substep's incremental sort (32-bit keys)
     unsigned mine = 0;
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
@@ -635,52 +689,6 @@ static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* 
     }
 }
 
-// Block dl (x*4 + y*2 + z, at +1 block) of the group whose first sorted key is key0, into the block hash; a block
-// seen for the first time takes the next grid slot (one slot counter atomic per group of converged lanes).
-template <class T>
-__device__ __forceinline__ void activate_block(const StepArgs<T>& a, uint64_t key0, uint32_t dl, int32_t* hpos)
-{
-    using L = typename LayoutOf<T>::type;
-    const uint64_t scene = a.kl.scene(key0);
-    uint32_t bi, bj, bk;
-    L::block_of_page(a.kl.page(key0), bi, bj, bk);
-    const uint64_t hk = (scene << 40) | L::page_of_block(bi + (dl >> 2), bj + ((dl >> 1) & 1), bk + (dl & 1));
-    uint32_t h = (uint32_t)hash64(hk) & a.h_mask;
-    bool done = false, fresh = false;
-    for (int p = 0; p < HASH_PROBES && !done; p++) {
-        const unsigned long long prev = atomicCAS((unsigned long long*)&a.h_keys[h], (unsigned long long)HASH_EMPTY, (unsigned long long)hk);
-        if (prev == HASH_EMPTY)
-            done = fresh = true;
-        else if (prev == hk)
-            done = true;
-        else
-            h = (h + 1) & a.h_mask;
-    }
-    if (!done) raise_flag(a.st, FLAG_CAPACITY);
-    // The group's neighbour entry gets the block's hash position, whether this thread inserted the block or found
-    // it: the slot is written by the inserting thread below, so it is read (nbr_slot) only by a later kernel.
-    *hpos = done ? (int32_t)h : -1;
-    const unsigned am = __activemask();
-    const unsigned nw = __ballot_sync(am, fresh);
-    if (nw) {
-        const int lane = threadIdx.x & 31, leader = __ffs(nw) - 1;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&a.st->n_blocks, (uint32_t)__popc(nw));
-        base = __shfl_sync(am, base, leader);
-        if (fresh) {
-            const uint32_t slot = base + (uint32_t)__popc(nw & ((1u << lane) - 1u));
-            if (slot >= a.b_cap) {
-                raise_flag(a.st, FLAG_CAPACITY);
-                a.h_vals[h] = -1;
-            }
-            else {
-                a.h_vals[h] = (int32_t)slot;
-                a.b_key[slot] = hk;
-            }
-        }
-    }
-}
-
 // the blocks of every group (after a full sort and k_group_heads), 8 per group
 template <class T>
 __global__ void k_activate(StepArgs<T> a)
@@ -689,121 +697,39 @@ __global__ void k_activate(StepArgs<T> a)
         for (int s = threadIdx.x; s < a.n_scenes; s += blockDim.x) a.grid_mass[s] = 0;
     if (aborted(a.st)) return;
     const uint32_t G = a.st->n_groups;
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.st->max_groups_seen = max(a.st->max_groups_seen, G);
     if (G > a.b_cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_flag(a.st, FLAG_CAPACITY);
         return;
     }
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < G * 8; t += gridDim.x * blockDim.x)
-        activate_block(a, a.kl.at(a.keys_sorted, a.g_start[t >> 3]), t & 7, a.g_nbr + t);
-}
-
-// After the incremental sort's merge, per tile: the group heads of the tile's output (sorted positions
-// [t_base of the tile, of the next tile), each compared with the sorted key before it) written in order into
-// g_start after the heads of the lower tiles (summed by the CTA itself from the merge's counts), then the 8 blocks
-// of each of these groups activated. The last tile stores the number of groups.
-template <class T>
-__global__ void __launch_bounds__(SORT_NT) k_heads_activate(StepArgs<T> a, SortBufs sb, uint32_t* g_start, uint32_t cap)
-{
-    constexpr int RMAX = (SORT_TILE + SORT_MAXM) / SORT_NT;
-    __shared__ uint32_t s_c[RMAX][SORT_NT / 32], s_part[SORT_NT / 32];
-    __shared__ uint32_t s_pos[RMAX * SORT_NT]; // sorted positions of the tile's heads, in order
-    __shared__ uint32_t s_g0, s_nh;
-    if (blockIdx.x == 0) // the per-scene grid mass k_grid accumulates
-        for (int s = threadIdx.x; s < a.n_scenes; s += blockDim.x) a.grid_mass[s] = 0;
-    if (aborted_cta(a.st)) return; // FLAG_SORT from the merge, or an earlier failure: the substep is repeated
-    const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const uint32_t* keys = reinterpret_cast<const uint32_t*>(a.keys_sorted); // the incremental sort's keys are 32-bit
-    const int64_t b0 = sb.t_base[j];
-    const int64_t b1 = j + 1 < sb.tiles ? (int64_t)sb.t_base[j + 1] : sb.n;
-    if (b1 < b0 || b1 > sb.n || b1 - b0 > (int64_t)RMAX * SORT_NT) { // the merge's outputs cannot give this range
-        if (tid == 0) check_failed(a.st, 9);
-        return;
-    }
-    // heads of the lower tiles
-    uint32_t pre = 0;
-    for (int q = tid; q < j; q += SORT_NT) pre += sb.t_heads[q];
-    for (int o = 16; o > 0; o >>= 1) pre += __shfl_down_sync(0xffffffffu, pre, o);
-    if (lane == 0) s_part[w] = pre;
-    // the range's keys and head flags, items (r, w, lane) = b0 + r*256 + w*32 + lane, every load issued first
-    const int R = (int)((b1 - b0 + SORT_NT - 1) / SORT_NT);
-    uint32_t k[RMAX], kl0[RMAX]; // the item's key; for lane 0 also the key before it (another warp's item)
-#pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        const int64_t p = b0 + r * SORT_NT + tid;
-        const bool in = r < R && p < b1;
-        k[r] = in ? keys[p] : 0u;
-        kl0[r] = (in && lane == 0 && p > 0) ? keys[p - 1] : 0u;
-    }
-    unsigned mine = 0;
-#pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        if (r >= R) break;
-        const int64_t p = b0 + r * SORT_NT + tid;
-        uint32_t prev = __shfl_up_sync(0xffffffffu, k[r], 1);
-        if (lane == 0) prev = kl0[r];
-        const bool head = p < b1 && (p == 0 || a.kl.group(k[r]) != a.kl.group(prev));
-        const unsigned b = __ballot_sync(0xffffffffu, head);
-        if (head) mine |= 1u << r;
-        if (lane == 0) s_c[r][w] = __popc(b);
-    }
-    __syncthreads();
-    if (w == 0) { // exclusive offsets of the (row, warp) counts in order, after the lower tiles' heads
-        uint32_t base = 0;
-        for (int q = 0; q < SORT_NT / 32; q++) base += s_part[q];
-        uint32_t carry = base;
-        for (int r = 0; r < R; r++) {
-            uint32_t c = lane < SORT_NT / 32 ? s_c[r][lane] : 0u, x = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (lane < SORT_NT / 32) s_c[r][lane] = carry + x - c;
-            carry += __shfl_sync(0xffffffffu, x, 31);
-        }
-        if (lane == 0) {
-            s_g0 = base;
-            s_nh = carry - base;
-            if (j + 1 == sb.tiles) {
-                a.st->n_groups = carry;
-                a.st->max_groups_seen = max(a.st->max_groups_seen, carry);
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t g0 = s_g0;
-#pragma unroll
-    for (int r = 0; r < RMAX; r++) {
-        if (r >= R) break;
-        const unsigned b = __ballot_sync(0xffffffffu, (mine >> r) & 1u);
-        if ((mine >> r) & 1u) {
-            const uint32_t pos = s_c[r][w] + __popc(b & ((1u << lane) - 1u)), p = (uint32_t)(b0 + r * SORT_NT + tid);
-            s_pos[pos - g0] = p; // pos - g0 < the tile's item count <= RMAX * SORT_NT
-            if (pos < cap) g_start[pos] = p;
-            else check_failed(a.st, 9);
-        }
-    }
-    __syncthreads();
-    const uint32_t nh = s_nh;
-    for (uint32_t t = tid; t < nh * 8; t += SORT_NT) {
-        if (g0 + (t >> 3) >= a.b_cap) { // more groups than grid blocks: the host grows the grid and repeats the substep
-            raise_flag(a.st, FLAG_CAPACITY);
-            continue;
-        }
-        activate_block(a, (uint64_t)keys[s_pos[t >> 3]], t & 7, a.g_nbr + (size_t)g0 * 8 + t);
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < G * 8; t += gridDim.x * blockDim.x) {
+        const uint32_t g = t >> 3;
+        const int32_t h = activate_block(a, a.kl.at(a.keys_sorted, a.g_start[g]), t & 7);
+        a.g_nbr[t] = h;
+        if ((t & 7) == 0 && h >= 0) a.g_end[h] = g + 1 < G ? a.g_start[g + 1] : a.n_total;
     }
 }
 
 // ---------------------------------------------------------------------------------------------------
-// neighbour slots: the grid slots of every group's block and its 7 neighbours at +1 block (read by P2G and
-// G2P). Activation leaves the hash position of each of these blocks in g_nbr; the slot behind it is final once
-// activation has ended. The fused P2G translates its groups' entries itself while it sets them up (and writes
-// the slots back for G2P); the other P2G forms read slots, so k_nbr translates every entry before them.
+// neighbour slots: the grid slots of every group's block and its 7 neighbours at +1 block, and the end of the group's
+// sorted range (read by P2G and G2P). Activation leaves the hash position of each of these blocks in g_nbr; the slot
+// behind it, and the range's end behind the group's own block (g_end), are final once activation has ended. The fused
+// P2G translates its groups' entries itself while it sets them up (and writes the slots and the end back for G2P, into
+// g_nbr and g_stop); the other P2G forms read those, so k_nbr translates every entry before them.
 // ---------------------------------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ int32_t nbr_slot(const StepArgs<T>& a, int32_t hpos)
 {
     return (uint32_t)hpos <= a.h_mask ? a.h_vals[hpos] : -1; // -1: the probe failed and raised FLAG_CAPACITY
+}
+// the end of the sorted range of the group that starts at `start` and whose own block has hash position hpos; an end
+// that cannot be one is a failed check and leaves one particle
+template <class T>
+__device__ __forceinline__ uint32_t group_stop(const StepArgs<T>& a, uint32_t start, int32_t hpos)
+{
+    const uint32_t en = (uint32_t)hpos <= a.h_mask ? a.g_end[hpos] : 0u;
+    if (en > start && en <= a.n_total) return en;
+    if (hpos >= 0) check_failed(a.st, 10);
+    return start + 1;
 }
 
 template <class T>
@@ -813,9 +739,10 @@ __global__ void k_nbr(StepArgs<T> a)
     const uint32_t G = a.st->n_groups;
     if (G > a.b_cap) return; // activation already raised FLAG_CAPACITY
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < G * 8; t += gridDim.x * blockDim.x) {
-        const int32_t slot = nbr_slot(a, a.g_nbr[t]);
+        const int32_t h = a.g_nbr[t], slot = nbr_slot(a, h);
         if (slot < 0) raise_flag(a.st, FLAG_CAPACITY);
         a.g_nbr[t] = slot;
+        if ((t & 7) == 0) a.g_stop[t >> 3] = group_stop(a, a.g_start[t >> 3], h);
     }
 }
 
@@ -1265,7 +1192,7 @@ __device__ void scatter_producer(const StepArgs<T>& a, unsigned char* dyn, uint6
         int32_t nbr[8];
         if (g < G) {
             qs = a.g_start[g];
-            qe = (g + 1 < G) ? a.g_start[g + 1] : a.n_total;
+            qe = a.g_stop[g];
             nf = a.scenes[a.kl.scene(a.kl.at(a.keys_sorted, qs))].damage ? NACC : 4;
 #pragma unroll
             for (int d = 0; d < 8; d++) {
@@ -1488,7 +1415,17 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         if (tid == 0) v = (int)atomicAdd(&a.st->work_p2g, 1u);
         return __shfl_sync(0xffffffffu, v, 0);
     };
-    auto setup_store = [&](int bb, int gn, uint32_t st, uint32_t en, int32_t slot, uint64_t key0) { // lanes 0-7 of warp 0
+    // A group's neighbour entries hold hash positions (activation); the set-up translates them into grid slots and
+    // writes the slots back for G2P, and the range's end likewise.
+    auto take_slot = [&](int gg, int32_t hpos) { // lanes 0-7 of warp 0
+        const int32_t slot = nbr_slot(a, hpos);
+        a.g_nbr[gg * 8 + tid] = slot;
+        return slot;
+    };
+    auto setup_store = [&](int bb, int gn, uint32_t st, int32_t hpos) { // lanes 0-7 of warp 0
+        const uint64_t key0 = tid == 0 ? a.kl.at(a.keys_sorted, st) : 0ull;
+        const uint32_t en = tid == 0 ? group_stop(a, st, hpos) : 0u;
+        const int32_t slot = take_slot(gn, hpos);
         const unsigned badm = __ballot_sync(0xffu, slot < 0 || (uint32_t)slot >= a.b_cap); // a failed lookup raised FLAG_CAPACITY
         s_nbr[bb][tid] = slot;
         if (tid == 0) {
@@ -1502,14 +1439,8 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             s_org[bb][2] = (int)(bk * L::sz);
             s_se[bb][0] = st;
             s_se[bb][1] = en;
+            a.g_stop[gn] = en;
         }
-    };
-    // A group's neighbour entries hold hash positions (activation); the set-up translates them into grid slots and
-    // writes the slots back for G2P.
-    auto take_slot = [&](int gg, int32_t hpos) { // lanes 0-7 of warp 0
-        const int32_t slot = nbr_slot(a, hpos);
-        a.g_nbr[gg * 8 + tid] = slot;
-        return slot;
     };
     const int ii = tid / NC, c = tid % NC;
     const int cx = c >> (L::zbits + L::ybits), cy = (c >> L::zbits) & (L::sy - 1), cz = c & (L::sz - 1);
@@ -1518,10 +1449,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
     if (tid < 32) { // the first group
         const int g0 = claim();
         if (g0 < (int)G) {
-            if (tid < 8) {
-                const uint32_t st = a.g_start[g0], en = g0 + 1 < (int)G ? a.g_start[g0 + 1] : a.n_total;
-                setup_store(0, g0, st, en, take_slot(g0, a.g_nbr[g0 * 8 + tid]), tid == 0 ? a.kl.at(a.keys_sorted, st) : 0ull);
-            }
+            if (tid < 8) setup_store(0, g0, a.g_start[g0], a.g_nbr[g0 * 8 + tid]);
         }
         else if (tid == 0)
             s_g[0] = g0;
@@ -1546,9 +1474,10 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         const int gpf = g + (int)gridDim.x, pfl = tid - 32;
         const bool pf = (a.opts & OPT_PREFETCH) && pfl >= 0 && pfl < NPF && gpf < (int)G;
         uint32_t pf_a = 0, pf_b = 0, pf_j0 = 0, pf_j1 = 0;
+        int32_t pf_h = -1;
         if (pf) {
             pf_a = a.g_start[gpf];
-            pf_b = gpf + 1 < (int)G ? a.g_start[gpf + 1] : a.n_total;
+            pf_h = a.g_nbr[gpf * 8];
         }
         for (uint32_t c0 = start; c0 < end && !bad; c0 += CHUNK) {
             const int cnt = (int)min((uint32_t)CHUNK, end - c0);
@@ -1592,13 +1521,13 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             add_to_offset_tile<T, L>(acc, tile, cx, cy, cz, ii, nf); // all lanes (an empty cell adds zeros)
             __syncthreads();
         }
-        uint32_t n_st = 0, n_en = 0;
+        uint32_t n_st = 0;
         int32_t n_hpos = -1;
         if (tid < 8 && gn < (int)G) {
             n_st = a.g_start[gn];
-            n_en = gn + 1 < (int)G ? a.g_start[gn + 1] : a.n_total;
             n_hpos = a.g_nbr[gn * 8 + tid];
         }
+        if (pf && (uint32_t)pf_h <= a.h_mask) pf_b = a.g_end[pf_h]; // (a range that is none is skipped)
         if (pf && pf_b > pf_a && pf_b <= a.n_total) {
             pf_j0 = a.vals_sorted[pf_a];
             pf_j1 = a.vals_sorted[pf_b - 1];
@@ -1614,7 +1543,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         // the next group's set-up into the other buffer (the flush above read this one)
         if (tid < 8) {
             if (gn < (int)G)
-                setup_store(bcur ^ 1, gn, n_st, n_en, take_slot(gn, n_hpos), tid == 0 ? a.kl.at(a.keys_sorted, n_st) : 0ull);
+                setup_store(bcur ^ 1, gn, n_st, n_hpos);
             else if (tid == 0)
                 s_g[bcur ^ 1] = gn;
         }
@@ -1687,7 +1616,7 @@ __global__ void __launch_bounds__(WsShape<T>::NT, 2) k_p2g_ws(StepArgs<T> a)
         uint32_t fallbacks = 0, k = 0;
         bool stop = false;
         for (uint32_t g = blockIdx.x; g < G && !stop; g += gridDim.x) {
-            const uint32_t start = a.g_start[g], end = (g + 1 < G) ? a.g_start[g + 1] : a.n_total;
+            const uint32_t start = a.g_start[g], end = a.g_stop[g];
             const uint64_t key0 = a.kl.at(a.keys_sorted, start);
             uint32_t bi, bj, bk;
             L::block_of_page(a.kl.page(key0), bi, bj, bk);
@@ -1833,7 +1762,10 @@ __global__ void __launch_bounds__(GRID_NT) k_grid(StepArgs<T> a)
     __shared__ int s_msc[GRID_NT / TPB];
     if (aborted_cta(a.st)) return;
     const uint32_t B = min(a.st->n_blocks, a.b_cap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.st->max_blocks_seen = max(a.st->max_blocks_seen, B);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.st->max_blocks_seen = max(a.st->max_blocks_seen, B);
+        a.st->max_groups_seen = max(a.st->max_groups_seen, a.st->n_groups);
+    }
     const uint32_t total = B * (L::nodes / GV);
     // every thread of the CTA runs the same iterations (the loop holds barriers)
     for (uint32_t base = blockIdx.x * GRID_NT; base < total; base += gridDim.x * GRID_NT) {
@@ -1908,7 +1840,8 @@ __global__ void __launch_bounds__(GRID_NT) k_grid(StepArgs<T> a)
         }
         __syncthreads();
     }
-    // the hash table is used only by activate and P2G: clear it for the next substep
+    // the sort's counters and the hash table are used only up to P2G: clear them for the next substep
+    for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < a.sort_zero_n; h += gridDim.x * blockDim.x) a.sort_zero[h] = 0;
     for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h <= a.h_mask; h += gridDim.x * blockDim.x) a.h_keys[h] = HASH_EMPTY;
 }
 
@@ -1946,7 +1879,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
     __shared__ Material<T> s_mat[MAX_MATERIALS]; // the group's scene's materials
     __shared__ T s_st[GS::NS]; // staged state of the thread's current and next particle
     __shared__ uint32_t s_pid[GS::NP];
-    __shared__ int s_g, s_nbr[8], s_scene, s_org[3];
+    __shared__ int s_g, s_last, s_nbr[8], s_scene, s_org[3];
     __shared__ uint16_t s_map[TN]; // tile node -> (neighbour block 0-7) << 8 | element in that block
     if (aborted_cta(a.st)) return;
     if (BULK && threadIdx.x == 0) {
@@ -1965,7 +1898,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         __syncthreads();
         const int g = s_g;
         if (g >= (int)G) break;
-        const uint32_t start = a.g_start[g], end = (g + 1 < (int)G) ? a.g_start[g + 1] : a.n_total;
+        const uint32_t start = a.g_start[g], end = a.g_stop[g];
         if (threadIdx.x < 8) {
             s_nbr[threadIdx.x] = a.g_nbr[g * 8 + threadIdx.x];
             if (threadIdx.x == 0) {
@@ -2283,6 +2216,29 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         if (flags) raise_flag(a.st, flags);
         __syncthreads();
     }
+    // The last CTA to finish ends the substep: the scenes' clocks, the substep count and the work counters, unless a
+    // particle raised an aborting flag (every CTA's flags precede its arrival). As a kernel of its own this was a
+    // launch for a few words (3.5 us).
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&a.st->g2p_done, 1u) + 1 == gridDim.x;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const bool ab = aborted(a.st);
+    if (!ab)
+        for (int s = threadIdx.x; s < a.n_scenes; s += NT) a.scenes[s].time += (double)a.scenes[s].dt;
+    if (threadIdx.x == 0 && !ab) {
+        DevStatus* st = a.st;
+        st->step += 1;
+        st->n_groups = 0;
+        st->n_blocks = 0;
+        st->work_p2g = 0;
+        st->work_g2p = 0;
+        st->work_dmg = 0;
+        st->g2p_done = 0;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -2446,7 +2402,7 @@ __device__ int dmg_claim(const StepArgs<T>& a, uint32_t* counter, bool need_unfi
         const int g = *s_g;
         if (g >= (int)G) return -1;
         start = a.g_start[g];
-        end = (g + 1 < (int)G) ? a.g_start[g + 1] : a.n_total;
+        end = a.g_stop[g];
         const uint32_t sc = kl.scene(kl.at(a.keys_sorted, start));
         if (threadIdx.x == 0) *s_skip = !a.scenes[sc].implicit || (need_unfinished && a.cgs[sc].done);
         if (threadIdx.x < 8) s_nbr[threadIdx.x] = a.g_nbr[g * 8 + threadIdx.x];
@@ -2794,21 +2750,6 @@ __global__ void k_cg_scalars(StepArgs<T> a, int n_scenes, cudaGraphConditionalHa
             const uint32_t loops = ++a.st->cg_loops;
             cudaGraphSetConditional(loop, (s_active > 0 && loops <= (uint32_t)CG_MAX_ITERATIONS) ? 1u : 0u);
         }
-    }
-}
-
-template <class T>
-__global__ void k_step_end(SceneParams<T>* scenes, int n_scenes, DevStatus* st)
-{
-    if (aborted(st)) return;
-    for (int s = threadIdx.x; s < n_scenes; s += blockDim.x) scenes[s].time += (double)scenes[s].dt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        st->step += 1;
-        st->n_blocks = 0;
-        st->work_p2g = 0;
-        st->work_g2p = 0;
-        st->work_dmg = 0;
     }
 }
 
