@@ -345,7 +345,11 @@ ZR_HD bool polar_rotation(const T* F, T* R)
         for (int i = 0; i < 9; i++) R[i] = X[i];
         return false;
     }
-    polar_rotation_fp64(F, R);
+    // copies for the call: its arguments live in local memory, and F and R themselves would with them on every path
+    T Fc[9], Rc[9];
+    for (int i = 0; i < 9; i++) Fc[i] = F[i];
+    polar_rotation_fp64(Fc, Rc);
+    for (int i = 0; i < 9; i++) R[i] = Rc[i];
     return true;
 }
 
@@ -482,7 +486,11 @@ ZR_HD void givens_qr3(const T* F, T* Q, T* R)
 {
     T M[9] = { 1, 0, 0, 0, 1, 0, 0, 0, 1 }; // Q^T
     for (int i = 0; i < 9; i++) R[i] = F[i];
+    // unrolled: with indices that vary at run time the matrices live in local memory (7.6 M sectors of it per P2G of 1.07 M
+    // particles), and so do those of every caller
+#pragma unroll
     for (int j = 0; j < 3; j++)
+#pragma unroll
         for (int i = 2; i > j; i--) {
             // rotation (c -s; s c) of rows (i-1, i) with (c -s; s c) (a; b) = (r; 0) (Givens.h GivensRotation)
             const T a = R[3 * (i - 1) + j], b = R[3 * i + j];
@@ -493,6 +501,7 @@ ZR_HD void givens_qr3(const T* F, T* Q, T* R)
                 c = a * t;
                 sn = -b * t;
             }
+#pragma unroll
             for (int k = 0; k < 3; k++) {
                 const T r1 = R[3 * (i - 1) + k], r2 = R[3 * i + k];
                 R[3 * (i - 1) + k] = c * r1 - sn * r2;
@@ -545,7 +554,9 @@ ZR_HD T tau_qrnh(const Material<T>& mt, const T* F, T g, T* tau, bool effective 
     T D[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 };
     const T lam = (J >= (T)1 ? g : (T)1) * mt.lambda * (J - (T)1) * J;
     for (int i = 0; i < 3; i++) D[4 * i] += lam / R[4 * i];
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
         for (int j = i; j < 3; j++) D[3 * i + j] += g * mt.mu * R[3 * i + j];
     for (int i = 0; i < 3; i++) D[4 * i] -= g * mt.mu * J / R[4 * i];
     D[0] += kx * (R[0] - (T)1);
@@ -555,9 +566,12 @@ ZR_HD T tau_qrnh(const Material<T>& mt, const T* F, T g, T* tau, bool effective 
         D[4] += ky * (ss - (T)1) * R[4] / ss;
     }
     T A[9];
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
         for (int j = i; j < 3; j++) { // (D R^T)_ij = sum_k D_ik R_jk, D upper triangular
             T acc = 0;
+#pragma unroll
             for (int k = j; k < 3; k++) acc += D[3 * i + k] * R[3 * j + k];
             A[3 * i + j] = acc;
             A[3 * j + i] = acc;
