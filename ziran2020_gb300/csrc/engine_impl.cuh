@@ -1080,13 +1080,122 @@ struct OffsetTiles {
     static constexpr int TY = L::sy + 2, TZ = L::sz + 2;
     static constexpr int TS = L::sx * TY * TZ; // nodes of one offset's tile (per field)
     static constexpr int ELEMS = 3 * NACC * TS;
+    // tile index of cell c's first node (of any offset)
+    __device__ static __forceinline__ int corner(int c)
+    {
+        const int cx = c >> (L::zbits + L::ybits), cy = (c >> L::zbits) & (L::sy - 1), cz = c & (L::sz - 1);
+        return (cx * TY + cy) * TZ + cz;
+    }
 };
 
+// The same sums where several lanes hold pieces of one cell (see CellSplit). FP32 spreads a cell over both warps of an
+// offset, so it adds with shared-memory atomics (8.5 lane-operations per clock and SM against 15.6 for the plain form); in
+// FP64 one warp holds all cells of an offset, so the pieces of a cell take turns (`parts` of them at most) and the plain
+// form stays. Every lane of the warp must call it.
 template <class T, class L>
-__device__ __forceinline__ void add_to_offset_tile(const NodeAcc<T>& acc, T* tiles, int cx, int cy, int cz, int ii, int nf)
+__device__ __forceinline__ void add_pieces_to_offset_tile(const NodeAcc<T>& acc, T* tiles, int cell, int ii, int nf, bool used, int part, int parts)
 {
     using OT = OffsetTiles<L>;
-    T* base = tiles + ii * NACC * OT::TS + (cx * OT::TY + cy) * OT::TZ + cz;
+    T* base = tiles + ii * NACC * OT::TS + OT::corner(cell);
+    if constexpr (L::nodes > 32) {
+        (void)part;
+        (void)parts;
+        if (!used) return;
+#pragma unroll
+        for (int jj = 0; jj < 3; jj++)
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) {
+                T* t = base + jj * OT::TZ + kk;
+#pragma unroll
+                for (int f = 0; f < NACC; f++)
+                    if (f < nf) atomicAdd(t + f * OT::TS, acc.field(jj * 3 + kk, f));
+            }
+    }
+    else
+        for (int turn = 0; turn < parts; turn++) {
+#pragma unroll
+            for (int jj = 0; jj < 3; jj++)
+#pragma unroll
+                for (int kk = 0; kk < 3; kk++) {
+                    T* t = base + jj * OT::TZ + kk;
+                    if (used && part == turn) {
+#pragma unroll
+                        for (int f = 0; f < NACC; f++)
+                            if (f < nf) t[f * OT::TS] += acc.field(jj * 3 + kk, f);
+                    }
+                    __syncwarp();
+                }
+        }
+}
+
+// Work of the accumulation's (cell, x-offset) threads when a chunk's cells are crowded. A chunk of 512 particles holds 64
+// cells at 8 per cell, but 19 at 27 per cell and a handful in a dense cluster: then few threads have a cell, and the chunk
+// takes as long as its fullest one. So the cells are cut into pieces of at most R particles, one piece per thread of an
+// offset, R the smallest count that is sure to fit: sum ceil(n_c / R) <= cnt / R + cells <= NC. It pays from cells that are
+// well above both SPLIT_MIN (16: never at 8 per cell, where the slots are taken anyway) and R.
+constexpr int SPLIT_MIN = 16;
+template <class L>
+struct CellSplit {
+    static constexpr int NC = L::nodes;
+    uint16_t n[NC], first[NC]; // per cell: particles, first particle of the chunk
+    uint16_t q0[NC], q1[NC]; // per piece: its particles of the chunk
+    uint8_t cell[NC], part[NC]; // per piece: its cell (0xff: unused), its number in the cell
+    int parts; // most pieces of a cell; 0: not split
+};
+
+// Every thread of the CTA calls it, with its cell's range [qa, qb) of the chunk's cnt particles; only the threads of
+// offset 0 (first) fill the table, which is complete after the call.
+template <class L>
+__device__ __forceinline__ void split_cells(CellSplit<L>& cs, bool first, int c, int qa, int qb, int cnt, int tid)
+{
+    constexpr int NC = L::nodes, PER = NC / 32;
+    if (first) {
+        cs.n[c] = (uint16_t)(qb - qa);
+        cs.first[c] = (uint16_t)qa;
+        cs.cell[c] = 0xff;
+        cs.q0[c] = cs.q1[c] = 0;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int n[PER], cells = 0, most = 0;
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            n[k] = cs.n[tid * PER + k];
+            cells += __popc(__ballot_sync(0xffffffffu, n[k] > 0));
+            most = max(most, n[k]);
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        const int R = cells < NC ? (cnt + NC - cells - 1) / (NC - cells) : most;
+        const bool split = 2 * most > 3 * R;
+        int p = 0;
+        if (split)
+#pragma unroll
+            for (int k = 0; k < PER; k++) p += (n[k] + R - 1) / R;
+        int x = p;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (tid >= o) x += y;
+        }
+        int s = x - p;
+        if (split)
+#pragma unroll
+            for (int k = 0; k < PER; k++)
+                for (int i = 0, q = cs.first[tid * PER + k]; i * R < n[k] && s < NC; i++, s++) { // (s < NC: by the choice of R)
+                    cs.cell[s] = (uint8_t)(tid * PER + k);
+                    cs.part[s] = (uint8_t)i;
+                    cs.q0[s] = (uint16_t)(q + i * R);
+                    cs.q1[s] = (uint16_t)(q + min(n[k], (i + 1) * R));
+                }
+        if (tid == 0) cs.parts = split ? (most + R - 1) / R : 0;
+    }
+    __syncthreads();
+}
+
+template <class T, class L>
+__device__ __forceinline__ void add_to_offset_tile(const NodeAcc<T>& acc, T* tiles, int cell, int ii, int nf)
+{
+    using OT = OffsetTiles<L>;
+    T* base = tiles + ii * NACC * OT::TS + OT::corner(cell);
 #pragma unroll
     for (int jj = 0; jj < 3; jj++)
 #pragma unroll
@@ -1398,6 +1507,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
     T* pay = reinterpret_cast<T*>(fused_dyn);
     __shared__ T tile[OffsetTiles<L>::ELEMS]; // one node tile per stencil x-offset
     __shared__ uint8_t cellof[CHUNK];
+    __shared__ CellSplit<L> s_split;
     // the set-up of the current group (buffer b) and of the next one (b ^ 1): group, scene, a bad neighbour slot,
     // the grid slots of the block and its +1 neighbours, the block origin, the sorted range
     __shared__ int s_g[2], s_scene[2], s_bad[2];
@@ -1443,7 +1553,6 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         }
     };
     const int ii = tid / NC, c = tid % NC;
-    const int cx = c >> (L::zbits + L::ybits), cy = (c >> L::zbits) & (L::sy - 1), cz = c & (L::sz - 1);
     for (int q = tid; q < OffsetTiles<L>::ELEMS; q += NT) tile[q] = (T)0;
     uint32_t fallbacks = 0;
     if (tid < 32) { // the first group
@@ -1487,6 +1596,14 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             uint32_t js[PER];
 #pragma unroll
             for (int k = 0; k < PER; k++) js[k] = tid + k * NT < cnt ? a.vals_sorted[c0 + tid + k * NT] : 0u;
+            // a cell holds particles q and q + SPLIT_MIN of the chunk for some multiple q of SPLIT_MIN: the cells are crowded
+            // (a cell of 2 SPLIT_MIN particles is always found, one of fewer often)
+            static_assert(CHUNK <= 32 * SPLIT_MIN, "one warp probes the chunk");
+            bool crowded = false;
+            if (tid < 32) {
+                const uint64_t k0 = tid * SPLIT_MIN < cnt ? a.kl.at(a.keys_sorted, c0 + tid * SPLIT_MIN) : ~(uint64_t)tid;
+                crowded = __shfl_down_sync(0xffffffffu, (unsigned long long)k0, 1) == k0 && tid < 31;
+            }
 #pragma unroll
             for (int k = 0; k < PER; k++) {
                 const int q = tid + k * NT;
@@ -1498,7 +1615,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 if (!inside) raise_flag(a.st, FLAG_CAPACITY); // keys and positions disagree: abort the substep
                 cellof[q] = inside ? (uint8_t)L::element(l0, l1, l2) : (uint8_t)0xff;
             }
-            __syncthreads();
+            bool split = __syncthreads_or(crowded) != 0;
             // ---- phases 2 and 3. Particles of one cell are contiguous and the cells ascend (sorted by cell inside
             // the block): the cell's range by two binary searches over the chunk's cells, no pass or barrier of its
             // own (a position that disagreed with its key has raised FLAG_CAPACITY; the searches stay in [0, cnt])
@@ -1511,14 +1628,27 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 }
                 return lo;
             };
-            const int qa = cell_lower(c), qb = cell_lower(c + 1);
+            int qa = cell_lower(c), qb = cell_lower(c + 1);
+            if (split) { // crowded cells: pieces of them (the whole CTA decides alike)
+                split_cells<L>(s_split, ii == 0, c, qa, qb, cnt, tid);
+                split = s_split.parts > 0;
+                if (split) {
+                    qa = s_split.q0[c];
+                    qb = s_split.q1[c];
+                }
+            }
             NodeAcc<T> acc;
             acc.zero();
             if (nf == NACC)
                 for (int q = qa; q < qb; q++) accumulate_particle<T, CPAD, true>(acc, pay + (q + (q >> 3)), ii);
             else
                 for (int q = qa; q < qb; q++) accumulate_particle<T, CPAD, false>(acc, pay + (q + (q >> 3)), ii);
-            add_to_offset_tile<T, L>(acc, tile, cx, cy, cz, ii, nf); // all lanes (an empty cell adds zeros)
+            if (split) {
+                const int cell = s_split.cell[c];
+                add_pieces_to_offset_tile<T, L>(acc, tile, cell & (NC - 1), ii, nf, cell < NC, s_split.part[c], s_split.parts);
+            }
+            else
+                add_to_offset_tile<T, L>(acc, tile, c, ii, nf); // all lanes (an empty cell adds zeros)
             __syncthreads();
         }
         uint32_t n_st = 0;
@@ -1686,7 +1816,6 @@ __global__ void __launch_bounds__(WsShape<T>::NT, 2) k_p2g_ws(StepArgs<T> a)
     }
     // ---------------- consumers: cell c, stencil x-offset ii
     const int ii = tid / NC, c = tid % NC, lane = tid & 31;
-    const int cx = c >> (L::zbits + L::ybits), cy = (c >> L::zbits) & (L::sy - 1), cz = c & (L::sz - 1);
     int tb = 0; // tile buffer of the current group
     uint32_t gseq = 0; // groups flushed (parity of the flush barrier)
     for (uint32_t k = 0;; k++) {
@@ -1724,7 +1853,7 @@ __global__ void __launch_bounds__(WsShape<T>::NT, 2) k_p2g_ws(StepArgs<T> a)
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]); // the buffer is free for the producers
-        if (use) add_to_offset_tile<T, L>(acc, tiles[tb], cx, cy, cz, ii, nf); // all lanes (an empty cell adds zeros)
+        if (use) add_to_offset_tile<T, L>(acc, tiles[tb], c, ii, nf); // all lanes (an empty cell adds zeros)
         if (fl & ITEM_LAST) {
             // every consumer warp has added the group: flush its tiles (the next group fills the other tile buffer)
             __syncwarp();
