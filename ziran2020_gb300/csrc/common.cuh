@@ -123,6 +123,7 @@ struct DevStatus {
     int32_t abort_step; // substep index (counted from the last reset) that raised an aborting flag
     uint32_t step; // substeps started since the last reset
     uint32_t n_groups; // groups (occupied SPGrid blocks) of the current substep
+    uint32_t n_items; // work items (groups, or pieces of large ones) of the current substep
     uint32_t n_blocks; // active blocks (occupied + neighbours) of the current substep
     uint32_t work_p2g; // dynamic work counters of the persistent kernels
     uint32_t work_g2p;

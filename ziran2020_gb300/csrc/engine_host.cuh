@@ -830,7 +830,9 @@ private:
     uint64_t *keys_in_ = nullptr, *keys_sorted_ = nullptr;
     uint32_t *iota_ = nullptr, *vals_sorted_ = nullptr, *g_start_ = nullptr;
     int32_t* g_nbr_ = nullptr;
-    uint32_t *g_stop_ = nullptr, *g_end_ = nullptr;
+    uint4* item_ = nullptr;
+    unsigned long long* open_ = nullptr;
+    int32_t* i_slot_ = nullptr;
     uint64_t* b_key_ = nullptr;
     T *acc_ = nullptr, *vel_ = nullptr;
     uint64_t* h_keys_ = nullptr;
@@ -1160,14 +1162,18 @@ private:
         dfree(p);
         p = h_vals_;
         dfree(p);
-        p = g_stop_;
+        p = item_;
         dfree(p);
-        p = g_end_;
+        p = i_slot_;
+        dfree(p);
+        p = open_;
         dfree(p);
         p = cg_;
         dfree(p);
         cg_ = nullptr;
-        g_stop_ = g_end_ = nullptr;
+        item_ = nullptr;
+        open_ = nullptr;
+        i_slot_ = nullptr;
         g_nbr_ = nullptr;
         b_key_ = nullptr;
         acc_ = vel_ = nullptr;
@@ -1179,20 +1185,22 @@ private:
         h_mask_ = hs - 1;
         if (alloc((void**)&g_nbr_, 32 * (size_t)cap) || alloc((void**)&b_key_, 8 * (size_t)cap) || alloc((void**)&acc_, sizeof(T) * (size_t)cap * NACC * L::nodes)
             || alloc((void**)&vel_, sizeof(T) * (size_t)cap * NVEL * L::nodes) || alloc((void**)&h_keys_, 8 * (size_t)hs) || alloc((void**)&h_vals_, 4 * (size_t)hs)
-            || alloc((void**)&g_stop_, 4 * (size_t)cap) || alloc((void**)&g_end_, 4 * (size_t)hs))
+            || alloc((void**)&item_, 16 * (size_t)cap) || alloc((void**)&i_slot_, 32 * (size_t)cap) || alloc((void**)&open_, 8 * (size_t)hs))
             return ZR_ERR_CUDA_;
         ZR_CUDA(cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)cap * NACC * L::nodes, stream_));
         ZR_CUDA(cudaMemsetAsync(vel_, 0, sizeof(T) * (size_t)cap * NVEL * L::nodes, stream_));
         ZR_CUDA(cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)hs, stream_));
+        ZR_CUDA(cudaMemsetAsync(open_, 0, 8 * (size_t)hs, stream_));
         return ensure_cg();
     }
 
-    // what a substep finds zero or empty and an aborted one may leave otherwise: the grid sums, the block hash, the
-    // damage solve's vectors and the sort's counters
+    // what a substep finds zero or empty and an aborted one may leave otherwise: the grid sums, the block hash, the open
+    // group ranges, the damage solve's vectors and the sort's counters
     cudaError_t clean_substep()
     {
         cudaError_t e = cudaMemsetAsync(acc_, 0, sizeof(T) * (size_t)b_cap_ * NACC * L::nodes, stream_);
         if (e == cudaSuccess) e = cudaMemsetAsync(h_keys_, 0xff, 8 * (size_t)(h_mask_ + 1), stream_);
+        if (e == cudaSuccess) e = cudaMemsetAsync(open_, 0, 8 * (size_t)(h_mask_ + 1), stream_);
         if (e == cudaSuccess && cg_) e = cudaMemsetAsync(cg_, 0, sizeof(T) * CG_NF * (size_t)b_cap_ * L::nodes, stream_);
         if (e == cudaSuccess) e = cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_);
         return e;
@@ -1250,9 +1258,10 @@ private:
         a.pin = pool(parity);
         a.pout = pool(parity ^ 1);
         a.g_start = g_start_;
-        a.g_stop = g_stop_;
-        a.g_end = g_end_;
         a.g_nbr = g_nbr_;
+        a.item = item_;
+        a.i_slot = i_slot_;
+        a.open = open_;
         a.pay = pay_;
         a.pstride = pstride_;
         a.cg = cg_;
@@ -1783,7 +1792,7 @@ private:
         free_io();
         void* ps[] = { pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, g_nbr_, b_key_, acc_, vel_, h_keys_, h_vals_,
             d_scenes_, grid_mass_, st_, sort_tmp_, stage_, pay_, scenes_backup_, ck_pool_, ck_pid_, ck_scenes_, cg_, cgs_,
-            sort_aux_, inc_bkey_, inc_bidx_, inv_, g_stop_, g_end_ };
+            sort_aux_, inc_bkey_, inc_bidx_, inv_, item_, i_slot_, open_ };
         for (void* p : ps)
             if (p) cudaFree(p);
         pool_[0] = pool_[1] = nullptr;
@@ -1807,7 +1816,9 @@ private:
         implicit_ = false;
         sort_aux_ = nullptr;
         inc_bkey_ = inc_bidx_ = nullptr;
-        g_stop_ = g_end_ = nullptr;
+        item_ = nullptr;
+        open_ = nullptr;
+        i_slot_ = nullptr;
         inv_ = nullptr;
         inv_cap_ = 0;
         sort_base_stale_ = true;

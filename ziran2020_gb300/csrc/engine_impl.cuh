@@ -47,6 +47,8 @@ constexpr int HASH_PROBES = 64;
 // particle pool: field k of storage slot i at f[k * stride + i]
 // P_MDT: the implicit damage solve's D~ history; P_DRV: the damage drive of the particle's current F (implicit
 // scenes), kept by G2P and refilled after state writes
+template <class T>
+constexpr uint32_t P2G_CHUNK = sizeof(T) == 4 ? 512 : 256; // particles P2G stages at once: a whole block at 8 per cell
 enum { P_X = 0, P_V = 3, P_C = 6, P_F = 15, P_M = 24, P_V0 = 25, P_D = 26, P_SC = 27, P_MDT = 28, P_DRV = 29, P_NF = 30 };
 
 template <class T>
@@ -93,10 +95,11 @@ struct StepArgs {
     const uint32_t* vals_sorted;
     uint64_t* keys_next;
     Pool<T> pin, pout;
-    uint32_t* g_start; // per group: first sorted index
-    uint32_t* g_stop; // per group: one past its last sorted index (from P2G's set-up or k_nbr on)
-    uint32_t* g_end; // the same per hash position of the group's own block (from activation on)
-    int32_t* g_nbr; // per group: hash positions (from activation on), then grid slots, of its block and the +1 neighbours
+    uint32_t* g_start; // group heads after a full sort, in key order
+    int32_t* g_nbr; // per group, at its first item's number: hash positions of its block and the +1 neighbours
+    uint4* item; // work items of P2G and G2P: first sorted index, one past the last, the group's first item
+    int32_t* i_slot; // per item: grid slots of its block and the +1 neighbours (from P2G's set-up or k_nbr on)
+    unsigned long long* open; // per hash position: a group's start or end while the other comes from another tile (see range_event)
     T* pay; // P2G payload, NPAY fields of pstride elements (also the implicit damage solve's particle scratch)
     int64_t pstride;
     T* cg; // implicit damage solve: CG_NF node vectors of b_cap * nodes
@@ -392,13 +395,60 @@ __device__ __forceinline__ int32_t activate_block(const StepArgs<T>& a, uint64_t
     return done ? (int32_t)h : -1;
 }
 
+// Work items. P2G and G2P claim pieces of groups: a group of up to 5/4 of P2G's chunk is one item, a larger one is cut into
+// equal items of at most a chunk. (One CTA per group made the group of a dense cluster the end of the kernel: 100,003
+// particles in uneven blobs, P2G 107 k active cycles on the average SM and 463 k on the one with the fullest group. Items
+// below 5/4 of a chunk would give the few blocks that hold a little more than 8 per cell a second node tile to flush.)
+template <class T>
+__device__ __forceinline__ uint32_t item_parts(uint32_t count)
+{
+    constexpr uint32_t CH = P2G_CHUNK<T>;
+    return count <= CH + CH / 4 ? 1u : (count + CH - 1) / CH;
+}
+// the items of a group with sorted range [start, stop): the first at `first` (also the group's row in g_nbr), others from `rest` on
+template <class T>
+__device__ __forceinline__ void emit_items(const StepArgs<T>& a, uint32_t first, uint32_t rest, uint32_t start, uint32_t stop)
+{
+    const uint32_t n = stop - start, parts = item_parts<T>(n);
+    for (uint32_t p = 0; p < parts; p++) {
+        const uint32_t at = p ? rest + p - 1 : first;
+        if (at >= a.b_cap) { // the host grows the grid (and the item list with it) and repeats the substep
+            raise_flag(a.st, FLAG_CAPACITY);
+            return;
+        }
+        a.item[at] = make_uint4(start + (uint32_t)((uint64_t)n * p / parts), start + (uint32_t)((uint64_t)n * (p + 1) / parts), first, 0u);
+    }
+}
+// A group whose range starts in one tile and ends in another: both tiles exchange what they know into the word of the
+// group's block (hash position h): the start with the group's reserved item, or the end. The one that comes second finds the
+// other's word, makes the items and clears the word.
+constexpr unsigned long long RANGE_END = 1ull << 63;
+template <class T>
+__device__ __forceinline__ void range_event(const StepArgs<T>& a, int32_t h, unsigned long long mine)
+{
+    const unsigned long long other = atomicExch(a.open + h, mine);
+    if (other == 0) return;
+    a.open[h] = 0;
+    const unsigned long long s = (mine & RANGE_END) ? other : mine, e = (mine & RANGE_END) ? mine : other;
+    const uint32_t start = (uint32_t)s, first = (uint32_t)(s >> 32) - 1, stop = (uint32_t)e;
+    if (!(e & RANGE_END) || (s & RANGE_END) || stop <= start) {
+        check_failed(a.st, 10);
+        return;
+    }
+    const uint32_t parts = item_parts<T>(stop - start);
+    emit_items(a, first, parts > 1 ? atomicAdd(&a.st->n_items, parts - 1) : 0u, start, stop);
+}
+
 // The shared buffers of k_sort_merge's two parts overlap.
 union MergeShared {
     struct {
         uint32_t s_key[SORT_TILE], s_idx[SORT_TILE]; // the tile's stayers in storage (= key) order
         uint32_t m_key[SORT_MAXM], m_idx[SORT_MAXM], m_key2[SORT_MAXM], m_idx2[SORT_MAXM];
     } m;
-    uint32_t pos[SORT_TILE + SORT_MAXM]; // output positions of the tile's group heads, in order
+    struct {
+        uint32_t pos[SORT_TILE + SORT_MAXM]; // output positions of the tile's group heads, in order
+        uint32_t off[SORT_TILE + SORT_MAXM]; // their first items, counted from the tile's first
+    } h;
 };
 
 template <class T>
@@ -409,7 +459,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
     __shared__ uint32_t o_key[SORT_TILE + SORT_MAXM]; // the tile's output in order
     __shared__ uint32_t s_wcnt[RMAX][SORT_NT / 32];
     __shared__ uint32_t s_red[2][SORT_NT / 32];
-    __shared__ uint32_t s_ns, s_nh, s_g0;
+    __shared__ uint32_t s_ns, s_nh, s_i0;
     uint32_t *s_key = sh.m.s_key, *s_idx = sh.m.s_idx, *m_key = sh.m.m_key, *m_idx = sh.m.m_idx, *m_key2 = sh.m.m_key2, *m_idx2 = sh.m.m_idx2;
     const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     DevStatus* st = a.st;
@@ -556,40 +606,70 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
         if (lane == 0) s_wcnt[r][w] = __popc(b);
     }
     __syncthreads();
-    if (w == 0) {
-        scan_counts(R, &s_nh);
-        __syncwarp();
-        if (lane == 0) s_g0 = s_nh ? atomicAdd(&st->n_groups, s_nh) : 0u; // group numbers: as tiles come
-    }
+    if (w == 0) scan_counts(R, &s_nh);
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < RMAX; r++) {
         if (r >= R) break;
         const unsigned b = __ballot_sync(0xffffffffu, (heads >> r) & 1u);
-        if (r == 0) __syncthreads(); // (after the first ballot: every warp takes part)
-        if ((heads >> r) & 1u) sh.pos[s_wcnt[r][w] + __popc(b & ((1u << lane) - 1u))] = (uint32_t)(r * SORT_NT + tid);
+        if ((heads >> r) & 1u) sh.h.pos[s_wcnt[r][w] + __popc(b & ((1u << lane) - 1u))] = (uint32_t)(r * SORT_NT + tid);
     }
     __syncthreads();
-    if (R == 0 && j + 1 < sb.tiles) return;
-    const uint32_t nh = s_nh, g0 = s_g0;
-    // per group: its 8 blocks, its first sorted index, and the end of the group before it (known by that group's own block)
-    for (uint32_t t = tid; t < nh * 9; t += SORT_NT) {
-        const uint32_t i = t / 9, q = t - 9 * i, p = sh.pos[i], g = g0 + i;
-        if (g >= a.b_cap || g >= (uint64_t)sb.n) { // more groups than grid blocks: the host grows the grid and repeats the substep
+    const uint32_t nh = s_nh;
+    const bool last_tile = j + 1 == sb.tiles;
+    if (nh == 0 && !last_tile) return;
+    // where head i's group ends, as an output position of the tile; ~0: in a later tile
+    auto stop_of = [&](uint32_t i) { return i + 1 < nh ? sh.h.pos[i + 1] : (last_tile ? (uint32_t)cnt : ~0u); };
+    // Tasks 8 i + q: block q of head i's group (q = 0 also makes the group's items, or reports its start); the last task
+    // reports the end of the group that was open before the tile's first head, or that the particles end. The blocks go into
+    // the hash while the last warp takes the items' numbers (one reserved for the group that stays open).
+    const uint32_t tasks = 8 * nh + 1;
+    for (uint32_t u0 = 0; u0 < tasks; u0 += SORT_NT) {
+        const uint32_t t = u0 + tid, i = t >> 3, q = t & 7;
+        int32_t h = -1;
+        if (t < 8 * nh)
+            h = activate_block(a, (uint64_t)o_key[sh.h.pos[i]], q);
+        else if (t == 8 * nh && (nh ? pred != SORT_NOKEY : last_tile))
+            h = activate_block(a, (uint64_t)(nh || !cnt ? pred : o_key[cnt - 1]), 0u);
+        if (u0 == 0 && nh) {
+            if (w == SORT_NT / 32 - 1) {
+                uint32_t carry = 0;
+                for (uint32_t k0 = 0; k0 < nh; k0 += 32) {
+                    const uint32_t k = k0 + lane, stop = k < nh ? stop_of(k) : ~0u;
+                    const uint32_t n = k >= nh ? 0u : (stop != ~0u ? item_parts<T>(stop - sh.h.pos[k]) : 1u);
+                    uint32_t x = n;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                        if (lane >= o) x += y;
+                    }
+                    if (k < nh) sh.h.off[k] = carry + x - n;
+                    carry += __shfl_sync(0xffffffffu, x, 31);
+                }
+                if (lane == 0) {
+                    s_i0 = atomicAdd(&st->n_items, carry);
+                    atomicAdd(&st->n_groups, nh);
+                }
+            }
+            __syncthreads();
+        }
+        if (t > 8 * nh || h < 0) continue; // (a failed probe raised FLAG_CAPACITY)
+        if (t == 8 * nh) {
+            range_event(a, h, RANGE_END | (unsigned long long)(nh ? base + sh.h.pos[0] : sb.n));
+            continue;
+        }
+        const uint32_t first = s_i0 + sh.h.off[i];
+        if (first >= a.b_cap) { // more items than grid blocks: the host grows the grid and repeats the substep
             raise_flag(st, FLAG_CAPACITY);
             continue;
         }
-        if (q == 8 && p == 0 && pred == SORT_NOKEY) continue; // nothing before the first group
-        const uint32_t k = q < 8 ? o_key[p] : (p == 0 ? pred : o_key[p - 1]);
-        const int32_t h = activate_block(a, (uint64_t)k, q & 7);
-        if (q < 8)
-            a.g_nbr[(size_t)g * 8 + q] = h;
-        else if (h >= 0)
-            a.g_end[h] = (uint32_t)(base + p);
-        if (q == 0) a.g_start[g] = (uint32_t)(base + p);
-    }
-    if (j + 1 == sb.tiles && tid == 0) { // the last group ends with the particles
-        const int32_t h = activate_block(a, (uint64_t)(cnt ? o_key[cnt - 1] : pred), 0);
-        if (h >= 0) a.g_end[h] = (uint32_t)sb.n;
+        a.g_nbr[(size_t)first * 8 + q] = h;
+        if (q == 0) {
+            const uint32_t start = (uint32_t)base + sh.h.pos[i], stop = stop_of(i);
+            if (stop != ~0u)
+                emit_items(a, first, first + 1, start, (uint32_t)base + stop);
+            else
+                range_event(a, h, ((unsigned long long)(first + 1) << 32) | start);
+        }
     }
 }
 
@@ -673,7 +753,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* 
         }
         if (lane == 0) {
             s_prefix = prefix;
-            if ((int64_t)(j + 1) * SORT_TILE >= n) st->n_groups = (uint32_t)(prefix + run); // the last tile
+            if ((int64_t)(j + 1) * SORT_TILE >= n) st->n_groups = st->n_items = (uint32_t)(prefix + run); // the last tile
         }
     }
     __syncthreads();
@@ -689,7 +769,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* 
     }
 }
 
-// the blocks of every group (after a full sort and k_group_heads), 8 per group
+// the blocks and items of every group (after a full sort and k_group_heads), 8 threads per group
 template <class T>
 __global__ void k_activate(StepArgs<T> a)
 {
@@ -702,47 +782,37 @@ __global__ void k_activate(StepArgs<T> a)
         return;
     }
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < G * 8; t += gridDim.x * blockDim.x) {
-        const uint32_t g = t >> 3;
-        const int32_t h = activate_block(a, a.kl.at(a.keys_sorted, a.g_start[g]), t & 7);
-        a.g_nbr[t] = h;
-        if ((t & 7) == 0 && h >= 0) a.g_end[h] = g + 1 < G ? a.g_start[g + 1] : a.n_total;
+        const uint32_t g = t >> 3, start = a.g_start[g], stop = g + 1 < G ? a.g_start[g + 1] : a.n_total;
+        a.g_nbr[t] = activate_block(a, a.kl.at(a.keys_sorted, start), t & 7); // (group g's first item is g)
+        if ((t & 7) == 0) {
+            const uint32_t parts = item_parts<T>(stop - start);
+            emit_items(a, g, parts > 1 ? atomicAdd(&a.st->n_items, parts - 1) : 0u, start, stop);
+        }
     }
 }
 
 // ---------------------------------------------------------------------------------------------------
-// neighbour slots: the grid slots of every group's block and its 7 neighbours at +1 block, and the end of the group's
-// sorted range (read by P2G and G2P). Activation leaves the hash position of each of these blocks in g_nbr; the slot
-// behind it, and the range's end behind the group's own block (g_end), are final once activation has ended. The fused
-// P2G translates its groups' entries itself while it sets them up (and writes the slots and the end back for G2P, into
-// g_nbr and g_stop); the other P2G forms read those, so k_nbr translates every entry before them.
+// neighbour slots: the grid slots of every item's block and its 7 neighbours at +1 block (read by P2G and G2P).
+// Activation leaves the hash position of each of these blocks in the group's g_nbr; the slot behind it is final once
+// activation has ended. The fused P2G translates its items' entries itself while it sets them up (and writes the slots
+// back for G2P, into i_slot); the other P2G forms read those, so k_nbr translates every entry before them.
 // ---------------------------------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ int32_t nbr_slot(const StepArgs<T>& a, int32_t hpos)
 {
     return (uint32_t)hpos <= a.h_mask ? a.h_vals[hpos] : -1; // -1: the probe failed and raised FLAG_CAPACITY
 }
-// the end of the sorted range of the group that starts at `start` and whose own block has hash position hpos; an end
-// that cannot be one is a failed check and leaves one particle
-template <class T>
-__device__ __forceinline__ uint32_t group_stop(const StepArgs<T>& a, uint32_t start, int32_t hpos)
-{
-    const uint32_t en = (uint32_t)hpos <= a.h_mask ? a.g_end[hpos] : 0u;
-    if (en > start && en <= a.n_total) return en;
-    if (hpos >= 0) check_failed(a.st, 10);
-    return start + 1;
-}
 
 template <class T>
 __global__ void k_nbr(StepArgs<T> a)
 {
     if (aborted(a.st)) return;
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     if (G > a.b_cap) return; // activation already raised FLAG_CAPACITY
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < G * 8; t += gridDim.x * blockDim.x) {
-        const int32_t h = a.g_nbr[t], slot = nbr_slot(a, h);
+        const int32_t slot = nbr_slot(a, a.g_nbr[(size_t)a.item[t >> 3].z * 8 + (t & 7)]);
         if (slot < 0) raise_flag(a.st, FLAG_CAPACITY);
-        a.g_nbr[t] = slot;
-        if ((t & 7) == 0) a.g_stop[t >> 3] = group_stop(a, a.g_start[t >> 3], h);
+        a.i_slot[t] = slot;
     }
 }
 
@@ -1289,7 +1359,7 @@ __device__ void scatter_producer(const StepArgs<T>& a, unsigned char* dyn, uint6
 {
     using S = ScatterShape<T, CHUNK, NBUF>;
     constexpr int WIN = S::WIN, VEC = S::VEC;
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     uint32_t ph_empty = 3u; // parity bit per buffer; a fresh barrier counts as released
     uint32_t issues0 = 0, issues1 = 0;
     int b = 0;
@@ -1300,12 +1370,13 @@ __device__ void scatter_producer(const StepArgs<T>& a, unsigned char* dyn, uint6
         int nf = 4;
         int32_t nbr[8];
         if (g < G) {
-            qs = a.g_start[g];
-            qe = a.g_stop[g];
+            const uint4 it = a.item[g];
+            qs = it.x;
+            qe = it.y;
             nf = a.scenes[a.kl.scene(a.kl.at(a.keys_sorted, qs))].damage ? NACC : 4;
 #pragma unroll
             for (int d = 0; d < 8; d++) {
-                nbr[d] = a.g_nbr[g * 8 + d];
+                nbr[d] = a.i_slot[(size_t)g * 8 + d];
                 if (nbr[d] < 0) flags |= ITEM_BAD; // the lookup failed and raised FLAG_CAPACITY
                 else if ((uint32_t)nbr[d] >= a.b_cap) {
                     check_failed(a.st, 4);
@@ -1476,7 +1547,7 @@ __global__ void __launch_bounds__(ScatterShape<T, CHUNK, NBUF>::NT, MIN_CTAS) k_
 // round trip through HBM, at the price of the state loads' latency inside the kernel: the autotuner times
 // both forms on the workload.
 // CH: particles staged per chunk (a whole block at 8 per cell by default; half of it lets more CTAs fit)
-template <class T, int CH = (sizeof(T) == 4 ? 512 : 256)>
+template <class T, int CH = (int)P2G_CHUNK<T>>
 struct FusedShape {
     using L = typename LayoutOf<T>::type;
     static constexpr int NT = 3 * L::nodes; // cells x stencil x-offsets
@@ -1514,28 +1585,19 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
     __shared__ int32_t s_nbr[2][8];
     __shared__ int s_org[2][3];
     __shared__ uint32_t s_se[2][2];
+    __shared__ __align__(16) uint4 s_next; // the item claimed ahead
     if (aborted_cta(a.st)) return;
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     const int tid = threadIdx.x;
-    // Groups are claimed one ahead: warp 0 claims the next group at the start of a group; around the group's flush
-    // lanes 0-7 load its range and neighbour slots (lane 0 also the key of its first particle) and write them into
-    // the other buffer before the group's last barrier, so no barrier waits on a claim alone.
-    auto claim = [&]() { // warp 0 only: the next group index, in every lane
-        int v = 0;
-        if (tid == 0) v = (int)atomicAdd(&a.st->work_p2g, 1u);
-        return __shfl_sync(0xffffffffu, v, 0);
-    };
-    // A group's neighbour entries hold hash positions (activation); the set-up translates them into grid slots and
-    // writes the slots back for G2P, and the range's end likewise.
-    auto take_slot = [&](int gg, int32_t hpos) { // lanes 0-7 of warp 0
-        const int32_t slot = nbr_slot(a, hpos);
-        a.g_nbr[gg * 8 + tid] = slot;
-        return slot;
-    };
-    auto setup_store = [&](int bb, int gn, uint32_t st, int32_t hpos) { // lanes 0-7 of warp 0
+    // Items (groups or pieces of them) are claimed one ahead: thread 0 claims the next item at the start of one and copies its
+    // range into shared memory while the accumulation runs; around the flush lanes 0-7 load its block's neighbours (lane 0
+    // also the key of its first particle) and write them into the other buffer before the last barrier, so no barrier waits
+    // on a claim alone. A group's neighbour entries are hash positions; the set-up translates them into grid slots and writes
+    // those for G2P.
+    auto setup_store = [&](int bb, int gn, uint32_t st, uint32_t en, int32_t hpos) { // lanes 0-7 of warp 0
         const uint64_t key0 = tid == 0 ? a.kl.at(a.keys_sorted, st) : 0ull;
-        const uint32_t en = tid == 0 ? group_stop(a, st, hpos) : 0u;
-        const int32_t slot = take_slot(gn, hpos);
+        const int32_t slot = nbr_slot(a, hpos);
+        a.i_slot[(size_t)gn * 8 + tid] = slot;
         const unsigned badm = __ballot_sync(0xffu, slot < 0 || (uint32_t)slot >= a.b_cap); // a failed lookup raised FLAG_CAPACITY
         s_nbr[bb][tid] = slot;
         if (tid == 0) {
@@ -1549,16 +1611,17 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             s_org[bb][2] = (int)(bk * L::sz);
             s_se[bb][0] = st;
             s_se[bb][1] = en;
-            a.g_stop[gn] = en;
         }
     };
     const int ii = tid / NC, c = tid % NC;
     for (int q = tid; q < OffsetTiles<L>::ELEMS; q += NT) tile[q] = (T)0;
     uint32_t fallbacks = 0;
-    if (tid < 32) { // the first group
-        const int g0 = claim();
+    // the first item is the CTA's own number (claims count from the grid's size)
+    if (tid < 8) {
+        const int g0 = blockIdx.x;
         if (g0 < (int)G) {
-            if (tid < 8) setup_store(0, g0, a.g_start[g0], a.g_nbr[g0 * 8 + tid]);
+            const uint4 it = a.item[g0];
+            setup_store(0, g0, it.x, it.y, a.g_nbr[(size_t)it.z * 8 + tid]);
         }
         else if (tid == 0)
             s_g[0] = g0;
@@ -1568,13 +1631,14 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
     for (;;) {
         const int g = s_g[bcur];
         if (g >= (int)G) break;
-        // the next group, claimed now (its set-up is loaded around this group's flush)
-        const int gn = tid < 32 ? claim() : (int)G;
+        // the next item, claimed now (its set-up is loaded around this item's flush)
+        int claimed = 0;
+        if (tid == 0) claimed = (int)(gridDim.x + atomicAdd(&a.st->work_p2g, 1u));
         const uint32_t start = s_se[bcur][0], end = s_se[bcur][1];
         const bool bad = s_bad[bcur] != 0;
         const SceneParams<T>& sp = a.scenes[s_scene[bcur]];
         const int nf = sp.damage ? NACC : 4;
-        // The state of the group one round of claims ahead (whichever CTA takes it) is prefetched into L2 while this
+        // The state of the item one round of claims ahead (whichever CTA takes it) is prefetched into L2 while this
         // group runs, so that its phase 1 reads L2: the lanes of warp 1 take one array each (state fields P_X .. P_D
         // and the particle ids). Its storage range is that of its first and last sorted particles (storage keeps the
         // previous substep's sorted order; a range that does not look like one group is skipped). The loads are
@@ -1583,10 +1647,10 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         const int gpf = g + (int)gridDim.x, pfl = tid - 32;
         const bool pf = (a.opts & OPT_PREFETCH) && pfl >= 0 && pfl < NPF && gpf < (int)G;
         uint32_t pf_a = 0, pf_b = 0, pf_j0 = 0, pf_j1 = 0;
-        int32_t pf_h = -1;
         if (pf) {
-            pf_a = a.g_start[gpf];
-            pf_h = a.g_nbr[gpf * 8];
+            const uint4 it = a.item[gpf];
+            pf_a = it.x;
+            pf_b = it.y;
         }
         for (uint32_t c0 = start; c0 < end && !bad; c0 += CHUNK) {
             const int cnt = (int)min((uint32_t)CHUNK, end - c0);
@@ -1616,6 +1680,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 cellof[q] = inside ? (uint8_t)L::element(l0, l1, l2) : (uint8_t)0xff;
             }
             bool split = __syncthreads_or(crowded) != 0;
+            if (tid == 0 && c0 == start && claimed < (int)G) cp_async<16>(&s_next, a.item + claimed);
             // ---- phases 2 and 3. Particles of one cell are contiguous and the cells ascend (sorted by cell inside
             // the block): the cell's range by two binary searches over the chunk's cells, no pass or barrier of its
             // own (a position that disagreed with its key has raised FLAG_CAPACITY; the searches stay in [0, cnt])
@@ -1651,13 +1716,21 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 add_to_offset_tile<T, L>(acc, tile, c, ii, nf); // all lanes (an empty cell adds zeros)
             __syncthreads();
         }
-        uint32_t n_st = 0;
+        int gn = (int)G;
+        uint4 nit = make_uint4(0, 0, 0, 0);
         int32_t n_hpos = -1;
-        if (tid < 8 && gn < (int)G) {
-            n_st = a.g_start[gn];
-            n_hpos = a.g_nbr[gn * 8 + tid];
+        if (tid < 32) {
+            if (tid == 0) {
+                if (bad && claimed < (int)G) s_next = a.item[claimed];
+                cp_async_wait_all();
+            }
+            __syncwarp();
+            gn = __shfl_sync(0xffffffffu, claimed, 0);
+            if (tid < 8 && gn < (int)G) {
+                nit = s_next;
+                n_hpos = a.g_nbr[(size_t)nit.z * 8 + tid];
+            }
         }
-        if (pf && (uint32_t)pf_h <= a.h_mask) pf_b = a.g_end[pf_h]; // (a range that is none is skipped)
         if (pf && pf_b > pf_a && pf_b <= a.n_total) {
             pf_j0 = a.vals_sorted[pf_a];
             pf_j1 = a.vals_sorted[pf_b - 1];
@@ -1673,7 +1746,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
         // the next group's set-up into the other buffer (the flush above read this one)
         if (tid < 8) {
             if (gn < (int)G)
-                setup_store(bcur ^ 1, gn, n_st, n_hpos);
+                setup_store(bcur ^ 1, gn, nit.x, nit.y, n_hpos);
             else if (tid == 0)
                 s_g[bcur ^ 1] = gn;
         }
@@ -1739,14 +1812,15 @@ __global__ void __launch_bounds__(WsShape<T>::NT, 2) k_p2g_ws(StepArgs<T> a)
     }
     for (int q = tid; q < 2 * OT::ELEMS; q += S::NT) (&tiles[0][0])[q] = (T)0;
     __syncthreads(); // the last CTA-wide barrier: the roles never meet again
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     if (tid >= NCONS) {
         // ---------------- producers
         const int pt = tid - NCONS;
         uint32_t fallbacks = 0, k = 0;
         bool stop = false;
         for (uint32_t g = blockIdx.x; g < G && !stop; g += gridDim.x) {
-            const uint32_t start = a.g_start[g], end = a.g_stop[g];
+            const uint4 wit = a.item[g];
+            const uint32_t start = wit.x, end = wit.y;
             const uint64_t key0 = a.kl.at(a.keys_sorted, start);
             uint32_t bi, bj, bk;
             L::block_of_page(a.kl.page(key0), bi, bj, bk);
@@ -1768,7 +1842,7 @@ __global__ void __launch_bounds__(WsShape<T>::NT, 2) k_p2g_ws(StepArgs<T> a)
                 if (pt < 32) { // the first producer warp fills the item; a failed slot lookup raised FLAG_CAPACITY
                     int slot = 0;
                     if (pt < 8) {
-                        slot = a.g_nbr[g * 8 + pt];
+                        slot = a.i_slot[(size_t)g * 8 + pt];
                         it.nbr[pt] = slot;
                     }
                     const bool nbad = __ballot_sync(0xffffffffu, pt < 8 && (slot < 0 || (uint32_t)slot >= a.b_cap)) != 0;
@@ -2020,16 +2094,17 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         const int ax = tx >= L::sx, ay = ty >= L::sy, az = tz >= L::sz;
         s_map[node] = (uint16_t)(((ax * 4 + ay * 2 + az) << 8) | L::element(tx - ax * L::sx, ty - ay * L::sy, tz - az * L::sz));
     }
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     const KeyLayout kl = a.kl;
     for (;;) {
         if (threadIdx.x == 0) s_g = (int)atomicAdd(&a.st->work_g2p, 1u);
         __syncthreads();
         const int g = s_g;
         if (g >= (int)G) break;
-        const uint32_t start = a.g_start[g], end = a.g_stop[g];
+        const uint4 it = a.item[g];
+        const uint32_t start = it.x, end = it.y;
         if (threadIdx.x < 8) {
-            s_nbr[threadIdx.x] = a.g_nbr[g * 8 + threadIdx.x];
+            s_nbr[threadIdx.x] = a.i_slot[(size_t)g * 8 + threadIdx.x];
             if (threadIdx.x == 0) {
                 uint64_t key0 = a.kl.at(a.keys_sorted, start);
                 uint32_t bi, bj, bk;
@@ -2362,6 +2437,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         DevStatus* st = a.st;
         st->step += 1;
         st->n_groups = 0;
+        st->n_items = 0;
         st->n_blocks = 0;
         st->work_p2g = 0;
         st->work_g2p = 0;
@@ -2524,17 +2600,18 @@ __device__ int dmg_claim(const StepArgs<T>& a, uint32_t* counter, bool need_unfi
     int* s_skip)
 {
     const KeyLayout kl = a.kl;
-    const uint32_t G = a.st->n_groups;
+    const uint32_t G = a.st->n_items;
     for (;;) {
         if (threadIdx.x == 0) *s_g = (int)atomicAdd(counter, 1u);
         __syncthreads();
         const int g = *s_g;
         if (g >= (int)G) return -1;
-        start = a.g_start[g];
-        end = a.g_stop[g];
+        const uint4 it = a.item[g];
+        start = it.x;
+        end = it.y;
         const uint32_t sc = kl.scene(kl.at(a.keys_sorted, start));
         if (threadIdx.x == 0) *s_skip = !a.scenes[sc].implicit || (need_unfinished && a.cgs[sc].done);
-        if (threadIdx.x < 8) s_nbr[threadIdx.x] = a.g_nbr[g * 8 + threadIdx.x];
+        if (threadIdx.x < 8) s_nbr[threadIdx.x] = a.i_slot[(size_t)g * 8 + threadIdx.x];
         __syncthreads();
         if (!*s_skip) return (int)sc;
         __syncthreads(); // every thread has read *s_skip before thread 0 claims again
