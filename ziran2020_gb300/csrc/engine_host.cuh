@@ -150,13 +150,13 @@ public:
             pay_ = nullptr;
             sort_aux_ = nullptr;
             inc_bkey_ = inc_bidx_ = nullptr;
-            // P2G payload: NPAY fields of sorted particles at q + q/8, plus the copy granularity at the end
+            // P2G payload: Pay<T>::N fields of sorted particles at q + q/8, plus the copy granularity at the end
             pstride_ = (int64_t)((pay_pos((uint64_t)cap) + 64 + 63) & ~(uint64_t)63);
             if (alloc((void**)&keys_in_, 8 * cap) || alloc((void**)&keys_sorted_, 8 * cap) || alloc((void**)&iota_, 4 * cap)
-                || alloc((void**)&vals_sorted_, 4 * cap) || alloc((void**)&g_start_, 4 * cap) || alloc((void**)&pay_, sizeof(T) * NPAY * (size_t)pstride_)
+                || alloc((void**)&vals_sorted_, 4 * cap) || alloc((void**)&g_start_, 4 * cap) || alloc((void**)&pay_, sizeof(T) * Pay<T>::N * (size_t)pstride_)
                 || alloc((void**)&sort_aux_, sort_aux_bytes(cap)) || alloc((void**)&inc_bkey_, 4 * bucket_slots(cap)) || alloc((void**)&inc_bidx_, 4 * bucket_slots(cap)))
                 return ZR_ERR_CUDA_;
-            ZR_CUDA(cudaMemsetAsync(pay_, 0, sizeof(T) * NPAY * (size_t)pstride_, stream_));
+            ZR_CUDA(cudaMemsetAsync(pay_, 0, sizeof(T) * Pay<T>::N * (size_t)pstride_, stream_));
             ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes(cap), stream_));
             k_iota<T><<<nsm_ * 4, 256, 0, stream_>>>(iota_, (uint32_t)cap);
             size_t sb = 0, sb32 = 0;

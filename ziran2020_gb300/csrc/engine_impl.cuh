@@ -100,7 +100,7 @@ struct StepArgs {
     uint4* item; // work items of P2G and G2P: first sorted index, one past the last, the group's first item
     int32_t* i_slot; // per item: grid slots of its block and the +1 neighbours (from P2G's set-up or k_nbr on)
     unsigned long long* open; // per hash position: a group's start or end while the other comes from another tile (see range_event)
-    T* pay; // P2G payload, NPAY fields of pstride elements (also the implicit damage solve's particle scratch)
+    T* pay; // P2G payload, Pay<T>::N fields of pstride elements (also the implicit damage solve's particle scratch)
     int64_t pstride;
     T* cg; // implicit damage solve: CG_NF node vectors of b_cap * nodes
     CgScalars* cgs; // per scene
@@ -820,9 +820,9 @@ __global__ void k_nbr(StepArgs<T> a)
 // P2G, in two kernels.
 //
 // k_stress (thread per sorted particle): stress V0 tau(F, g(d)) (FBasedMpmForceHelper.cpp:43-63) and a
-// 27-value payload per particle, written in sorted order: fractional index-space position
-// f = x/dx - base, m, A = m v - dx (m C) f, Bc = dx m C, K = -dt V0 tau / dx, d, and the particle's
-// cell inside its block. With xm = (delta - f) dx for stencil offset delta,
+// payload per particle, written in sorted order: fractional index-space position f = x/dx - base (or the weights it gives),
+// m, A = m v - dx (m C) f, Bc = dx m C, K = -dt V0 tau / dx, d, and the particle's cell inside its block. With
+// xm = (delta - f) dx for stencil offset delta,
 //   m v + m C xm = A + Bc delta   and   dt f_i = K . (dw_i w_j w_k, w_i dw_j w_k, w_i w_j dw_k),
 // so a node receives m w, w (A + Bc delta) + K grad-hat w, d w and w. The force enters the momentum
 // directly (m v + dt f), which the grid update turns into v + f dt/m + g dt as the reference's
@@ -842,13 +842,23 @@ __global__ void k_nbr(StepArgs<T> a)
 // upper triangle, each off-diagonal entry the mean of the two that were computed: six fields instead of nine,
 // three shared-memory loads fewer per particle and stencil x-offset in the accumulation.
 // ---------------------------------------------------------------------------------------------------
-constexpr int NPAY = 24;
-enum { Y_F = 0, Y_M = 3, Y_A = 4, Y_B = 7, Y_K = 16, Y_D = 22, Y_CELL = 23 };
-enum { K_00 = 0, K_01 = 1, K_02 = 2, K_11 = 3, K_12 = 4, K_22 = 5 }; // offsets of the K entries from Y_K
+//
+// FP32 keeps the fractional position and evaluates the weights in each of a particle's three offset threads; FP64, whose
+// pipe is 64 times slower than the FP32 one while shared memory is not, keeps the weights themselves, and per stencil
+// z-offset k the vector Z_k = k wz_k B2 + dwz_k K2 (B2, K2: the third columns), which all of them use (accumulate_particle).
+template <class T>
+struct Pay {
+    enum { F = 0, M = 3, A = 4, B = 7, K = 16, D = 22, CELL = 23, N = 24 };
+};
+template <>
+struct Pay<double> { // WX .. WZ: 3 weights or derivatives per axis; B0, B1: the first columns; Z: 3 per z-offset
+    enum { WX = 0, DWX = 3, WY = 6, DWY = 9, WZ = 12, M = 15, A = 16, B0 = 19, B1 = 22, K = 25, Z = 30, D = 39, CELL = 40, N = 41 };
+};
+enum { K_00 = 0, K_01 = 1, K_02 = 2, K_11 = 3, K_12 = 4, K_22 = 5 }; // offsets of the K entries (FP64 keeps the first five)
 
 __host__ __device__ __forceinline__ uint64_t pay_pos(uint64_t q) { return q + (q >> 3); }
 
-// Stress and payload of one particle (storage slot j of pool P): fields Y_F..Y_D at y[f * S]; b gets the
+// Stress and payload of one particle (storage slot j of pool P): the fields of Pay<T> but CELL at y[f * S]; b gets the
 // base node. V0 tau(F) of the particle's model (FBasedMpmForceHelper.cpp:43-63) with the degradation g(d).
 template <class T, int MODELS>
 __device__ __forceinline__ void particle_payload(const Pool<T>& P, uint32_t j, const SceneParams<T>& sp, T* y, int64_t S, int (&b)[3],
@@ -893,26 +903,51 @@ __device__ __forceinline__ void particle_payload(const Pool<T>& P, uint32_t j, c
         b[e] = int_floor(sub_rn(xs, (T)0.5));
         fr[e] = xs - (T)b[e];
     }
-    const T kf = -dt * V0 * inv_dx;
+    using Y = Pay<T>;
+    const T kf = -dt * V0 * inv_dx, hk = (T)0.5 * kf;
+    const T K[6] = { kf * tau[0], hk * (tau[1] + tau[3]), hk * (tau[2] + tau[6]), kf * tau[4], hk * (tau[5] + tau[7]), kf * tau[8] };
+    y[Y::M * S] = mass;
+    y[Y::D * S] = dd;
+    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-    for (int e = 0; e < 3; e++) y[(Y_F + e) * S] = fr[e];
-    y[Y_M * S] = mass;
+        for (int e = 0; e < 3; e++) y[(Y::F + e) * S] = fr[e];
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-        const T m0 = mass * Cm[3 * r], m1 = mass * Cm[3 * r + 1], m2 = mass * Cm[3 * r + 2];
-        y[(Y_A + r) * S] = mass * v[r] - dx * (m0 * fr[0] + m1 * fr[1] + m2 * fr[2]);
-        y[(Y_B + 3 * r) * S] = dx * m0;
-        y[(Y_B + 3 * r + 1) * S] = dx * m1;
-        y[(Y_B + 3 * r + 2) * S] = dx * m2;
+        for (int r = 0; r < 3; r++) {
+            const T m0 = mass * Cm[3 * r], m1 = mass * Cm[3 * r + 1], m2 = mass * Cm[3 * r + 2];
+            y[(Y::A + r) * S] = mass * v[r] - dx * (m0 * fr[0] + m1 * fr[1] + m2 * fr[2]);
+            y[(Y::B + 3 * r) * S] = dx * m0;
+            y[(Y::B + 3 * r + 1) * S] = dx * m1;
+            y[(Y::B + 3 * r + 2) * S] = dx * m2;
+        }
+#pragma unroll
+        for (int e = 0; e < 6; e++) y[(Y::K + e) * S] = K[e];
     }
-    const T hk = (T)0.5 * kf;
-    y[(Y_K + K_00) * S] = kf * tau[0];
-    y[(Y_K + K_01) * S] = hk * (tau[1] + tau[3]);
-    y[(Y_K + K_02) * S] = hk * (tau[2] + tau[6]);
-    y[(Y_K + K_11) * S] = kf * tau[4];
-    y[(Y_K + K_12) * S] = hk * (tau[5] + tau[7]);
-    y[(Y_K + K_22) * S] = kf * tau[8];
-    y[Y_D * S] = dd;
+    else {
+        T w[3][3], dw[3][3];
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            bspline_w(fr[e], 0, w[e], dw[e]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                y[((e == 0 ? Y::WX : e == 1 ? Y::WY : Y::WZ) + k) * S] = w[e][k];
+                if (e < 2) y[((e == 0 ? Y::DWX : Y::DWY) + k) * S] = dw[e][k];
+            }
+        }
+        const T kw2 = (T)2 * w[2][2], md = mass * dx;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const T b0 = md * Cm[3 * r], b1 = md * Cm[3 * r + 1], b2 = md * Cm[3 * r + 2];
+            y[(Y::A + r) * S] = mass * v[r] - (b0 * fr[0] + b1 * fr[1] + b2 * fr[2]);
+            y[(Y::B0 + r) * S] = b0;
+            y[(Y::B1 + r) * S] = b1;
+            const T k2 = K[r == 0 ? K_02 : r == 1 ? K_12 : K_22];
+            y[(Y::Z + r) * S] = dw[2][0] * k2;
+            y[(Y::Z + 3 + r) * S] = w[2][1] * b2 + dw[2][1] * k2;
+            y[(Y::Z + 6 + r) * S] = kw2 * b2 + dw[2][2] * k2;
+        }
+#pragma unroll
+        for (int e = 0; e < 5; e++) y[(Y::K + e) * S] = K[e];
+    }
 }
 
 template <class T, int MODELS>
@@ -933,10 +968,10 @@ __global__ void __launch_bounds__(256) k_stress(StepArgs<T> a)
         const uint64_t want = (key >> kl.ib) & cmask;
         const bool ok = b[0] >= 0 && b[1] >= 0 && b[2] >= 0 && (L::offset(b[0], b[1], b[2]) >> L::data_bits) == want;
         if (!ok) flags |= FLAG_CAPACITY;
-        y[Y_CELL * S] = ok ? (T)(int)(want & (L::nodes - 1)) : (T)255;
+        y[Pay<T>::CELL * S] = ok ? (T)(int)(want & (L::nodes - 1)) : (T)255;
         if ((q & 7) == 7) { // the gap slot after every 8th particle: writing it keeps every 32-byte sector whole
 #pragma unroll
-            for (int f = 0; f < NPAY; f++) y[f * S + 1] = (T)0;
+            for (int f = 0; f < Pay<T>::N; f++) y[f * S + 1] = (T)0;
         }
     }
     if (flags) raise_flag(a.st, flags);
@@ -1019,83 +1054,112 @@ struct NodeAcc {
 
 // One particle's contribution to the 9 nodes (ii, jj, kk) of a (cell, stencil x-offset ii) thread; y points
 // at the particle's payload, fields STRIDE apart. Weights from the fractional position (BSplines.h:73-100).
-// Node (ii, jj, kk) receives, per momentum component r,
-//   wz_k al_r(j) + k wz_k be_r(j) + dwz_k ga_r(j)   with
-//   al = wx wy (A + j B1) + K0 dwx wy + K1 wx dwy,  be = wx wy B2,  ga = wx wy K2
-// Everything that does not depend on (jj, kk) is folded first, per particle and offset ii:
-//   U = wx (A + ii B0) + dwx K0,  V = wx B1,  Wk = wx K1,  X = wx B2,  Y = wx K2
-// so that al = wy_j U + j wy_j V + dwy_j Wk, be = wy_j X, ga = wy_j Y. All of it runs on pairs (two FP32 lanes
-// per instruction): (x, y) and (z, m), the mass lane carrying wx m through U and zeros elsewhere, and (d w, w).
+// Node (ii, jj, kk) receives, per momentum component,
+//   wz_k al(j) + e(j) Z_k   with   e = wx wy,   al = e (A + ii B0 + j B1) + dwx wy K0 + wx dwy K1,   Z_k = k wz_k B2 + dwz_k K2
+// so the terms that depend on k through k wz_k and dwz_k are summed once per particle (Z), not per j, and a node takes two
+// FMAs a component instead of three. What does not depend on (j, k) is folded first:
+//   U = wx (A + ii B0) + dwx K0,  V = wx B1,  Wk = wx K1,   al = wy_j U + j wy_j V + dwy_j Wk.
+// FP32 runs on pairs (two lanes per instruction): (x, y) and (z, m), and (d w, w). The mass lane has neither B nor K, so the
+// z lane's terms with them are single FMAs.
 template <class T, int STRIDE, bool DAMAGE>
 __device__ __forceinline__ void accumulate_particle(NodeAcc<T>& acc, const T* y, int ii)
 {
-    using P = typename NodeAcc<T>::P;
-    T wy[3], dwy[3], wz[3], dwz[3];
-    T wx, dwx;
-    {
-        const T d0 = y[Y_F * STRIDE];
-        const T z = (T)1.5 - d0, d1 = d0 - (T)1, zz = d0 - (T)0.5;
-        wx = ii == 0 ? (T)0.5 * z * z : (ii == 1 ? (T)0.75 - d1 * d1 : (T)0.5 * zz * zz);
-        dwx = ii == 0 ? -z : (ii == 1 ? (T)-2 * d1 : zz);
-    }
-#pragma unroll
-    for (int e = 1; e < 3; e++) {
-        const T d0 = y[(Y_F + e) * STRIDE];
-        const T z = (T)1.5 - d0, d1 = d0 - (T)1, zz = d0 - (T)0.5;
-        T* w = e == 1 ? wy : wz;
-        T* dw = e == 1 ? dwy : dwz;
-        w[0] = (T)0.5 * z * z;
-        w[1] = (T)0.75 - d1 * d1;
-        w[2] = (T)0.5 * zz * zz;
-        dw[0] = -z;
-        dw[1] = (T)-2 * d1;
-        dw[2] = zz;
-    }
-    const T mass = y[Y_M * STRIDE];
-    const T dd = DAMAGE ? y[Y_D * STRIDE] : (T)0;
-    const T fi = (T)ii;
-    const P WX = pmake<P>(wx, wx), DWX = pmake<P>(dwx, dwx), FI = pmake<P>(fi, fi);
-    // pairs of payload fields: (x, y) and (z, mass lane)
-    auto pr = [&](int f0, int f1) { return pmake<P>(y[f0 * STRIDE], y[f1 * STRIDE]); };
-    auto pz = [&](int f0) { return pmake<P>(y[f0 * STRIDE], (T)0); };
-    const P A01 = pr(Y_A, Y_A + 1), A2 = pmake<P>(y[(Y_A + 2) * STRIDE], mass);
-    // K is symmetric: column c of it is (K0c, K1c, K2c) read from the upper triangle
-    const P U01 = pfma(DWX, pr(Y_K + K_00, Y_K + K_01), pmul(WX, pfma(FI, pr(Y_B, Y_B + 3), A01)));
-    const P U2 = pfma(DWX, pz(Y_K + K_02), pmul(WX, pfma(FI, pz(Y_B + 6), A2)));
-    const P V01 = pmul(WX, pr(Y_B + 1, Y_B + 4)), V2 = pmul(WX, pz(Y_B + 7));
-    const P K01 = pmul(WX, pr(Y_K + K_01, Y_K + K_11)), K2 = pmul(WX, pz(Y_K + K_12));
-    const P X01 = pmul(WX, pr(Y_B + 2, Y_B + 5)), X2 = pmul(WX, pz(Y_B + 8));
-    const P Y01 = pmul(WX, pr(Y_K + K_02, Y_K + K_12)), Y2 = pmul(WX, pz(Y_K + K_22));
-    const P D = pmake<P>(wx * dd, wx);
-#pragma unroll
-    for (int jj = 0; jj < 3; jj++) {
-        const P WY = pmake<P>(wy[jj], wy[jj]), DWY = pmake<P>(dwy[jj], dwy[jj]);
-        P AL0 = pfma(DWY, K01, pmul(WY, U01)), AL1 = pfma(DWY, K2, pmul(WY, U2));
-        if (jj) {
-            const T jw = (T)jj * wy[jj];
-            const P JW = pmake<P>(jw, jw);
-            AL0 = pfma(JW, V01, AL0);
-            AL1 = pfma(JW, V2, AL1);
+    using Y = Pay<T>;
+    if constexpr (sizeof(T) == 4) {
+        using P = typename NodeAcc<T>::P;
+        T wy[3], dwy[3], wz[3], dwz[3];
+        T wx, dwx;
+        {
+            const T d0 = y[Y::F * STRIDE];
+            const T z = (T)1.5 - d0, d1 = d0 - (T)1, zz = d0 - (T)0.5;
+            wx = ii == 0 ? (T)0.5 * z * z : (ii == 1 ? (T)0.75 - d1 * d1 : (T)0.5 * zz * zz);
+            dwx = ii == 0 ? -z : (ii == 1 ? (T)-2 * d1 : zz);
         }
-        const P BE0 = pmul(WY, X01), BE1 = pmul(WY, X2);
-        const P GA0 = pmul(WY, Y01), GA1 = pmul(WY, Y2);
-        const P DW = pmul(WY, D);
+        bspline_w(y[(Y::F + 1) * STRIDE], 0, wy, dwy);
+        bspline_w(y[(Y::F + 2) * STRIDE], 0, wz, dwz);
+        const T mass = y[Y::M * STRIDE];
+        const T dd = DAMAGE ? y[Y::D * STRIDE] : (T)0;
+        const T fi = (T)ii;
+        const P WX = pmake<P>(wx, wx), DWX = pmake<P>(dwx, dwx), FI = pmake<P>(fi, fi);
+        auto f = [&](int k) { return y[k * STRIDE]; };
+        auto pr = [&](int f0, int f1) { return pmake<P>(y[f0 * STRIDE], y[f1 * STRIDE]); };
+        // K is symmetric: column c of it is (K0c, K1c, K2c) read from the upper triangle
+        const P U01 = pfma(DWX, pr(Y::K + K_00, Y::K + K_01), pmul(WX, pfma(FI, pr(Y::B, Y::B + 3), pr(Y::A, Y::A + 1))));
+        const P U2 = pmake<P>(dwx * f(Y::K + K_02) + wx * (fi * f(Y::B + 6) + f(Y::A + 2)), wx * mass);
+        const P V01 = pmul(WX, pr(Y::B + 1, Y::B + 4)), K01 = pmul(WX, pr(Y::K + K_01, Y::K + K_11));
+        const T V2 = wx * f(Y::B + 7), K2 = wx * f(Y::K + K_12);
+        P Z01[3];
+        T Z2[3];
+        {
+            const P b01 = pr(Y::B + 2, Y::B + 5), k01 = pr(Y::K + K_02, Y::K + K_12);
+            const T b2 = f(Y::B + 8), k2 = f(Y::K + K_22);
 #pragma unroll
-        for (int kk = 0; kk < 3; kk++) {
-            const T wk = wz[kk], dwk = dwz[kk];
-            const P W = pmake<P>(wk, wk), DWK = pmake<P>(dwk, dwk);
-            P* ac = acc.a[jj * 3 + kk];
-            ac[0] = pfma(W, AL0, ac[0]);
-            ac[1] = pfma(W, AL1, ac[1]);
-            if (kk) {
-                const T kw = (T)kk * wk;
-                const P KW = pmake<P>(kw, kw);
-                ac[0] = pfma(KW, BE0, ac[0]);
-                ac[1] = pfma(KW, BE1, ac[1]);
+            for (int kk = 0; kk < 3; kk++) {
+                Z01[kk] = pmul(pmake<P>(dwz[kk], dwz[kk]), k01);
+                Z2[kk] = dwz[kk] * k2;
+                if (kk) {
+                    const T kw = (T)kk * wz[kk];
+                    Z01[kk] = pfma(pmake<P>(kw, kw), b01, Z01[kk]);
+                    Z2[kk] = kw * b2 + Z2[kk];
+                }
             }
-            ac[0] = pfma(DWK, GA0, ac[0]);
-            ac[1] = pfma(DWK, GA1, ac[1]);
-            if (DAMAGE) ac[2] = pfma(W, DW, ac[2]);
+        }
+#pragma unroll
+        for (int jj = 0; jj < 3; jj++) {
+            const P WY = pmake<P>(wy[jj], wy[jj]), E = pmul(WY, WX);
+            P AL0 = pfma(pmake<P>(dwy[jj], dwy[jj]), K01, pmul(WY, U01)), AL1 = pmul(WY, U2);
+            AL1.x = dwy[jj] * K2 + AL1.x;
+            if (jj) {
+                const T jw = (T)jj * wy[jj];
+                AL0 = pfma(pmake<P>(jw, jw), V01, AL0);
+                AL1.x = jw * V2 + AL1.x;
+            }
+            const P DW = pmake<P>(E.x * dd, E.y);
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) {
+                const P W = pmake<P>(wz[kk], wz[kk]);
+                P* ac = acc.a[jj * 3 + kk];
+                ac[0] = pfma(W, AL0, ac[0]);
+                ac[0] = pfma(E, Z01[kk], ac[0]);
+                ac[1] = pfma(W, AL1, ac[1]);
+                ac[1].x = E.x * Z2[kk] + ac[1].x;
+                if (DAMAGE) ac[2] = pfma(W, DW, ac[2]);
+            }
+        }
+    }
+    else {
+        auto f = [&](int k) { return y[k * STRIDE]; };
+        const T wx = f(Y::WX + ii), dwx = f(Y::DWX + ii), fi = (T)ii;
+        T U[3], V[3], Wk[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            U[r] = dwx * f(Y::K + r) + wx * (fi * f(Y::B0 + r) + f(Y::A + r)); // K's first column: 00, 01, 02
+            V[r] = wx * f(Y::B1 + r);
+            Wk[r] = wx * f(Y::K + (r == 0 ? K_01 : r == 1 ? K_11 : K_12));
+        }
+        const T mass = f(Y::M), dd = DAMAGE ? f(Y::D) : (T)0;
+#pragma unroll
+        for (int jj = 0; jj < 3; jj++) {
+            const T wy = f(Y::WY + jj), dwy = f(Y::DWY + jj), e = wx * wy, em = e * mass, ed = e * dd, jw = (T)jj * wy;
+            T al[3];
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                al[r] = dwy * Wk[r] + wy * U[r];
+                if (jj) al[r] = jw * V[r] + al[r];
+            }
+#pragma unroll
+            for (int kk = 0; kk < 3; kk++) {
+                const T w = f(Y::WZ + kk);
+                auto* ac = acc.a[jj * 3 + kk];
+                ac[0].x = e * f(Y::Z + 3 * kk) + (w * al[0] + ac[0].x);
+                ac[0].y = e * f(Y::Z + 3 * kk + 1) + (w * al[1] + ac[0].y);
+                ac[1].x = e * f(Y::Z + 3 * kk + 2) + (w * al[2] + ac[1].x);
+                ac[1].y = w * em + ac[1].y;
+                if (DAMAGE) {
+                    ac[2].x = w * ed + ac[2].x;
+                    ac[2].y = w * e + ac[2].y;
+                }
+            }
         }
     }
 }
@@ -1335,7 +1399,7 @@ struct ScatterShape {
     static constexpr int NT = NCONS + 32;
     static constexpr int VEC = 16 / (int)sizeof(T); // elements per 16 bytes: copy granularity
     static constexpr int WIN = CHUNK + CHUNK / 8 + 8; // payload window per field, >= the span of CHUNK particles
-    static constexpr size_t buf_bytes = sizeof(T) * NPAY * WIN;
+    static constexpr size_t buf_bytes = sizeof(T) * Pay<T>::N * WIN;
     static constexpr size_t dyn_bytes = NBUF * buf_bytes;
     static constexpr int MIN_CTAS = sizeof(T) == 4 ? 2 : 1;
     static_assert(CHUNK % 32 == 0 && (WIN * sizeof(T)) % 16 == 0 && (NBUF == 1 || NBUF == 2), "copy alignment, buffers");
@@ -1428,8 +1492,8 @@ __device__ void scatter_producer(const StepArgs<T>& a, unsigned char* dyn, uint6
             for (int d = 0; d < 8; d++) it.nbr[d] = nbr[d];
             T* dst = reinterpret_cast<T*>(dyn + b * S::buf_bytes);
             fence_async_smem();
-            mbar_arrive_expect_tx(&full[b], bytes * NPAY);
-            for (int f = 0; f < NPAY; f++) bulk_load(dst + f * WIN, a.pay + f * a.pstride + src0, bytes, &full[b]);
+            mbar_arrive_expect_tx(&full[b], bytes * Pay<T>::N);
+            for (int f = 0; f < Pay<T>::N; f++) bulk_load(dst + f * WIN, a.pay + f * a.pstride + src0, bytes, &full[b]);
             b = NBUF == 2 ? b ^ 1 : 0;
             q0 = q1;
         } while (q0 < qe);
@@ -1498,7 +1562,7 @@ __global__ void __launch_bounds__(ScatterShape<T, CHUNK, NBUF>::NT, MIN_CTAS) k_
             if (!(fl & (ITEM_DONE | ITEM_BAD))) {
                 // runs of equal cells (particles are sorted by cell inside a block)
                 const uint32_t q1 = it.q1;
-                const T* cellv = buf + Y_CELL * WIN;
+                const T* cellv = buf + Pay<T>::CELL * WIN;
                 for (uint32_t q = q0 + tid; q < q1; q += NCONS) {
                     const int e = (int)cellv[pay_pos(q) - base];
                     if ((unsigned)e >= (unsigned)NC) continue; // 255 marks a particle whose key disagreed
@@ -1553,7 +1617,7 @@ struct FusedShape {
     static constexpr int NT = 3 * L::nodes; // cells x stencil x-offsets
     static constexpr int CHUNK = CH;
     static constexpr int CPAD = CHUNK + CHUNK / 8;
-    static constexpr size_t dyn_bytes = sizeof(T) * Y_CELL * CPAD; // fields Y_F..Y_D
+    static constexpr size_t dyn_bytes = sizeof(T) * Pay<T>::CELL * CPAD; // every field but the cell
 };
 
 // Elements [lo, hi] of one array, prefetched into L2 (widened to 16-byte boundaries, kept inside [base, end)).
@@ -1776,8 +1840,8 @@ struct WsShape {
     static constexpr int CHUNK = sizeof(T) == 4 ? 256 : 128;
     static constexpr int CPAD = CHUNK + CHUNK / 8;
     static constexpr int NSTAGE = 2;
-    static constexpr size_t pay_bytes = sizeof(T) * Y_CELL * CPAD;
-    static constexpr size_t stage_bytes = pay_bytes + CHUNK; // payload fields Y_F..Y_D, then the cells
+    static constexpr size_t pay_bytes = sizeof(T) * Pay<T>::CELL * CPAD;
+    static constexpr size_t stage_bytes = pay_bytes + CHUNK; // payload fields, then the cells
     static constexpr size_t dyn_bytes = NSTAGE * stage_bytes;
     static_assert(pay_bytes % 16 == 0 && NCONS % 32 == 0 && NPROD % 32 == 0, "whole warps, aligned buffers");
 };
