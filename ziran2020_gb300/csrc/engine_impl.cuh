@@ -2126,6 +2126,120 @@ struct G2pStage {
     static constexpr int NS = ON ? 2 * G2P_SF * NT : 1, NP = ON ? 2 * NT : 1;
 };
 
+// Sums of a particle's 27 nodes. Separable: the stencil weight is wx_i wy_j wz_k, so sums over k, then j, then i give
+//   pv = sum w v,  M_rc = sum w v_r delta_c,  Gv_rc = sum v_r (grad w)_c dx,
+// and with damage the Laplacian (below) and pw = sum w (phase field).
+// Along z the sums come from the middle node v1 and the differences e0 = v1 - v0, e1 = v2 - v1 of the line's three nodes,
+// staged beside the velocities: as sum w = 1, sum dw = 0 and w1 + 2 w2 = f (the fractional position),
+//   sum w v = v1 - w0 e0 + w2 e1,   sum dw v = -dw0 e0 + dw2 e1,   sum k w v = f v1 + 2 w2 e1,
+// six operations a component instead of eight, and the gradients are sums of differences that are already taken. FP32 runs
+// on pairs (velocity lanes (x, y) and (z, phase field)), FP64 on scalars without the phase field where there is none (DMG).
+// tv, te: the particle's corner in the staged tiles, Z1 / Z2 nodes per line.
+template <class T>
+struct Gathered {
+    T pv[3], M[9], Gv[9], lap, pw;
+};
+template <class T, class L, bool DMG>
+__device__ __forceinline__ void gather(const Quad<T>* tv, const Quad<T>* te, const T (&w)[3][3], const T (&dw)[3][3], T fz, Gathered<T>& o)
+{
+    constexpr int TY = L::sy + 2, Z1 = L::sz, Z2 = L::sz + 1;
+#pragma unroll
+    for (int r = 0; r < 3; r++) o.pv[r] = 0;
+#pragma unroll
+    for (int r = 0; r < 9; r++) o.M[r] = o.Gv[r] = 0;
+    o.lap = o.pw = 0;
+    const T nw0 = -w[2][0], w2 = w[2][2], nd0 = -dw[2][0], d2 = dw[2][2], kw2 = (T)2 * w2;
+#pragma unroll
+    for (int ii = 0; ii < 3; ii++) {
+        // per x-offset: S = sum wy s, U = sum dwy s, Tz = sum wy t, K = sum wy u, J = sum j wy s; lA, lB, lC of the phase field
+        T Si[3], Ui[3], Ti[3], Ki[3], Ji[3], lA, lB, lC;
+        if constexpr (sizeof(T) == 4) {
+            using PT = typename PairOf<T>::type;
+            const PT Z = pmake<PT>((T)0, (T)0);
+            const PT NW0 = pmake<PT>(nw0, nw0), W2 = pmake<PT>(w2, w2), ND0 = pmake<PT>(nd0, nd0), D2 = pmake<PT>(d2, d2), KW2 = pmake<PT>(kw2, kw2),
+                     FZ = pmake<PT>(fz, fz);
+            // (S_x, S_y) (S_z, lA) (U_x, U_y) (U_z, lB) (T_x, T_y) (T_z, lC) (K_x, K_y) (K_z, -) (J_x, J_y) (J_z, -)
+            PT S01 = Z, S2A = Z, U01 = Z, U2B = Z, T01 = Z, T2C = Z, K01 = Z, J01 = Z;
+            T K2 = 0, J2 = 0;
+#pragma unroll
+            for (int jj = 0; jj < 3; jj++) {
+                const Quad<T> v1 = tv[(ii * TY + jj) * Z1], e0 = te[(ii * TY + jj) * Z2], e1 = te[(ii * TY + jj) * Z2 + 1];
+                const PT v01 = pmake<PT>(v1.x, v1.y), v2f = pmake<PT>(v1.z, v1.w), a01 = pmake<PT>(e0.x, e0.y), a2f = pmake<PT>(e0.z, e0.w),
+                         b01 = pmake<PT>(e1.x, e1.y), b2f = pmake<PT>(e1.z, e1.w);
+                // (s_x, s_y) (s_z, pz) (t_x, t_y) (t_z, p1) (u_x, u_y) u_z
+                const PT s01 = pfma(W2, b01, pfma(NW0, a01, v01)), s2z = pfma(W2, b2f, pfma(NW0, a2f, v2f));
+                const PT t01 = pfma(D2, b01, pmul(ND0, a01));
+                PT t2p = pfma(pmake<PT>(d2, (T)1), b2f, pmul(pmake<PT>(nd0, (T)-1), a2f));
+                t2p.y = (T)3 * v1.w + t2p.y;
+                const PT u01 = pfma(KW2, b01, pmul(FZ, v01));
+                const T u2 = kw2 * e1.z + fz * v1.z;
+                const T wj = w[1][jj], dwj = dw[1][jj];
+                const PT WJ = pmake<PT>(wj, wj);
+                S01 = pfma(WJ, s01, S01);
+                S2A = pfma(WJ, s2z, S2A);
+                U01 = pfma(pmake<PT>(dwj, dwj), s01, U01);
+                U2B = pfma(pmake<PT>(dwj, (T)1), s2z, U2B);
+                T01 = pfma(WJ, t01, T01);
+                T2C = pfma(WJ, t2p, T2C);
+                K01 = pfma(WJ, u01, K01);
+                K2 = wj * u2 + K2;
+                if (jj) {
+                    const T jw = (T)jj * wj;
+                    J01 = pfma(pmake<PT>(jw, jw), s01, J01);
+                    J2 = jw * s2z.x + J2;
+                }
+            }
+            Si[0] = S01.x, Si[1] = S01.y, Si[2] = S2A.x;
+            Ui[0] = U01.x, Ui[1] = U01.y, Ui[2] = U2B.x;
+            Ti[0] = T01.x, Ti[1] = T01.y, Ti[2] = T2C.x;
+            Ki[0] = K01.x, Ki[1] = K01.y, Ki[2] = K2;
+            Ji[0] = J01.x, Ji[1] = J01.y, Ji[2] = J2;
+            lA = S2A.y, lB = U2B.y, lC = T2C.y;
+        }
+        else {
+            lA = lB = lC = 0;
+#pragma unroll
+            for (int jj = 0; jj < 3; jj++) {
+                const Quad<T> v1 = tv[(ii * TY + jj) * Z1], e0 = te[(ii * TY + jj) * Z2], e1 = te[(ii * TY + jj) * Z2 + 1];
+                const T v[3] = { v1.x, v1.y, v1.z }, a[3] = { e0.x, e0.y, e0.z }, b[3] = { e1.x, e1.y, e1.z };
+                const T wj = w[1][jj], dwj = dw[1][jj], jw = (T)jj * wj;
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const T sr = w2 * b[r] + (nw0 * a[r] + v[r]), tr = d2 * b[r] + nd0 * a[r], ur = kw2 * b[r] + fz * v[r];
+                    Si[r] = jj ? wj * sr + Si[r] : wj * sr;
+                    Ui[r] = jj ? dwj * sr + Ui[r] : dwj * sr;
+                    Ti[r] = jj ? wj * tr + Ti[r] : wj * tr;
+                    Ki[r] = jj ? wj * ur + Ki[r] : wj * ur;
+                    if (jj) Ji[r] = jj > 1 ? jw * sr + Ji[r] : jw * sr;
+                }
+                if (DMG) {
+                    const T ps = w2 * e1.w + (nw0 * e0.w + v1.w), p1 = (T)3 * v1.w + (e1.w - e0.w);
+                    lA = wj * ps + lA;
+                    lB += ps;
+                    lC = wj * p1 + lC;
+                }
+            }
+        }
+        const T wi = w[0][ii], dwi = dw[0][ii];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            o.pv[r] += wi * Si[r];
+            if (ii) o.M[3 * r] += ((T)ii * wi) * Si[r];
+            o.M[3 * r + 1] += wi * Ji[r];
+            o.M[3 * r + 2] += wi * Ki[r];
+            o.Gv[3 * r] += dwi * Si[r];
+            o.Gv[3 * r + 1] += wi * Ui[r];
+            o.Gv[3 * r + 2] += wi * Ti[r];
+        }
+        // the reference's 3D Laplacian weights every term with d2w(i) = (1,-2,1)(i) (MpmGrid.h:607-613):
+        // sum_jk pf * d2w_i (wy_j wz_k + wx_i wz_k + wx_i wy_j)
+        if (DMG) {
+            o.lap += (ii == 1 ? (T)-2 : (T)1) * (lA + wi * (lB + lC));
+            o.pw += wi * lA; // sum w times the node field (the damage change of an implicit solve)
+        }
+    }
+}
+
 // BULK: the 8 neighbouring blocks' velocities reach shared memory by bulk asynchronous copies (one 4-field block of
 // NVEL * nodes values per copy, completing on an mbarrier) and the node tile is built from there; otherwise each
 // thread loads its tile nodes from global memory
@@ -2142,7 +2256,10 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
     // + side of every axis, the reach of the quadratic stencil): every stencil read is a fixed offset
     constexpr int TY = L::sy + 2, TZ = L::sz + 2, TN = (L::sx + 2) * TY * TZ;
     static_assert(NVEL == 4, "one Quad per tile node");
-    __shared__ Quad<T> tq[TN]; // node-major: the 4 fields of a node in one access
+    // node-major (the 4 fields of a node in one access): the nodes that can be the middle of a z line, and the z differences
+    constexpr int Z1 = L::sz, Z2 = L::sz + 1, COLS = (L::sx + 2) * TY;
+    static_assert(TZ == 6, "five columns of six nodes per warp");
+    __shared__ Quad<T> tv[COLS * Z1], te[COLS * Z2];
     __shared__ Material<T> s_mat[MAX_MATERIALS]; // the group's scene's materials
     __shared__ T s_st[GS::NS]; // staged state of the thread's current and next particle
     __shared__ uint32_t s_pid[GS::NP];
@@ -2217,30 +2334,29 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
             }
             if (!mbar_wait(&s_hbar, hphase, WAIT_LIMIT_NS)) raise_flag(a.st, FLAG_TIMEOUT);
             hphase ^= 1u;
-            for (int node = threadIdx.x; node < TN; node += NT) {
-                const int m = s_map[node], slot = s_nbr[m >> 8];
-                const bool ok = slot >= 0 && (uint32_t)slot < a.b_cap;
-                const T* src = s_halo + (m >> 8) * BLK + (m & 0xff);
-                Quad<T> qv;
-                qv.x = ok ? src[0] : (T)0;
-                qv.y = ok ? src[L::nodes] : (T)0;
-                qv.z = ok ? src[2 * L::nodes] : (T)0;
-                qv.w = ok ? src[3 * L::nodes] : (T)0;
-                tq[node] = qv;
+        }
+        // a warp takes five z columns of six nodes; a node's upper neighbour is the next lane's
+        for (int n0 = (threadIdx.x >> 5) * 30; n0 < TN; n0 += (NT / 32) * 30) {
+            const int lane = threadIdx.x & 31, node = n0 + lane;
+            const bool in = lane < 30 && node < TN;
+            const int m = in ? s_map[node] : 0, slot = s_nbr[m >> 8];
+            const bool ok = in && slot >= 0 && (uint32_t)slot < a.b_cap;
+            const T* src = BULK ? s_halo + (m >> 8) * BLK + (m & 0xff) : a.vel + (size_t)(ok ? slot : 0) * NVEL * L::nodes + (m & 0xff);
+            Quad<T> qv, ev;
+            qv.x = ok ? src[0] : (T)0;
+            qv.y = ok ? src[L::nodes] : (T)0;
+            qv.z = ok ? src[2 * L::nodes] : (T)0;
+            qv.w = ok ? src[3 * L::nodes] : (T)0;
+            ev.x = __shfl_down_sync(0xffffffffu, qv.x, 1) - qv.x;
+            ev.y = __shfl_down_sync(0xffffffffu, qv.y, 1) - qv.y;
+            ev.z = __shfl_down_sync(0xffffffffu, qv.z, 1) - qv.z;
+            ev.w = __shfl_down_sync(0xffffffffu, qv.w, 1) - qv.w;
+            if (in) {
+                const int col = node / TZ, z = node - col * TZ;
+                if (z >= 1 && z <= Z1) tv[col * Z1 + z - 1] = qv;
+                if (z < Z2) te[col * Z2 + z] = ev;
             }
         }
-        else
-            for (int node = threadIdx.x; node < TN; node += NT) {
-                const int m = s_map[node], slot = s_nbr[m >> 8];
-                const bool ok = slot >= 0 && (uint32_t)slot < a.b_cap;
-                const T* src = a.vel + (size_t)(ok ? slot : 0) * NVEL * L::nodes + (m & 0xff);
-                Quad<T> qv;
-                qv.x = ok ? src[0] : (T)0;
-                qv.y = ok ? src[L::nodes] : (T)0;
-                qv.z = ok ? src[2 * L::nodes] : (T)0;
-                qv.w = ok ? src[3 * L::nodes] : (T)0;
-                tq[node] = qv;
-            }
         {
             constexpr int MW = (int)(sizeof(Material<T>) / 4);
             const uint32_t* ms = reinterpret_cast<const uint32_t*>(sp.materials);
@@ -2305,77 +2421,17 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
                 flags |= FLAG_CAPACITY; // a particle outside its group's block: keys and positions disagree
                 continue;
             }
-            // Separable gather: the stencil weight is wx_i wy_j wz_k, so sums over k, then j, then i give
-            //   pv = sum w v,  M_rc = sum w v_r delta_c,  G_rc = sum v_r (grad w)_c dx,
-            // and the APIC moment sum w v (x_i - x_p)^T = dx (M - pv fr^T) because x_i - x_p = (delta - fr) dx.
-            T pv[3] = { 0, 0, 0 }, M[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 }, Gv[9] = { 0, 0, 0, 0, 0, 0, 0, 0, 0 }, lap = 0, pw = 0;
-            const Quad<T>* nq0 = tq + (l[0] * TY + l[1]) * TZ + l[2];
-            // the z and y sums run on pairs (two fields per instruction): velocity lanes (x, y) and (z, phase field)
-            using PT = typename PairOf<T>::type;
-            const PT Z = pmake<PT>((T)0, (T)0);
-#pragma unroll
-            for (int ii = 0; ii < 3; ii++) {
-                // (S_x, S_y) (S_z, lA) (U_x, U_y) (U_z, lB) (T_x, T_y) (T_z, lC) (K_x, K_y) (K_z, -) (J_x, J_y) (J_z, -)
-                PT S01 = Z, S2A = Z, U01 = Z, U2B = Z, T01 = Z, T2C = Z, K01 = Z, K2 = Z, J01 = Z, J2 = Z;
-#pragma unroll
-                for (int jj = 0; jj < 3; jj++) {
-                    // (s_x, s_y) (s_z, pz) (t_x, t_y) (t_z, p1) (u_x, u_y) (u_z, -)
-                    PT s01 = Z, s2z = Z, t01 = Z, t2p = Z, u01 = Z, u2 = Z;
-#pragma unroll
-                    for (int kk = 0; kk < 3; kk++) {
-                        const Quad<T> nv = nq0[(ii * TY + jj) * TZ + kk];
-                        const T wk = w[2][kk], dwk = dw[2][kk];
-                        const PT v01 = pmake<PT>(nv.x, nv.y), v2f = pmake<PT>(nv.z, damage ? nv.w : (T)0);
-                        const PT W = pmake<PT>(wk, wk);
-                        s01 = pfma(W, v01, s01);
-                        s2z = pfma(W, v2f, s2z);
-                        t01 = pfma(pmake<PT>(dwk, dwk), v01, t01);
-                        t2p = pfma(pmake<PT>(dwk, (T)1), v2f, t2p);
-                        if (kk) {
-                            const T kw = (T)kk * wk;
-                            const PT KW = pmake<PT>(kw, kw);
-                            u01 = pfma(KW, v01, u01);
-                            u2 = pfma(KW, v2f, u2);
-                        }
-                    }
-                    const T wj = w[1][jj], dwj = dw[1][jj];
-                    const PT WJ = pmake<PT>(wj, wj);
-                    S01 = pfma(WJ, s01, S01);
-                    S2A = pfma(WJ, s2z, S2A);
-                    U01 = pfma(pmake<PT>(dwj, dwj), s01, U01);
-                    U2B = pfma(pmake<PT>(dwj, (T)1), s2z, U2B);
-                    T01 = pfma(WJ, t01, T01);
-                    T2C = pfma(WJ, t2p, T2C);
-                    K01 = pfma(WJ, u01, K01);
-                    K2 = pfma(WJ, u2, K2);
-                    if (jj) {
-                        const T jw = (T)jj * wj;
-                        const PT JW = pmake<PT>(jw, jw);
-                        J01 = pfma(JW, s01, J01);
-                        J2 = pfma(JW, s2z, J2);
-                    }
-                }
-                const T Si[3] = { S01.x, S01.y, S2A.x }, Ui[3] = { U01.x, U01.y, U2B.x }, Ti[3] = { T01.x, T01.y, T2C.x };
-                const T Ki[3] = { K01.x, K01.y, K2.x }, Ji[3] = { J01.x, J01.y, J2.x };
-                const T lA = S2A.y, lB = U2B.y, lC = T2C.y;
-                const T wi = w[0][ii], dwi = dw[0][ii];
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    pv[r] += wi * Si[r];
-                    if (ii) M[3 * r] += ((T)ii * wi) * Si[r];
-                    M[3 * r + 1] += wi * Ji[r];
-                    M[3 * r + 2] += wi * Ki[r];
-                    Gv[3 * r] += dwi * Si[r];
-                    Gv[3 * r + 1] += wi * Ui[r];
-                    Gv[3 * r + 2] += wi * Ti[r];
-                }
-                // the reference's 3D Laplacian weights every term with d2w(i) = (1,-2,1)(i) (MpmGrid.h:607-613):
-                // sum_jk pf * d2w_i (wy_j wz_k + wx_i wz_k + wx_i wy_j)
-                if (damage) {
-                    lap += (ii == 1 ? (T)-2 : (T)1) * (lA + wi * (lB + lC));
-                    pw += wi * lA; // sum w times the node field (the damage change of an implicit solve)
-                }
+            // the APIC moment sum w v (x_i - x_p)^T = dx (M - pv fr^T) because x_i - x_p = (delta - fr) dx
+            Gathered<T> gt;
+            {
+                const int col = l[0] * TY + l[1];
+                const Quad<T>*pv0 = tv + col * Z1 + l[2], *pe0 = te + col * Z2 + l[2];
+                if (sizeof(T) == 4 || damage) // FP32 carries the phase field in the fourth lane anyway (zero without damage)
+                    gather<T, L, true>(pv0, pe0, w, dw, fr[2], gt);
+                else
+                    gather<T, L, false>(pv0, pe0, w, dw, fr[2], gt);
             }
+            T (&pv)[3] = gt.pv, (&M)[9] = gt.M, (&Gv)[9] = gt.Gv, &lap = gt.lap, &pw = gt.pw;
             lap *= inv_dx * inv_dx;
             T Bm[9];
 #pragma unroll
