@@ -145,6 +145,25 @@ ZR_HD double rcbrt_(double x)
 #endif
 }
 
+ZR_HD void sincos_(float x, float& s, float& c)
+{
+#if defined(__CUDA_ARCH__)
+    sincosf(x, &s, &c);
+#else
+    s = std::sin(x);
+    c = std::cos(x);
+#endif
+}
+ZR_HD void sincos_(double x, double& s, double& c)
+{
+#if defined(__CUDA_ARCH__)
+    sincos(x, &s, &c);
+#else
+    s = std::sin(x);
+    c = std::cos(x);
+#endif
+}
+
 // ------------------------------------------------------------------------------------------------
 // Robust FP64 SVD by one-sided (Hestenes) Jacobi, with Ziran's sign convention: U and V proper
 // rotations, |s0| >= |s1| >= |s2|, only s2 may be negative (ImplicitQRSVD.h:455-460 contract).
@@ -300,6 +319,13 @@ __device__ __forceinline__ float newton_step<float>(float* X, float* Cf, float a
 }
 #endif
 
+ZR_HD float newton_scale(float J) { return rcbrt_(J); }
+ZR_HD double newton_scale(double J)
+{
+    // det F within the condition bound, but beyond FP32's range: the FP64 root
+    return J > 1e-30 && J < 1e30 ? (double)rcbrt_((float)J) : rcbrt_(J);
+}
+
 // The FP64 path of polar_rotation, kept out of line: it is rare, and inlining it into every kernel that
 // decomposes F would crowd the instruction cache of the hot loops.
 template <class T>
@@ -329,7 +355,8 @@ ZR_HD bool polar_rotation(const T* F, T* R)
         // Frobenius condition number ||F|| ||F^-1|| = sqrt(nf nc) / J
         if (J > 0 && nf * nc < (Eps<T>::polar_kappa * Eps<T>::polar_kappa) * (J * J)) {
             for (int it = 0; it < Eps<T>::polar_iters; it++) {
-                T g = rcbrt_(J);
+                // the scaling only speeds convergence up, so FP64 takes it from FP32 (any g that enters both terms alike serves)
+                const T g = newton_scale(J);
                 T a = (T)0.5 * g, b = (T)0.5 / (g * J);
                 const T diff = newton_step(X, Cf, a, b);
                 if (diff < Eps<T>::polar_tol * Eps<T>::polar_tol) {
@@ -414,8 +441,11 @@ ZR_HD void tension_part(const T* S, T* Sp)
         T r = (T)0.5 * (B00 * (B11 * B22 - B12 * B12) - B01 * (B01 * B22 - B12 * B02) + B02 * (B01 * B12 - B11 * B02));
         r = r < (T)-1 ? (T)-1 : (r > (T)1 ? (T)1 : r);
         const T phi = acos(r) * ((T)1 / (T)3);
-        l1 = q + (T)2 * p * cos(phi);
-        l3 = q + (T)2 * p * cos(phi + (T)2.0943951023931954923);
+        // cos(phi + 2 pi / 3) = -cos(phi) / 2 - sqrt(3) / 2 sin(phi)
+        T sphi, cphi;
+        sincos_(phi, sphi, cphi);
+        l1 = q + (T)2 * p * cphi;
+        l3 = q - p * (cphi + (T)1.7320508075688772935 * sphi);
         l2 = (T)3 * q - l1 - l3;
     }
     if (l3 >= (T)0) { // all tensile
@@ -461,19 +491,25 @@ ZR_HD bool tau_corotated(const Material<T>& mt, const T* F, T* tau)
 // Neo-Hookean (Borden): tau = g (tau_dev + tau_vol) for J >= 1, g tau_dev + tau_vol otherwise
 // (NeoHookeanBorden.cpp:71-94); kappa = 0.666666 mu + lambda (NeoHookeanBorden.cpp:20)
 template <class T>
-ZR_HD void tau_nhb(const Material<T>& mt, const T* F, T g, T* tau)
+ZR_HD T tau_nhb(const Material<T>& mt, const T* F, T g, T* tau) // returns J
 {
-    T B[9];
-    mul3_bt(F, F, B);
+    // B = F F^T is symmetric: six entries
+    const T b00 = F[0] * F[0] + F[1] * F[1] + F[2] * F[2], b11 = F[3] * F[3] + F[4] * F[4] + F[5] * F[5], b22 = F[6] * F[6] + F[7] * F[7] + F[8] * F[8];
+    const T b01 = F[0] * F[3] + F[1] * F[4] + F[2] * F[5], b02 = F[0] * F[6] + F[1] * F[7] + F[2] * F[8], b12 = F[3] * F[6] + F[4] * F[7] + F[5] * F[8];
     T J = det3(F);
-    T tr3 = (B[0] + B[4] + B[8]) * ((T)1 / (T)3);
+    T tr3 = (b00 + b11 + b22) * ((T)1 / (T)3);
     T rc = rcbrt_(J);
     T s = J > (T)0 ? mt.mu * (rc * rc) : (T)NAN; // mu J^{-2/3}; pow() of a negative J is NaN in the reference too
-    T vol = J * (mt.kappa * (T)0.5 * (J - (T)1 / J));
+    T vol = mt.kappa * (T)0.5 * ((J - (T)1) * (J + (T)1)); // J (kappa/2 (J - 1/J)) without the division
     bool tension = J >= (T)1;
     T gd = g * s, gv = tension ? g * vol : vol;
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) tau[3 * r + c] = gd * (B[3 * r + c] - (r == c ? tr3 : (T)0)) + (r == c ? gv : (T)0);
+    tau[0] = gd * (b00 - tr3) + gv;
+    tau[4] = gd * (b11 - tr3) + gv;
+    tau[8] = gd * (b22 - tr3) + gv;
+    tau[1] = tau[3] = gd * b01;
+    tau[2] = tau[6] = gd * b02;
+    tau[5] = tau[7] = gd * b12;
+    return J;
 }
 
 // Givens QR of a 3x3 matrix, F = Q R, with Ziran's rotation order (GivensQR.h: for each column j, rows
@@ -610,8 +646,7 @@ ZR_HD T damage_drive(const Material<T>& mt, const T* F, T sigma_c, bool& fallbac
     }
     else {
         const T Ft[9] = { F[0], F[3], F[6], F[1], F[4], F[7], F[2], F[5], F[8] };
-        tau_nhb(mt, Ft, (T)1, tau); // tau~ = R^T tau R: the formula on F^T F
-        invJ = (T)1 / det3(F);
+        invJ = (T)1 / tau_nhb(mt, Ft, (T)1, tau); // tau~ = R^T tau R: the formula on F^T F
     }
     T S[9], sp[9], s2 = 0;
     for (int i = 0; i < 9; i++) {
