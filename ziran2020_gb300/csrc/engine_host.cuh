@@ -1260,6 +1260,7 @@ private:
         a.g_start = g_start_;
         a.g_nbr = g_nbr_;
         a.item = item_;
+        a.item_max = item_size();
         a.i_slot = i_slot_;
         a.open = open_;
         a.pay = pay_;
@@ -1283,6 +1284,18 @@ private:
         a.opts = prefetch_ ? OPT_PREFETCH : 0u;
         a.kl = kl_;
         return a;
+    }
+
+    // Particles of a P2G / G2P item: a chunk (a whole block at 8 per cell), less where that leaves SMs idle: down to 128 in
+    // FP32 where it gives fewer than two items per SM (more are taken up by two or three CTAs at once; items of 64 pay for
+    // more node tiles than they save), down to 64 in FP64, bound by its pipe, where it gives fewer than four. Per substep with
+    // 512 (256 in FP64) against this rule: FP32 4,096 particles 48.2 / 40.0 us, 32,768 53.1 / 47.3 us (64: 58.2), 106,496
+    // 60.9 / 59.6 (four items per SM: 70.1); FP64 P2G + G2P 4,096 particles 210 / 84 us, 32,768 277 / 215, 52,224 359 / 310.
+    uint32_t item_size() const
+    {
+        const uint32_t per_sm = sizeof(T) == 4 ? 2 : 4, least = sizeof(T) == 4 ? 128 : 64;
+        const uint32_t even = (N_ / (per_sm * (uint32_t)nsm_) + 31) / 32 * 32;
+        return std::min<uint32_t>(P2G_CHUNK<T>, std::max<uint32_t>(least, even));
     }
 
     // Enqueue one substep reading buffer `parity`. With ev != nullptr, events are recorded between the

@@ -98,6 +98,7 @@ struct StepArgs {
     uint32_t* g_start; // group heads after a full sort, in key order
     int32_t* g_nbr; // per group, at its first item's number: hash positions of its block and the +1 neighbours
     uint4* item; // work items of P2G and G2P: first sorted index, one past the last, the group's first item
+    uint32_t item_max; // particles of an item (a group of up to 5/4 of it stays whole)
     int32_t* i_slot; // per item: grid slots of its block and the +1 neighbours (from P2G's set-up or k_nbr on)
     unsigned long long* open; // per hash position: a group's start or end while the other comes from another tile (see range_event)
     T* pay; // P2G payload, Pay<T>::N fields of pstride elements (also the implicit damage solve's particle scratch)
@@ -399,17 +400,16 @@ __device__ __forceinline__ int32_t activate_block(const StepArgs<T>& a, uint64_t
 // equal items of at most a chunk. (One CTA per group made the group of a dense cluster the end of the kernel: 100,003
 // particles in uneven blobs, P2G 107 k active cycles on the average SM and 463 k on the one with the fullest group. Items
 // below 5/4 of a chunk would give the few blocks that hold a little more than 8 per cell a second node tile to flush.)
-template <class T>
-__device__ __forceinline__ uint32_t item_parts(uint32_t count)
+// Scenes too small for four items per SM at that size get smaller ones (item_max, see the host's item_size).
+__device__ __forceinline__ uint32_t item_parts(uint32_t item_max, uint32_t count)
 {
-    constexpr uint32_t CH = P2G_CHUNK<T>;
-    return count <= CH + CH / 4 ? 1u : (count + CH - 1) / CH;
+    return count <= item_max + item_max / 4 ? 1u : (count + item_max - 1) / item_max;
 }
 // the items of a group with sorted range [start, stop): the first at `first` (also the group's row in g_nbr), others from `rest` on
 template <class T>
 __device__ __forceinline__ void emit_items(const StepArgs<T>& a, uint32_t first, uint32_t rest, uint32_t start, uint32_t stop)
 {
-    const uint32_t n = stop - start, parts = item_parts<T>(n);
+    const uint32_t n = stop - start, parts = item_parts(a.item_max, n);
     for (uint32_t p = 0; p < parts; p++) {
         const uint32_t at = p ? rest + p - 1 : first;
         if (at >= a.b_cap) { // the host grows the grid (and the item list with it) and repeats the substep
@@ -435,7 +435,7 @@ __device__ __forceinline__ void range_event(const StepArgs<T>& a, int32_t h, uns
         check_failed(a.st, 10);
         return;
     }
-    const uint32_t parts = item_parts<T>(stop - start);
+    const uint32_t parts = item_parts(a.item_max, stop - start);
     emit_items(a, first, parts > 1 ? atomicAdd(&a.st->n_items, parts - 1) : 0u, start, stop);
 }
 
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
                 uint32_t carry = 0;
                 for (uint32_t k0 = 0; k0 < nh; k0 += 32) {
                     const uint32_t k = k0 + lane, stop = k < nh ? stop_of(k) : ~0u;
-                    const uint32_t n = k >= nh ? 0u : (stop != ~0u ? item_parts<T>(stop - sh.h.pos[k]) : 1u);
+                    const uint32_t n = k >= nh ? 0u : (stop != ~0u ? item_parts(a.item_max, stop - sh.h.pos[k]) : 1u);
                     uint32_t x = n;
                     for (int o = 1; o < 32; o <<= 1) {
                         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -785,7 +785,7 @@ __global__ void k_activate(StepArgs<T> a)
         const uint32_t g = t >> 3, start = a.g_start[g], stop = g + 1 < G ? a.g_start[g + 1] : a.n_total;
         a.g_nbr[t] = activate_block(a, a.kl.at(a.keys_sorted, start), t & 7); // (group g's first item is g)
         if ((t & 7) == 0) {
-            const uint32_t parts = item_parts<T>(stop - start);
+            const uint32_t parts = item_parts(a.item_max, stop - start);
             emit_items(a, g, parts > 1 ? atomicAdd(&a.st->n_items, parts - 1) : 0u, start, stop);
         }
     }
@@ -1262,11 +1262,14 @@ __device__ __forceinline__ void add_pieces_to_offset_tile(const NodeAcc<T>& acc,
         }
 }
 
-// Work of the accumulation's (cell, x-offset) threads when a chunk's cells are crowded. A chunk of 512 particles holds 64
-// cells at 8 per cell, but 19 at 27 per cell and a handful in a dense cluster: then few threads have a cell, and the chunk
-// takes as long as its fullest one. So the cells are cut into pieces of at most R particles, one piece per thread of an
-// offset, R the smallest count that is sure to fit: sum ceil(n_c / R) <= cnt / R + cells <= NC. It pays from cells that are
-// well above both SPLIT_MIN (16: never at 8 per cell, where the slots are taken anyway) and R.
+// Work of the accumulation's (cell, x-offset) threads where cells hold unequal numbers of particles. A chunk takes as long as
+// its fullest cell, and a cell without particles leaves its threads idle: so the cells are cut into pieces of at most R
+// particles, one piece per thread of an offset, R the smallest count for which the pieces fit.
+// FP32 does so where cells are crowded: a chunk of 512 particles holds 64 cells at 8 per cell, but 19 at 27 per cell and a
+// handful in a dense cluster. It pays from cells well above both SPLIT_MIN (16: at 8 per cell the threads are taken anyway)
+// and R. FP64 does so in every chunk: there an instruction occupies the FP64 pipe for 16 clocks whatever its active lanes, and
+// on the 425,984-particle slab (a warp's 32 cells hold 5.8 particles on average, the fullest about 12) 61% of the lanes the
+// pipe was issued were active.
 constexpr int SPLIT_MIN = 16;
 template <class L>
 struct CellSplit {
@@ -1299,12 +1302,17 @@ __device__ __forceinline__ void split_cells(CellSplit<L>& cs, bool first, int c,
             most = max(most, n[k]);
         }
         most = __reduce_max_sync(0xffffffffu, most);
-        const int R = cells < NC ? (cnt + NC - cells - 1) / (NC - cells) : most;
-        const bool split = 2 * most > 3 * R;
-        int p = 0;
-        if (split)
+        int R = (cnt + NC - 1) / NC, p = 0;
+        for (; cells > 0; R++) { // (R = most always fits: at most one piece per cell)
+            p = 0;
 #pragma unroll
             for (int k = 0; k < PER; k++) p += (n[k] + R - 1) / R;
+            if (__reduce_add_sync(0xffffffffu, p) <= NC) break;
+        }
+        // FP64's pieces of a cell take turns in the tile, a turn costs about half a particle's accumulation
+        const int parts = cells ? (most + R - 1) / R : 1;
+        const bool split = PER > 1 ? 2 * most > 3 * R : 2 * most > 2 * R + parts - 1;
+        if (!split) p = 0;
         int x = p;
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1320,7 +1328,7 @@ __device__ __forceinline__ void split_cells(CellSplit<L>& cs, bool first, int c,
                     cs.q0[s] = (uint16_t)(q + i * R);
                     cs.q1[s] = (uint16_t)(q + min(n[k], (i + 1) * R));
                 }
-        if (tid == 0) cs.parts = split ? (most + R - 1) / R : 0;
+        if (tid == 0) cs.parts = split ? parts : 0;
     }
     __syncthreads();
 }
@@ -1727,8 +1735,8 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             // a cell holds particles q and q + SPLIT_MIN of the chunk for some multiple q of SPLIT_MIN: the cells are crowded
             // (a cell of 2 SPLIT_MIN particles is always found, one of fewer often)
             static_assert(CHUNK <= 32 * SPLIT_MIN, "one warp probes the chunk");
-            bool crowded = false;
-            if (tid < 32) {
+            bool crowded = sizeof(T) == 8;
+            if (sizeof(T) == 4 && tid < 32) {
                 const uint64_t k0 = tid * SPLIT_MIN < cnt ? a.kl.at(a.keys_sorted, c0 + tid * SPLIT_MIN) : ~(uint64_t)tid;
                 crowded = __shfl_down_sync(0xffffffffu, (unsigned long long)k0, 1) == k0 && tid < 31;
             }
@@ -2126,6 +2134,10 @@ struct G2pStage {
     static constexpr int NS = ON ? 2 * G2P_SF * NT : 1, NP = ON ? 2 * NT : 1;
 };
 
+// infinity or NaN; FP64 looks at the exponent bits, as a comparison would occupy the FP64 pipe
+__device__ __forceinline__ bool nonfinite(float x) { return !isfinite(x); }
+__device__ __forceinline__ bool nonfinite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+
 // Sums of a particle's 27 nodes. Separable: the stencil weight is wx_i wy_j wz_k, so sums over k, then j, then i give
 //   pv = sum w v,  M_rc = sum w v_r delta_c,  Gv_rc = sum v_r (grad w)_c dx,
 // and with damage the Laplacian (below) and pw = sum w (phase field).
@@ -2365,8 +2377,8 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         }
         if (GS::ON && i0 < end) stage(0, j_cur);
         __syncthreads();
-        const T dx = sp.dx, inv_dx = sp.inv_dx, dt = sp.dt, D_inv = sp.D_inv;
-        const T ca = sp.apic_a, cb = sp.apic_b;
+        const T dx = sp.dx, inv_dx = sp.inv_dx, dt = sp.dt;
+        const T caD = sp.apic_a * dx * sp.D_inv, cbD = sp.apic_b * dx * sp.D_inv, gdt = dt * inv_dx;
         const T dx2 = dx * dx, half_cfl2 = dx2 * (T)0.25 * (sp.cfl * sp.cfl);
         // scene constants in registers: read through sp inside the loop they would be re-read after every store
         const int key_cells = sp.domain_cells - 3, n_mat = sp.n_materials;
@@ -2433,35 +2445,32 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
             }
             T (&pv)[3] = gt.pv, (&M)[9] = gt.M, (&Gv)[9] = gt.Gv, &lap = gt.lap, &pw = gt.pw;
             lap *= inv_dx * inv_dx;
-            T Bm[9];
+            T Bm[9]; // the moment over dx; the factors dx and 4 / dx^2 are in caD and cbD, dt / dx in gdt
 #pragma unroll
             for (int r = 0; r < 3; r++)
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    Bm[3 * r + c] = dx * (M[3 * r + c] - fr[c] * pv[r]);
-                    Gv[3 * r + c] *= inv_dx;
-                }
+                for (int c = 0; c < 3; c++) Bm[3 * r + c] = M[3 * r + c] - fr[c] * pv[r];
             // finish the transfer first so the gather accumulators die before the damage update
             {
                 T Fn[9], A[9];
+                bool bad = false;
 #pragma unroll
                 for (int r = 0; r < 3; r++)
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
-                        const T cn = (ca * Bm[3 * r + c] + cb * Bm[3 * c + r]) * D_inv;
+                        const T cn = caD * Bm[3 * r + c] + cbD * Bm[3 * c + r];
                         Q.f[(P_C + 3 * r + c) * Q.stride + i] = cn;
-                        if (!isfinite(cn)) flags |= FLAG_NONFINITE;
-                        A[3 * r + c] = (r == c ? (T)1 : (T)0) + dt * Gv[3 * r + c];
+                        bad = bad || nonfinite(cn);
+                        A[3 * r + c] = (r == c ? (T)1 : (T)0) + gdt * Gv[3 * r + c];
                     }
                 if constexpr (GS::ON) {
 #pragma unroll
                     for (int c = 0; c < 9; c++) F[c] = dsl[(GS_F + c) * NT];
                 }
                 mul3(A, F, Fn);
-                bool finite = true;
 #pragma unroll
                 for (int c = 0; c < 9; c++) {
-                    finite = finite && isfinite(Fn[c]);
+                    bad = bad || nonfinite(Fn[c]);
                     Q.f[(P_F + c) * Q.stride + i] = Fn[c];
                 }
                 T xn[3], inc2 = 0;
@@ -2475,7 +2484,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
                 }
                 if (inc2 > dx2) flags |= FLAG_CFL;
                 if (inc2 > half_cfl2) flags |= FLAG_CFL_HALF;
-                if (!finite || !isfinite(inc2)) flags |= FLAG_NONFINITE;
+                if (bad || nonfinite(inc2)) flags |= FLAG_NONFINITE;
                 // key of the next substep
                 int nb[3];
                 bool in_dom = true;
@@ -2531,7 +2540,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
                         dd = damage_update(mt, F, dd, lap, sc, dt, fb);
                         if (fb) atomicAdd(&a.st->fallback, 1u);
                     }
-                    if (!isfinite(dd)) flags |= FLAG_NONFINITE;
+                    if (nonfinite(dd)) flags |= FLAG_NONFINITE;
                 }
                 Q.f[P_D * Q.stride + i] = dd;
                 Q.f[P_SC * Q.stride + i] = sc;
