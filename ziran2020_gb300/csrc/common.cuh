@@ -132,8 +132,7 @@ struct DevStatus {
     uint32_t max_groups_seen;
     uint32_t check_code; // first failed internal check (0 = none)
     uint32_t check_count;
-    uint32_t work_dmg; // work counters of the implicit damage solve's group kernels
-    uint32_t work_cg;
+    uint32_t cg_done; // CTAs of a kernel of the implicit damage solve that have finished
     uint32_t cg_loops; // iterations of the damage solve's loop in this substep (any scene)
     uint32_t g2p_done; // CTAs of the substep's G2P that have finished
     uint32_t max_movers; // particles that left the key their slot was sorted by (counted when a state is written)

@@ -1366,26 +1366,31 @@ private:
         return 0;
     }
 
-    // Implicit damage solve of the substep (AnisoFractureSimulation.h:437-626): D~ history and coefficients,
-    // right-hand side and preconditioner sums, CG initialisation, the iterations, the nodal change for G2P.
+    // Implicit damage solve of the substep (AnisoFractureSimulation.h:437-626): D~ history, coefficients, right-hand side
+    // and preconditioner sums, CG initialisation, the first iteration, a conditional loop with the others, the nodal change
+    // for G2P. Every solve runs one iteration (r.z is only below the tolerance at the start where it is zero); more are rare.
     int enqueue_damage_solve(const StepArgs<T>& a)
     {
-        ZR_CUDA(cudaMemsetAsync(cgs_, 0, sizeof(CgScalars) * h_scenes_.size(), stream_));
-        k_dmg_prep<T><<<nsm_ * 8, 256, 0, stream_>>>(a);
+        const int ng = cg_ctas();
         k_dmg_rhs<T><<<nsm_ * occ_dmg_[0], DmgShape<T>::NT, 0, stream_>>>(a);
-        k_cg_nodes<T, 0><<<nsm_ * 8, 256, 0, stream_>>>(a);
-        k_cg_scalars<T, 0><<<1, 256, 0, stream_>>>(a, n_scenes(), cudaGraphConditionalHandle{});
+        k_cg_nodes<T, CG_INIT><<<ng, CG_NT, 0, stream_>>>(a, cudaGraphConditionalHandle{}, 0);
+        k_dmg_apply<T><<<nsm_ * occ_dmg_[1], DmgShape<T>::NT, 0, stream_>>>(a);
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         ZR_CUDA(cudaStreamIsCapturing(stream_, &cs));
         if (cs == cudaStreamCaptureStatusActive) {
-            int rc = capture_cg_loop(a);
-            if (rc) return rc;
+            cudaGraphConditionalHandle h;
+            if (int rc = cg_loop_handle(h, 0)) return rc; // the step below sets it when some scene goes on
+            k_cg_nodes<T, CG_STEP><<<ng, CG_NT, 0, stream_>>>(a, h, 1);
+            if (int rc = capture_cg_loop(a, h)) return rc;
         }
         else {
+            k_cg_nodes<T, CG_STEP><<<ng, CG_NT, 0, stream_>>>(a, cudaGraphConditionalHandle{}, 0);
             if (!cg_exec_) {
                 cudaGraph_t g;
                 ZR_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-                int rc = capture_cg_loop(a);
+                cudaGraphConditionalHandle h;
+                int rc = cg_loop_handle(h, 1); // a first pass (with nothing to do when every scene is done) sets it
+                if (!rc) rc = capture_cg_loop(a, h);
                 cudaError_t e = cudaStreamEndCapture(stream_, &g);
                 if (rc) return rc;
                 if (e != cudaSuccess) return fail(ZR_ERR_CUDA_, std::string("damage solve capture: ") + cudaGetErrorString(e));
@@ -1395,14 +1400,26 @@ private:
             }
             ZR_CUDA(cudaGraphLaunch(cg_exec_, stream_));
         }
-        k_cg_nodes<T, 4><<<nsm_ * 8, 256, 0, stream_>>>(a);
+        k_cg_nodes<T, CG_END><<<ng, CG_NT, 0, stream_>>>(a, cudaGraphConditionalHandle{}, 0);
         return 0;
     }
 
-    // Append the CG iterations to the capture under way on stream_: a conditional WHILE node whose body (one
+    int cg_ctas() const { return nsm_ * 4; } // node passes: their chains of dependent reads, not their bytes, take the time
+
+    // the condition of a CG loop in the graph being captured on stream_, with its value at the graph's launch
+    int cg_loop_handle(cudaGraphConditionalHandle& h, unsigned first)
+    {
+        cudaStreamCaptureStatus cs;
+        cudaGraph_t g;
+        ZR_CUDA(cudaStreamGetCaptureInfo(stream_, &cs, nullptr, &g, nullptr, nullptr, nullptr));
+        ZR_CUDA(cudaGraphConditionalHandleCreate(&h, g, first, cudaGraphCondAssignDefault));
+        return 0;
+    }
+
+    // Append CG iterations to the capture under way on stream_: a conditional WHILE node whose body (one
     // iteration) is captured on the side stream; the body's last kernel sets the condition and ends the loop
     // after at most CG_MAX_ITERATIONS + 1 passes.
-    int capture_cg_loop(const StepArgs<T>& a)
+    int capture_cg_loop(const StepArgs<T>& a, cudaGraphConditionalHandle h)
     {
         cudaStreamCaptureStatus cs;
         cudaGraph_t g;
@@ -1410,8 +1427,6 @@ private:
         const cudaGraphEdgeData* edges = nullptr;
         size_t nd = 0;
         ZR_CUDA(cudaStreamGetCaptureInfo(stream_, &cs, nullptr, &g, &deps, &edges, &nd));
-        cudaGraphConditionalHandle h;
-        ZR_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
         cudaGraphNodeParams np = {}; // reserved fields zero
         np.type = cudaGraphNodeTypeConditional;
         np.conditional.handle = h;
@@ -1422,11 +1437,9 @@ private:
         cudaGraph_t body = np.conditional.phGraph_out[0];
         ZR_CUDA(cudaStreamUpdateCaptureDependencies(stream_, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
         ZR_CUDA(cudaStreamBeginCaptureToGraph(side_, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+        k_cg_nodes<T, CG_DIR><<<cg_ctas(), CG_NT, 0, side_>>>(a, cudaGraphConditionalHandle{}, 0);
         k_dmg_apply<T><<<nsm_ * occ_dmg_[1], DmgShape<T>::NT, 0, side_>>>(a);
-        k_cg_nodes<T, 1><<<nsm_ * 8, 256, 0, side_>>>(a);
-        k_cg_nodes<T, 2><<<nsm_ * 8, 256, 0, side_>>>(a);
-        k_cg_nodes<T, 3><<<nsm_ * 8, 256, 0, side_>>>(a);
-        k_cg_scalars<T, 1><<<1, 256, 0, side_>>>(a, n_scenes(), h);
+        k_cg_nodes<T, CG_STEP><<<cg_ctas(), CG_NT, 0, side_>>>(a, h, 1);
         cudaGraph_t out = nullptr;
         const cudaError_t le = cudaGetLastError();
         ZR_CUDA(cudaStreamEndCapture(side_, &out));

@@ -85,8 +85,8 @@ struct CgScalars {
     double zr_new;
     double pAp; // p . A p
     double tol; // min(|r0|_z, 1e-6)
+    double alpha, beta; // step length; of the next search direction
     int32_t iter, done;
-    int32_t pad0, pad1;
 };
 
 template <class T>
@@ -2570,7 +2570,6 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         st->n_blocks = 0;
         st->work_p2g = 0;
         st->work_g2p = 0;
-        st->work_dmg = 0;
         st->g2p_done = 0;
     }
 }
@@ -2588,7 +2587,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
 // batch runs the iterations it would run alone. G2P then adds sum_i w_ip (x_i - pf_i) to the damage.
 // ---------------------------------------------------------------------------------------------------
 enum { CG_SA = 0, CG_SV, CG_DIAG, CG_X, CG_R, CG_Z, CG_P, CG_AP, CG_NF }; // node vectors
-enum { DS_F = 0, DS_A = 3, DS_VOL = 4, DS_C = 5, DS_E = 6 }; // particle scratch fields in the payload buffer
+enum { DS_F = 0, DS_E = 3 }; // particle scratch fields in the payload buffer: fractional position, e_p
 constexpr int CG_MAX_ITERATIONS = 100;
 
 template <class T>
@@ -2619,55 +2618,6 @@ __global__ void k_dmg_drive(StepArgs<T> a, const uint64_t* keys)
         P.f[P_DRV * P.stride + i] = drive;
     }
     if (fallbacks) atomicAdd(&a.st->fallback, fallbacks);
-}
-
-// Per sorted particle of an implicit scene (one thread each, no barriers): the D~ history folded with the drive
-// of the particle's F (cached in P_DRV), and into the particle scratch the fractional position, vol D~ dt/eta,
-// vol, c_p and e_p.
-template <class T>
-__global__ void k_dmg_prep(StepArgs<T> a)
-{
-    using L = typename LayoutOf<T>::type;
-    if (aborted(a.st)) return;
-    const KeyLayout kl = a.kl;
-    const int64_t S = a.pstride;
-    const Pool<T>& P = a.pin;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_total; q += gridDim.x * blockDim.x) {
-        const SceneParams<T>& sp = a.scenes[kl.scene(kl.at(a.keys_sorted, q))];
-        const uint32_t j = a.vals_sorted[q];
-        // every state load of the particle at once (one latency), ahead of the scene and material tests
-        T x[3], F[9];
-#pragma unroll
-        for (int e = 0; e < 3; e++) x[e] = P.f[(P_X + e) * P.stride + j];
-#pragma unroll
-        for (int e = 0; e < 9; e++) F[e] = P.f[(P_F + e) * P.stride + j];
-        const T V0 = P.f[P_V0 * P.stride + j], drive = P.f[P_DRV * P.stride + j];
-        T hist = P.f[P_MDT * P.stride + j];
-        const uint32_t pid = P.pid[j];
-        if (!sp.implicit) continue;
-        T* y = a.pay + pay_pos(q);
-#pragma unroll
-        for (int e = 0; e < 3; e++) {
-            const T xs = mul_rn(x[e], sp.inv_dx);
-            y[(DS_F + e) * S] = xs - (T)int_floor(sub_rn(xs, (T)0.5));
-        }
-        const uint32_t mat = pid >> L::index_bits;
-        const Material<T>& mt = sp.materials[mat < (uint32_t)sp.n_materials ? mat : 0];
-        T av = 0, vol = 0, c = 0, ev = 0;
-        if (mt.damage && (mt.model == MODEL_NEOHOOKEAN_BORDEN || mt.model == MODEL_QR_STABLE_NEOHOOKEAN)) {
-            vol = V0 * det3(F);
-            hist = drive > hist ? drive : hist;
-            P.f[P_MDT * P.stride + j] = hist;
-            const T dt = sp.dt;
-            av = ((dt * hist) / mt.eta) * vol;
-            c = vol * ((T)1 + ((dt / mt.eta) * (hist + (T)1)));
-            ev = vol * (dt / mt.eta) * mt.l0 * mt.l0;
-        }
-        y[DS_A * S] = av;
-        y[DS_VOL * S] = vol;
-        y[DS_C * S] = c;
-        y[DS_E * S] = ev;
-    }
 }
 
 // node tile of a group (its block plus 2 nodes on the + side): index of node (lx, ly, lz)
@@ -2722,30 +2672,36 @@ __device__ void flush_offset_tiles_cg(const StepArgs<T>& a, T* tiles, const int3
     }
 }
 
-// Claim the next group of an implicit scene for a damage-solve kernel (thread 0 claims, all threads get the same
-// answer): the group's particle range and neighbour blocks. Returns the scene, or -1 when the groups are exhausted.
+// The items of a damage-solve kernel, dealt to the CTAs in rounds (they are of about equal size). The set-up of the next item
+// (its range, the grid slots of its blocks, its scene and whether the kernel has work there) is a chain of four dependent
+// reads: threads 0-7 advance it by one link at each next_* call while the CTA works on the current item.
+struct DmgItem {
+    uint32_t start, end;
+    int32_t nbr[8];
+    int scene; // -1: nothing to do (a scene without the solve, or finished); -2: no further items
+};
 template <class T>
-__device__ int dmg_claim(const StepArgs<T>& a, uint32_t* counter, bool need_unfinished, uint32_t& start, uint32_t& end, int32_t* s_nbr, int* s_g,
-    int* s_skip)
-{
-    const KeyLayout kl = a.kl;
-    const uint32_t G = a.st->n_items;
-    for (;;) {
-        if (threadIdx.x == 0) *s_g = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int g = *s_g;
-        if (g >= (int)G) return -1;
-        const uint4 it = a.item[g];
-        start = it.x;
-        end = it.y;
-        const uint32_t sc = kl.scene(kl.at(a.keys_sorted, start));
-        if (threadIdx.x == 0) *s_skip = !a.scenes[sc].implicit || (need_unfinished && a.cgs[sc].done);
-        if (threadIdx.x < 8) s_nbr[threadIdx.x] = a.i_slot[(size_t)g * 8 + threadIdx.x];
-        __syncthreads();
-        if (!*s_skip) return (int)sc;
-        __syncthreads(); // every thread has read *s_skip before thread 0 claims again
+struct DmgNext {
+    uint4 it;
+    int32_t slot;
+    int scene;
+    uint32_t g;
+    __device__ __forceinline__ void range(const StepArgs<T>& a, uint32_t gg, uint32_t G) // threads 0-7
+    {
+        g = gg;
+        it = g < G ? a.item[g] : make_uint4(0, 0, 0, 0);
+        slot = g < G ? a.i_slot[(size_t)g * 8 + threadIdx.x] : -1;
     }
-}
+    __device__ __forceinline__ void key(const StepArgs<T>& a, uint32_t G) { scene = g < G ? (int)a.kl.scene(a.kl.at(a.keys_sorted, it.x)) : -2; }
+    __device__ __forceinline__ void store(const StepArgs<T>& a, DmgItem& d, bool need_unfinished) const
+    {
+        d.nbr[threadIdx.x] = slot;
+        if (threadIdx.x) return;
+        d.start = it.x;
+        d.end = it.y;
+        d.scene = scene < 0 ? scene : ((!a.scenes[scene].implicit || (need_unfinished && a.cgs[scene].done)) ? -1 : scene);
+    }
+};
 
 // threads and particle chunk of the damage solve's group kernels: one thread per (in-block cell, stencil x-offset);
 // a chunk's per-particle values are staged in shared memory for the per-cell sums
@@ -2758,6 +2714,13 @@ struct DmgShape {
     static constexpr int MINB = 4; // CTAs per SM the registers are cut for: these kernels wait on memory
 };
 
+// v[i] by selects (an index that varies at run time puts the array into local memory)
+template <class T>
+__device__ __forceinline__ T pick3(const T (&v)[3], int i)
+{
+    return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]);
+}
+
 // cell ranges of a staged chunk: particles of one cell are contiguous (sorted by cell inside the block)
 template <int NC>
 __device__ __forceinline__ void chunk_cells(const uint8_t* cellof, int cnt, int16_t* cfirst, int16_t* clast, int tid, int nt)
@@ -2769,8 +2732,9 @@ __device__ __forceinline__ void chunk_cells(const uint8_t* cellof, int cnt, int1
     }
 }
 
-// Right-hand side parts and the preconditioner's diagonal. Per chunk: the particles' scratch values staged in
-// shared memory (phase 1), then one thread per (in-block cell, x-offset) sums the 9 (y, z) nodes over its cell's
+// Per particle of an implicit scene the D~ history folded with the drive of its F (cached in P_DRV) and its coefficients,
+// then the right-hand side parts and the preconditioner's diagonal. Per chunk: the particles' values staged in shared memory
+// (phase 1, which also leaves the fractional position and e_p for the operator), then one thread per (in-block cell, x-offset) sums the 9 (y, z) nodes over its cell's
 // particles in registers (phase 2) and adds them to the group's shared node tile; the tile goes to the node
 // vectors CG_SA, CG_SV, CG_DIAG.
 template <class T>
@@ -2784,19 +2748,31 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
     __shared__ T st[D::NS][CHUNK]; // fr x3, vol D~ dt/eta, vol, c
     __shared__ uint8_t cellof[CHUNK];
     __shared__ int16_t cfirst[NC], clast[NC];
-    __shared__ int s_g, s_skip;
-    __shared__ int32_t s_nbr[8];
+    __shared__ DmgItem s_item[2];
     if (aborted_cta(a.st)) return;
+    const uint32_t G = a.st->n_items;
     const KeyLayout kl = a.kl;
+    const Pool<T>& P = a.pin;
     const int64_t S = a.pstride;
     const int tid = threadIdx.x, ii = tid / NC, c = tid % NC;
     const int cx = c >> (L::zbits + L::ybits), cy = (c >> L::zbits) & (L::sy - 1), cz = c & (L::sz - 1);
+    if (blockIdx.x == 0) // the sums the node passes accumulate
+        for (int s = tid; s < a.n_scenes; s += NT) a.cgs[s].zr = a.cgs[s].zr_new = a.cgs[s].pAp = 0;
     for (int q = tid; q < TE; q += NT) tile[q] = (T)0;
     const int f_of[3] = { CG_SA, CG_SV, CG_DIAG };
-    for (;;) {
-        uint32_t start, end;
-        const int sc = dmg_claim<T>(a, &a.st->work_dmg, false, start, end, s_nbr, &s_g, &s_skip);
-        if (sc < 0) break;
+    DmgNext<T> nx;
+    if (tid < 8) {
+        nx.range(a, blockIdx.x, G);
+        nx.key(a, G);
+        nx.store(a, s_item[0], false);
+    }
+    __syncthreads();
+    for (uint32_t g = blockIdx.x, cur = 0; g < G; g += gridDim.x, cur ^= 1) {
+        const DmgItem& item = s_item[cur];
+        const int sc = item.scene;
+        const uint32_t start = item.start, end = sc >= 0 ? item.end : item.start;
+        if (tid < 8) nx.range(a, g + gridDim.x, G);
+        const SceneParams<T>& sp = a.scenes[sc >= 0 ? sc : 0];
         bool any = false;
         for (uint32_t c0 = start; c0 < end; c0 += CHUNK) {
             const int cnt = (int)min((uint32_t)CHUNK, end - c0);
@@ -2805,9 +2781,38 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
                 clast[tid] = 0;
             }
             for (int q = tid; q < cnt; q += NT) {
-                const T* y = a.pay + pay_pos(c0 + q);
+                const uint32_t j = a.vals_sorted[c0 + q];
+                // every state load of the particle at once (one latency), ahead of the material test
+                T x[3], F[9];
 #pragma unroll
-                for (int f = 0; f < D::NS; f++) st[f][q] = y[(DS_F + f) * S];
+                for (int e = 0; e < 3; e++) x[e] = P.f[(P_X + e) * P.stride + j];
+#pragma unroll
+                for (int e = 0; e < 9; e++) F[e] = P.f[(P_F + e) * P.stride + j];
+                const T V0 = P.f[P_V0 * P.stride + j], drive = P.f[P_DRV * P.stride + j];
+                T hist = P.f[P_MDT * P.stride + j];
+                const uint32_t mat = P.pid[j] >> L::index_bits;
+                const Material<T>& mt = sp.materials[mat < (uint32_t)sp.n_materials ? mat : 0];
+                T* y = a.pay + pay_pos(c0 + q);
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    const T xs = mul_rn(x[e], sp.inv_dx), fr = xs - (T)int_floor(sub_rn(xs, (T)0.5));
+                    st[e][q] = fr;
+                    y[(DS_F + e) * S] = fr;
+                }
+                T av = 0, vol = 0, cc = 0, ev = 0;
+                if (mt.damage && (mt.model == MODEL_NEOHOOKEAN_BORDEN || mt.model == MODEL_QR_STABLE_NEOHOOKEAN)) {
+                    vol = V0 * det3(F);
+                    hist = drive > hist ? drive : hist;
+                    P.f[P_MDT * P.stride + j] = hist;
+                    const T dt = sp.dt;
+                    av = ((dt * hist) / mt.eta) * vol;
+                    cc = vol * ((T)1 + ((dt / mt.eta) * (hist + (T)1)));
+                    ev = vol * (dt / mt.eta) * mt.l0 * mt.l0;
+                }
+                st[3][q] = av;
+                st[4][q] = vol;
+                st[5][q] = cc;
+                y[DS_E * S] = ev;
                 cellof[q] = (uint8_t)((kl.at(a.keys_sorted, c0 + q) >> kl.ib) & (NC - 1));
             }
             __syncthreads();
@@ -2824,7 +2829,7 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
                 T w[3][3], dw[3][3];
 #pragma unroll
                 for (int e = 0; e < 3; e++) bspline_w(st[e][q], 0, w[e], dw[e]);
-                const T wx = w[0][ii];
+                const T wx = pick3(w[0], ii);
 #pragma unroll
                 for (int j = 0; j < 3; j++)
 #pragma unroll
@@ -2839,7 +2844,9 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
             any = true;
             __syncthreads();
         }
-        if (any) flush_offset_tiles_cg<T, L, 3>(a, tile, s_nbr, f_of, tid, NT);
+        if (tid < 8) nx.key(a, G);
+        if (any) flush_offset_tiles_cg<T, L, 3>(a, tile, item.nbr, f_of, tid, NT);
+        if (tid < 8) nx.store(a, s_item[cur ^ 1], false);
         __syncthreads();
     }
 }
@@ -2847,7 +2854,8 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
 // The operator's particle part for the search direction p. Per chunk: per particle gc = e_p / dx^2 sum_j p_j
 // grad w_jp (gradients per unit cell; phase 1, from p staged on the group's tile), staged with the fractional
 // position; then per (cell, x-offset) thread the sums gc . grad w over its cell's particles for its 9 nodes
-// (phase 2) into the tile, which goes to A p (CG_AP).
+// (phase 2) into the tile, which goes to A p (CG_AP). The particles' share of p . A p is sum gc . (sum_j p_j grad w_jp): it is
+// summed here, so no pass over the nodes stands between the operator and the step length.
 template <class T>
 __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_apply(StepArgs<T> a)
 {
@@ -2860,10 +2868,11 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
     __shared__ T st[D::NS][CHUNK]; // fr x3, gc x3
     __shared__ uint8_t cellof[CHUNK];
     __shared__ int16_t cfirst[NC], clast[NC];
-    __shared__ int s_g, s_skip;
-    __shared__ int32_t s_nbr[8];
+    __shared__ DmgItem s_item[2];
+    __shared__ int s_last;
     __shared__ uint16_t s_map[TN]; // tile node -> (neighbour block 0-7) << 8 | element in that block
     if (aborted_cta(a.st)) return;
+    const uint32_t G = a.st->n_items;
     const KeyLayout kl = a.kl;
     const int64_t S = a.pstride;
     const int tid = threadIdx.x, ii = tid / NC, c = tid % NC;
@@ -2875,12 +2884,47 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
         s_map[q] = (uint16_t)(((ax * 4 + ay * 2 + az) << 8) | L::element(tx - ax * L::sx, ty - ay * L::sy, tz - az * L::sz));
     }
     const int f_of[1] = { CG_AP };
-    for (;;) {
-        uint32_t start, end;
-        const int sc = dmg_claim<T>(a, &a.st->work_cg, true, start, end, s_nbr, &s_g, &s_skip);
-        if (sc < 0) break;
-        for (int q = tid; q < TN; q += NT) { // (s_map was built before the claim's first barrier)
-            const int m = s_map[q], slot = s_nbr[m >> 8];
+    __shared__ double s_en[NT / 32];
+    double energy = 0; // of the items of scene esc
+    int esc = -1;
+    auto add_energy = [&]() { // every thread of the CTA
+        double v = energy;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        __syncthreads();
+        if ((tid & 31) == 0) s_en[tid >> 5] = v;
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < NT / 32; w++) v += s_en[w];
+            if (esc >= 0 && v != 0.0) atomicAdd(&a.cgs[esc].pAp, v);
+        }
+        energy = 0;
+    };
+    DmgNext<T> nx;
+    if (tid < 8) {
+        nx.range(a, blockIdx.x, G);
+        nx.key(a, G);
+        nx.store(a, s_item[0], true);
+    }
+    __syncthreads();
+    for (uint32_t g = blockIdx.x, cur = 0; g < G; g += gridDim.x, cur ^= 1) {
+        const DmgItem& item = s_item[cur];
+        const int sc = item.scene;
+        if (tid < 8) nx.range(a, g + gridDim.x, G);
+        if (sc < 0) { // the whole CTA
+            if (tid < 8) {
+                nx.key(a, G);
+                nx.store(a, s_item[cur ^ 1], true);
+            }
+            __syncthreads();
+            continue;
+        }
+        const uint32_t start = item.start, end = item.end;
+        if (sc != esc) {
+            if (esc >= 0) add_energy();
+            esc = sc;
+        }
+        for (int q = tid; q < TN; q += NT) {
+            const int m = s_map[q], slot = item.nbr[m >> 8];
             ptile[q] = (slot >= 0 && (uint32_t)slot < a.b_cap) ? cgv(a, CG_P, slot)[m & 0xff] : (T)0;
         }
         __syncthreads();
@@ -2929,6 +2973,7 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
                         g2 += w[0][i] * sC;
                     }
                     const T sgc = ev * inv_dx * inv_dx; // both gradients carry 1/dx
+                    energy += (double)(sgc * (g0 * g0 + g1 * g1 + g2 * g2));
                     g0 *= sgc;
                     g1 *= sgc;
                     g2 *= sgc;
@@ -2950,7 +2995,7 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
                 T w[3][3], dw[3][3];
 #pragma unroll
                 for (int e = 0; e < 3; e++) bspline_w(st[e][q], 0, w[e], dw[e]);
-                const T a0 = g0 * dw[0][ii], a1 = g1 * w[0][ii], a2 = g2 * w[0][ii];
+                const T wx = pick3(w[0], ii), a0 = g0 * pick3(dw[0], ii), a1 = g1 * wx, a2 = g2 * wx;
 #pragma unroll
                 for (int j = 0; j < 3; j++)
 #pragma unroll
@@ -2959,50 +3004,121 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
             add_to_offset_tile_cg<L, 1>(tile, cx, cy, cz, ii, [&](int n, int) { return acc[n]; }); // all lanes
             __syncthreads();
         }
-        flush_offset_tiles_cg<T, L, 1>(a, tile, s_nbr, f_of, tid, NT);
+        if (tid < 8) nx.key(a, G);
+        flush_offset_tiles_cg<T, L, 1>(a, tile, item.nbr, f_of, tid, NT);
+        if (tid < 8) nx.store(a, s_item[cur ^ 1], true);
         __syncthreads();
     }
+    add_energy();
+    // the step lengths, once per scene, by the CTA that finishes last (its counter wraps to zero): a division in every thread
+    // of the node pass would be an FP64 division
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicInc(&a.st->cg_done, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last)
+        for (int s = tid; s < a.n_scenes; s += NT)
+            if (a.scenes[s].implicit && !a.cgs[s].done) a.cgs[s].alpha = a.cgs[s].zr / __ldcg(&a.cgs[s].pAp);
 }
 
-// per scene of a node, with the warp's nodes all of one block (and so of one scene)
-template <class T>
-__device__ __forceinline__ void scene_sum(double v, int scene, double* dst)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int s0 = __shfl_sync(0xffffffffu, scene, 0);
-    if ((threadIdx.x & 31) == 0 && s0 >= 0 && v != 0.0) atomicAdd(dst + (size_t)s0 * (sizeof(CgScalars) / sizeof(double)), v);
-}
+// Per-scene sums of a node pass: a warp's nodes are of one block (and so of one scene). A warp keeps its sum while the scene
+// stays; the CTA adds its warps' sums with one atomic per run of warps of one scene (an atomic per warp to the one address
+// of a scene took longer than the pass).
+constexpr int CG_NT = 256;
+struct SceneSum {
+    double sum = 0;
+    int scene = -1;
+    __device__ __forceinline__ void add(double v, int sc, CgScalars* cgs, double CgScalars::* to) // whole warps
+    {
+        const int s0 = __shfl_sync(0xffffffffu, sc, 0);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (s0 < 0) return;
+        if (s0 != scene && scene >= 0) {
+            if ((threadIdx.x & 31) == 0 && sum != 0.0) atomicAdd(&(cgs[scene].*to), sum);
+            sum = 0;
+        }
+        scene = s0;
+        sum += v; // (lane 0's is the warp's)
+    }
+    __device__ __forceinline__ void finish(CgScalars* cgs, double CgScalars::* to, double* s_v, int* s_s) // whole CTAs
+    {
+        if ((threadIdx.x & 31) == 0) {
+            s_v[threadIdx.x >> 5] = sum;
+            s_s[threadIdx.x >> 5] = scene;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double run = 0;
+            int rsc = -1;
+            for (int w = 0; w <= CG_NT / 32; w++) {
+                const int sc = w < CG_NT / 32 ? s_s[w] : -1;
+                if (sc != rsc) {
+                    if (rsc >= 0 && run != 0.0) atomicAdd(&(cgs[rsc].*to), run);
+                    rsc = sc;
+                    run = 0;
+                }
+                if (w < CG_NT / 32) run += s_v[w];
+            }
+        }
+        __syncthreads();
+    }
+};
 
-// node kernels: STAGE 0 init (r = rhs, z = r/diag, p = z, r.z), 1 A p += diag p and p.Ap, 2 x, r, z update
-// and r.z, 3 p = z + beta p and A p = 0, 4 finish (the grid's phase field becomes x - pf)
+// Node passes of the solve. CG_INIT: r = rhs, z = r / diag, p = z, with r.z and the diagonal's share of p.Ap. CG_STEP: the
+// operator's diagonal added, x, r and z moved along p, r.z, A p cleared. CG_DIR: p = z + beta p and the diagonal's share of
+// p.Ap. CG_END: the grid's phase field becomes x - pf, the vectors are cleared for the next solve. The last CTA of CG_INIT and
+// CG_STEP does the scenes' bookkeeping (per scene: tolerance; iteration count, beta and whether it is done) and, after a step,
+// sets the condition of the loop that runs the further iterations: some scene unfinished, and never more than
+// CG_MAX_ITERATIONS + 1 passes (each scene stops itself at CG_MAX_ITERATIONS, so the loop always ends).
+// An iteration is three kernels (direction, operator, step). With the operator's product, its dot product, the step, the
+// direction and the bookkeeping in one kernel each it was five, and the first iteration a pass of the conditional loop.
+enum { CG_INIT = 0, CG_STEP, CG_DIR, CG_END };
 template <class T, int STAGE>
-__global__ void k_cg_nodes(StepArgs<T> a)
+__global__ void __launch_bounds__(CG_NT) k_cg_nodes(StepArgs<T> a, cudaGraphConditionalHandle loop, int has_loop)
 {
     using L = typename LayoutOf<T>::type;
-    if (aborted(a.st)) return;
+    __shared__ double s_v[CG_NT / 32];
+    __shared__ int s_s[CG_NT / 32], s_last;
+    __shared__ uint32_t s_active;
+    if (aborted_cta(a.st)) { // by an earlier kernel: every CTA leaves, and the loop ends
+        if (STAGE == CG_STEP && has_loop && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, 0u);
+        return;
+    }
     const uint32_t B = min(a.st->n_blocks, a.b_cap);
     const uint32_t total = B * L::nodes;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ((total + 31) & ~31u); t += gridDim.x * blockDim.x) {
-        double acc = 0;
+    SceneSum zr, pAp;
+    for (uint32_t t = blockIdx.x * CG_NT + threadIdx.x; t < ((total + 31) & ~31u); t += gridDim.x * CG_NT) {
+        double acc = 0, dsum = 0;
         int scene = -1;
         if (t < total) {
             const uint32_t b = t / L::nodes, e = t % L::nodes;
+            T* dg = cgv(a, CG_DIAG, b) + e;
+            T* x = cgv(a, CG_X, b) + e;
+            T* r = cgv(a, CG_R, b) + e;
+            T* z = cgv(a, CG_Z, b) + e;
+            T* p = cgv(a, CG_P, b) + e;
+            T* Ap = cgv(a, CG_AP, b) + e;
+            T* sa = cgv(a, CG_SA, b) + e;
+            T* sv = cgv(a, CG_SV, b) + e;
+            T* pf = a.vel + (size_t)b * NVEL * L::nodes + 3 * L::nodes + e;
+            // every load of the node at once, ahead of the scene's test
+            T diag, xv = 0, rv = 0, zv = 0, pv = 0, apv = 0, sav = 0, svv = 0, pfv = 0;
+            diag = *dg;
+            if (STAGE == CG_INIT) sav = *sa, svv = *sv;
+            if (STAGE == CG_INIT || STAGE == CG_END) pfv = *pf;
+            if (STAGE == CG_STEP) rv = *r, apv = *Ap;
+            if (STAGE == CG_STEP || STAGE == CG_END) xv = *x;
+            if (STAGE == CG_STEP || STAGE == CG_DIR) pv = *p;
+            if (STAGE == CG_DIR) zv = *z;
             const int sc = (int)(a.b_key[b] >> 40);
-            const SceneParams<T>& sp = a.scenes[sc];
-            CgScalars& cs = a.cgs[sc];
-            if (sp.implicit && (STAGE == 0 || STAGE == 4 || !cs.done)) {
+            const CgScalars& cs = a.cgs[sc];
+            if (a.scenes[sc].implicit && (STAGE == CG_INIT || STAGE == CG_END || !cs.done)) {
                 scene = sc;
-                T* dg = cgv(a, CG_DIAG, b) + e;
-                const T diag = *dg;
-                T* x = cgv(a, CG_X, b) + e;
-                T* r = cgv(a, CG_R, b) + e;
-                T* z = cgv(a, CG_Z, b) + e;
-                T* p = cgv(a, CG_P, b) + e;
-                T* Ap = cgv(a, CG_AP, b) + e;
-                T* pf = a.vel + (size_t)b * NVEL * L::nodes + 3 * L::nodes + e;
                 const bool on = diag > (T)0;
-                if (STAGE == 0) {
-                    const T rhs = on ? cgv(a, CG_SA, b)[e] + *pf * cgv(a, CG_SV, b)[e] : (T)0;
+                if (STAGE == CG_INIT) {
+                    const T rhs = on ? sav + pfv * svv : (T)0;
                     const T zz = on ? rhs / diag : (T)0;
                     *x = 0;
                     *r = rhs;
@@ -3010,80 +3126,80 @@ __global__ void k_cg_nodes(StepArgs<T> a)
                     *p = zz;
                     *Ap = 0;
                     acc = (double)rhs * (double)zz;
+                    dsum = on ? (double)(diag * zz) * (double)zz : 0.0;
                 }
-                else if (STAGE == 1) {
-                    const T ap = on ? *Ap + diag * *p : (T)0;
-                    *Ap = ap;
-                    acc = (double)ap * (double)*p;
-                }
-                else if (STAGE == 2) {
-                    const T alpha = (T)(cs.zr / cs.pAp);
-                    const T xn = *x + *p * alpha, rn = *r - *Ap * alpha, zn = on ? rn / diag : (T)0;
-                    *x = xn;
+                else if (STAGE == CG_STEP) {
+                    const T alpha = (T)cs.alpha;
+                    const T ap = on ? apv + diag * pv : (T)0;
+                    const T rn = rv - ap * alpha, zn = on ? rn / diag : (T)0;
+                    *x = xv + pv * alpha;
                     *r = rn;
                     *z = zn;
+                    *Ap = 0;
                     acc = (double)zn * (double)rn;
                 }
-                else if (STAGE == 3) {
-                    const T beta = (T)(cs.zr_new / cs.zr);
-                    *p = *z + beta * *p;
-                    *Ap = 0;
+                else if (STAGE == CG_DIR) {
+                    const T pn = zv + (T)cs.beta * pv;
+                    *p = pn;
+                    dsum = on ? (double)(diag * pn) * (double)pn : 0.0;
                 }
                 else {
-                    *pf = on ? *x - *pf : (T)0;
+                    *pf = on ? xv - pfv : (T)0;
                     // the solve's vectors start from zero next time
-                    cgv(a, CG_SA, b)[e] = 0;
-                    cgv(a, CG_SV, b)[e] = 0;
+                    *sa = 0;
+                    *sv = 0;
                     *dg = 0;
                     *Ap = 0;
                 }
             }
         }
-        if (STAGE == 0 || STAGE == 2) scene_sum<T>(acc, scene, STAGE == 0 ? &a.cgs[0].zr : &a.cgs[0].zr_new);
-        if (STAGE == 1) scene_sum<T>(acc, scene, &a.cgs[0].pAp);
+        if (STAGE == CG_INIT) zr.add(acc, scene, a.cgs, &CgScalars::zr);
+        if (STAGE == CG_STEP) zr.add(acc, scene, a.cgs, &CgScalars::zr_new);
+        if (STAGE == CG_INIT || STAGE == CG_DIR) pAp.add(dsum, scene, a.cgs, &CgScalars::pAp);
     }
-}
-
-// per-scene CG bookkeeping (one block): STAGE 0 after init, 1 after an iteration. STAGE 1 runs as the last
-// kernel of the loop body and sets the loop's condition: some scene unfinished, and never more than
-// CG_MAX_ITERATIONS + 1 passes (each scene stops itself at CG_MAX_ITERATIONS, so the loop always ends).
-template <class T, int STAGE>
-__global__ void k_cg_scalars(StepArgs<T> a, int n_scenes, cudaGraphConditionalHandle loop)
-{
-    __shared__ uint32_t s_active;
-    if (threadIdx.x == 0) s_active = 0;
+    if (STAGE == CG_INIT) zr.finish(a.cgs, &CgScalars::zr, s_v, s_s);
+    if (STAGE == CG_STEP) zr.finish(a.cgs, &CgScalars::zr_new, s_v, s_s);
+    if (STAGE == CG_INIT || STAGE == CG_DIR) pAp.finish(a.cgs, &CgScalars::pAp, s_v, s_s);
+    if (STAGE != CG_INIT && STAGE != CG_STEP) return;
+    // the bookkeeping, by the CTA that finishes last (its counter wraps to zero)
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(&a.st->cg_done, gridDim.x - 1) == gridDim.x - 1;
+        s_active = 0;
+        __threadfence();
+    }
     __syncthreads();
-    const bool ab = aborted(a.st);
-    for (int s = threadIdx.x; s < n_scenes; s += blockDim.x) {
+    if (!s_last) return;
+    for (int s = threadIdx.x; s < a.n_scenes; s += CG_NT) {
         CgScalars& cs = a.cgs[s];
         if (!a.scenes[s].implicit) {
             cs.done = 1;
             continue;
         }
-        if (STAGE == 0) {
-            const double res = sqrt(cs.zr);
+        if (STAGE == CG_INIT) {
+            const double res = sqrt(__ldcg(&cs.zr));
             cs.tol = res < 1e-6 ? res : 1e-6;
             cs.iter = 0;
             cs.done = res <= cs.tol;
         }
         else if (!cs.done) {
-            cs.zr = cs.zr_new;
+            const double zn = __ldcg(&cs.zr_new);
+            cs.beta = zn / cs.zr;
+            cs.zr = zn;
             cs.iter++;
-            cs.done = sqrt(cs.zr) <= cs.tol || cs.iter >= CG_MAX_ITERATIONS;
+            cs.done = sqrt(zn) <= cs.tol || cs.iter >= CG_MAX_ITERATIONS;
+            cs.pAp = 0;
         }
-        cs.pAp = 0;
         cs.zr_new = 0;
-        if (ab) cs.done = 1;
         if (!cs.done) atomicAdd(&s_active, 1u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        a.st->work_cg = 0;
-        if (STAGE == 0)
+        if (STAGE == CG_INIT)
             a.st->cg_loops = 0;
         else {
             const uint32_t loops = ++a.st->cg_loops;
-            cudaGraphSetConditional(loop, (s_active > 0 && loops <= (uint32_t)CG_MAX_ITERATIONS) ? 1u : 0u);
+            if (has_loop) cudaGraphSetConditional(loop, (s_active > 0 && loops <= (uint32_t)CG_MAX_ITERATIONS) ? 1u : 0u);
         }
     }
 }
