@@ -1,4 +1,4 @@
-"""GPU: the incremental sort's group ranges at the edges of its tiles (2,048 storage indices): particle counts around whole
+"""GPU: the incremental sort's group ranges at the edges of its tiles (512 storage indices, 2,048 in large scenes): particle counts around whole
 tiles, groups longer than a tile, tiles whose particles all move, groups that start and end with a tile. FP64 against the
 oracle: only the order of sums differs."""
 import numpy as np
@@ -20,7 +20,7 @@ def scene(x, v):
             "objects": []}
 
 
-@pytest.mark.parametrize("n", [1, 31, 2047, 2048, 2049, 4096, 6145])
+@pytest.mark.parametrize("n", [1, 31, 511, 512, 513, 2047, 2048, 2049, 4096, 6145])
 @pytest.mark.parametrize("spread", [0.5, 8.0], ids=["one or two long groups", "many groups"])
 def test_ranges_at_tile_edges(n, spread):
     rng = np.random.default_rng(17 * n)

@@ -908,15 +908,24 @@ private:
             kl_.total(), stream_);
     }
 
-    // tiles of the sort and of the group-head pass (SORT_TILE keys each) for up to cap particles
-    static int64_t sort_tiles(int64_t n) { return std::max<int64_t>(1, (n + SORT_TILE - 1) / SORT_TILE); }
-    // movers' fixed bucket slots: SORT_MAXM per tile
-    static int64_t bucket_slots(int64_t cap) { return sort_tiles(cap) * SORT_MAXM; }
+    // items per thread of the incremental sort's kernels (tiles of 256 times that): its passes are chains of dependent reads
+    // and of rounds over a tile, and a small scene leaves most SMs idle with long tiles. Per substep with 8 / 2 items: 4,096
+    // particles 40.6 / 37.4 us, 32,768 48.4 / 43.5, 425,984 114.9 / 112.9; 1,068,849 334.8 / 353.5 (each tile sums the counts
+    // of all lower ones), 3,407,872 614 / 657.
+    int sort_per() const { return N_ <= SORT_SMALL ? 2 : SORT_PER; }
+    static constexpr uint32_t SORT_SMALL = 600000;
+    static int64_t sort_tiles(int64_t n, int per) { return std::max<int64_t>(1, (n + per * SORT_NT - 1) / (per * SORT_NT)); }
+    static int64_t max_tiles(int64_t cap) { return std::max(sort_tiles(cap, SORT_PER), sort_tiles(std::min<int64_t>(cap, SORT_SMALL), 2)); }
+    // movers' fixed bucket slots
+    static int64_t bucket_slots(int64_t cap)
+    {
+        return std::max(sort_tiles(cap, SORT_PER) * SortTile<SORT_PER>::MAXM, sort_tiles(std::min<int64_t>(cap, SORT_SMALL), 2) * SortTile<2>::MAXM);
+    }
     // sort_aux_: [zero at the start of a substep: b_cnt, b_max (tiles u32 each)]
     // [stay bits: ceil(cap/32) u32][t_first, t_stay, t_last: tiles u32 each][look-back: tiles + 1 u64]
-    static size_t sort_zero_bytes(int64_t cap) { return 8 * (size_t)sort_tiles(cap); }
-    static size_t sort_aux_words(int64_t cap) { return sort_zero_bytes(cap) / 4 + (size_t)((cap + 31) / 32) + 3 * (size_t)sort_tiles(cap) + 1; }
-    static size_t sort_aux_bytes(int64_t cap) { return 4 * sort_aux_words(cap) + 8 * ((size_t)sort_tiles(cap) + 2); }
+    static size_t sort_zero_bytes(int64_t cap) { return 8 * (size_t)max_tiles(cap); }
+    static size_t sort_aux_words(int64_t cap) { return sort_zero_bytes(cap) / 4 + (size_t)((cap + 31) / 32) + 3 * (size_t)max_tiles(cap) + 1; }
+    static size_t sort_aux_bytes(int64_t cap) { return 4 * sort_aux_words(cap) + 8 * ((size_t)sort_tiles(cap, SORT_PER) + 2); }
     uint64_t* lookback_words() const
     {
         const size_t off = (4 * sort_aux_words((int64_t)cap_) + 7) & ~(size_t)7;
@@ -931,7 +940,7 @@ private:
     cudaError_t bin_incremental(int64_t n, const StepArgs<T>& a)
     {
         SortBufs sb;
-        const int64_t tiles = sort_tiles(n), tcap = sort_tiles((int64_t)cap_);
+        const int64_t tiles = sort_tiles(n, sort_per()), tcap = max_tiles((int64_t)cap_);
         sb.b_cnt = reinterpret_cast<uint32_t*>(sort_aux_);
         sb.b_max = sb.b_cnt + tcap;
         sb.stay_bits = sb.b_max + tcap;
@@ -943,20 +952,26 @@ private:
         sb.n = n;
         sb.tiles = (int)tiles;
         const uint32_t* nk = (const uint32_t*)keys_in_;
-        k_sort_tiles<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, (const uint32_t*)keys_sorted_, sb, st_);
-        k_sort_merge<T><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(a, nk, sb, (uint32_t*)keys_sorted_, vals_sorted_);
+        if (sort_per() == 2) {
+            k_sort_tiles<2><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, (const uint32_t*)keys_sorted_, sb, st_);
+            k_sort_merge<T, 2><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(a, nk, sb, (uint32_t*)keys_sorted_, vals_sorted_);
+        }
+        else {
+            k_sort_tiles<SORT_PER><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, (const uint32_t*)keys_sorted_, sb, st_);
+            k_sort_merge<T, SORT_PER><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(a, nk, sb, (uint32_t*)keys_sorted_, vals_sorted_);
+        }
         return cudaGetLastError();
     }
 
     // first sorted index of every (scene, page) into g_start_, their number into st_->n_groups
     cudaError_t group_heads(int64_t n)
     {
-        const int64_t tiles = sort_tiles(n);
+        const int64_t tiles = sort_tiles(n, SORT_PER);
         uint64_t* lb = lookback_words();
         cudaError_t e = cudaMemsetAsync(lb, 0, 8 * ((size_t)tiles + 1), stream_);
         if (e != cudaSuccess) return e;
         k_group_heads<<<(unsigned)tiles, SORT_NT, 0, stream_>>>(keys_sorted_, n, kl_, lb, reinterpret_cast<uint32_t*>(lb + tiles), g_start_,
-            (uint32_t)cap_, tile_first(), st_);
+            (uint32_t)cap_, tile_first(), sort_per() * SORT_NT, st_);
         return cudaGetLastError();
     }
 

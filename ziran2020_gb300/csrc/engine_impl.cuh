@@ -153,15 +153,7 @@ __device__ inline bool aborted(const DevStatus* st) { return (*(volatile const u
 
 // the same decision for every thread of the CTA (kernels with barriers or full-warp shuffles must not
 // let some threads leave early)
-__device__ inline bool aborted_cta(const DevStatus* st)
-{
-    __shared__ int s_abort;
-    if (threadIdx.x == 0) s_abort = aborted(st) ? 1 : 0;
-    __syncthreads();
-    bool r = s_abort != 0;
-    __syncthreads();
-    return r;
-}
+__device__ inline bool aborted_cta(const DevStatus* st) { return __syncthreads_or(aborted(st) ? 1 : 0) != 0; }
 
 // ---------------------------------------------------------------------------------------------------
 // keys of the current particle positions (used after a load or a host upload; afterwards G2P writes
@@ -244,7 +236,7 @@ struct GroupHead {
 // particles whose cell did not change ("stayers") are already sorted; only the particles that changed cell
 // ("movers", ~2% per substep at the slab's speeds) need placing.
 //
-// Storage is cut into tiles of SORT_TILE indices. B[j] = the first old key of tile j (the old keys ascend with the
+// Storage is cut into tiles (SortTile: 2,048 indices, or 512 in small scenes, see the host's sort_per). B[j] = the first old key of tile j (the old keys ascend with the
 // storage index). Mover key k belongs to bucket b(k) = the largest j with B[j] <= k (0 when there is none): every
 // element of bucket j (its movers) and tile j (its stayers) lies in [B[j], B[j+1]] and comes after every element of
 // lower tiles and buckets, so tile j's merged output starts at (stayers in tiles < j) + (movers in buckets < j). Inside
@@ -266,9 +258,13 @@ struct GroupHead {
 // a third kernel behind the merge, for the head counts of the lower tiles): as five nodes (a memset
 // and four kernels) the substep took 57.0 us on 32,768 particles and 125.6 us on 425,984, with two 49.3 and 118.8 us.
 //
-// A bucket larger than SORT_MAXM raises FLAG_SORT: the host repeats the substep with a full radix sort.
+// A bucket larger than its slots (SortTile::MAXM) raises FLAG_SORT: the host repeats the substep with a full radix sort.
 // ---------------------------------------------------------------------------------------------------
-constexpr int SORT_NT = 256, SORT_PER = 8, SORT_TILE = SORT_NT * SORT_PER, SORT_MAXM = 1024;
+constexpr int SORT_NT = 256, SORT_PER = 8, SORT_TILE = SORT_NT * SORT_PER; // the group-head pass, and tiles of large scenes
+template <int PER>
+struct SortTile { // PER items per thread: a tile, and its bucket's slots
+    static constexpr int TILE = SORT_NT * PER, MAXM = PER > 4 ? TILE / 2 : TILE;
+};
 constexpr uint32_t SORT_NOKEY = 0xffffffffu; // keys of the incremental sort hold at most 31 bits
 
 struct SortBufs {
@@ -278,26 +274,28 @@ struct SortBufs {
     uint32_t* t_first; // [tiles] first old key per tile: B (k_group_heads or the previous merge wrote it)
     uint32_t* t_stay; // [tiles] stayers per tile
     uint32_t* t_last; // [tiles] last stayer key per tile (SORT_NOKEY: none)
-    uint32_t* b_key; // [tiles * SORT_MAXM] movers' keys: bucket j's at j * SORT_MAXM + ticket
-    uint32_t* b_idx; // [tiles * SORT_MAXM] movers' storage indices, likewise
+    uint32_t* b_key; // [tiles * MAXM] movers' keys: bucket j's at j * MAXM + ticket
+    uint32_t* b_idx; // [tiles * MAXM] movers' storage indices, likewise
     int64_t n;
     int tiles;
 };
 constexpr int SORT_FIRST = 4096; // tiles whose first keys a CTA copies to shared memory for its searches
 
-static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, const uint32_t* kold, SortBufs sb, const DevStatus* st)
+template <int PER>
+__global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, const uint32_t* kold, SortBufs sb, const DevStatus* st)
 {
+    constexpr int TILE = SortTile<PER>::TILE, MAXM = SortTile<PER>::MAXM;
     __shared__ uint32_t s_first[SORT_FIRST];
     __shared__ uint32_t s_cnt[SORT_NT / 32], s_last[SORT_NT / 32];
     const int j = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, T = sb.tiles;
-    const int64_t t0 = (int64_t)j * SORT_TILE;
+    const int64_t t0 = (int64_t)j * TILE;
     uint32_t nst = 0, last = SORT_NOKEY;
     unsigned moves = 0; // bit r: this thread's item of round r moved
     // items in storage order; a warp takes 256 consecutive ones, 32 at a time; every load issued first
-    uint32_t kn[SORT_PER], ko[SORT_PER];
+    uint32_t kn[PER], ko[PER];
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
-        const int64_t i = t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane;
+    for (int r = 0; r < PER; r++) {
+        const int64_t i = t0 + (int64_t)w * (32 * PER) + r * 32 + lane;
         kn[r] = i < sb.n ? knew[i] : 0u;
         ko[r] = i < sb.n ? kold[i] : 1u;
     }
@@ -306,8 +304,8 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* k
         for (int q = threadIdx.x; q < T; q += SORT_NT) s_first[q] = sb.t_first[q];
     const uint32_t* B = T <= SORT_FIRST ? s_first : sb.t_first;
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
-        const int64_t i = t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane;
+    for (int r = 0; r < PER; r++) {
+        const int64_t i = t0 + (int64_t)w * (32 * PER) + r * 32 + lane;
         const bool valid = i < sb.n, stay = valid && kn[r] == ko[r];
         const unsigned bs = __ballot_sync(0xffffffffu, stay);
         if (lane == 0 && valid) sb.stay_bits[i >> 5] = bs; // the merge reads these: it overwrites the old keys
@@ -331,7 +329,7 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* k
     }
     if (ab || !moves) return; // (an aborted substep's tickets would not be cleared)
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
+    for (int r = 0; r < PER; r++) {
         if (!((moves >> r) & 1u)) continue;
         const uint32_t k = kn[r];
         int lo = 0, hi = T; // first q with B[q] > k
@@ -343,9 +341,9 @@ static __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* k
         const uint32_t b = lo > 0 ? (uint32_t)(lo - 1) : 0u;
         const uint32_t t = atomicAdd(&sb.b_cnt[b], 1u);
         atomicMax(&sb.b_max[b], k);
-        if (t < (uint32_t)SORT_MAXM) { // a fuller bucket makes the merge raise FLAG_SORT
-            sb.b_key[(size_t)b * SORT_MAXM + t] = k;
-            sb.b_idx[(size_t)b * SORT_MAXM + t] = (uint32_t)(t0 + (int64_t)w * (32 * SORT_PER) + r * 32 + lane);
+        if (t < (uint32_t)MAXM) { // a fuller bucket makes the merge raise FLAG_SORT
+            sb.b_key[(size_t)b * MAXM + t] = k;
+            sb.b_idx[(size_t)b * MAXM + t] = (uint32_t)(t0 + (int64_t)w * (32 * PER) + r * 32 + lane);
         }
     }
 }
@@ -440,23 +438,24 @@ __device__ __forceinline__ void range_event(const StepArgs<T>& a, int32_t h, uns
 }
 
 // The shared buffers of k_sort_merge's two parts overlap.
+template <int TILE, int MAXM>
 union MergeShared {
     struct {
-        uint32_t s_key[SORT_TILE], s_idx[SORT_TILE]; // the tile's stayers in storage (= key) order
-        uint32_t m_key[SORT_MAXM], m_idx[SORT_MAXM], m_key2[SORT_MAXM], m_idx2[SORT_MAXM];
+        uint32_t s_key[TILE], s_idx[TILE]; // the tile's stayers in storage (= key) order
+        uint32_t m_key[MAXM], m_idx[MAXM], m_key2[MAXM], m_idx2[MAXM];
     } m;
     struct {
-        uint32_t pos[SORT_TILE + SORT_MAXM]; // output positions of the tile's group heads, in order
-        uint32_t off[SORT_TILE + SORT_MAXM]; // their first items, counted from the tile's first
+        uint32_t pos[TILE + MAXM]; // output positions of the tile's group heads, in order
+        uint32_t off[TILE + MAXM]; // their first items, counted from the tile's first
     } h;
 };
 
-template <class T>
+template <class T, int PER>
 __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uint32_t* knew, SortBufs sb, uint32_t* out_keys, uint32_t* out_vals)
 {
-    constexpr int RMAX = (SORT_TILE + SORT_MAXM) / SORT_NT; // rounds over a tile's output
-    __shared__ MergeShared sh;
-    __shared__ uint32_t o_key[SORT_TILE + SORT_MAXM]; // the tile's output in order
+    constexpr int TILE = SortTile<PER>::TILE, MAXM = SortTile<PER>::MAXM, RMAX = (TILE + MAXM) / SORT_NT; // rounds over a tile's output
+    __shared__ MergeShared<TILE, MAXM> sh;
+    __shared__ uint32_t o_key[TILE + MAXM]; // the tile's output in order
     __shared__ uint32_t s_wcnt[RMAX][SORT_NT / 32];
     __shared__ uint32_t s_red[2][SORT_NT / 32];
     __shared__ uint32_t s_ns, s_nh, s_i0;
@@ -467,11 +466,11 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
     if (blockIdx.x == 0) // the per-scene grid mass k_grid accumulates
         for (int s = tid; s < a.n_scenes; s += SORT_NT) a.grid_mass[s] = 0;
     // the tile's new keys and stay bits: issued ahead of everything that is tested. Item (r, w, lane) = t0 + r*256 + w*32 + lane
-    const int64_t t0 = (int64_t)j * SORT_TILE;
-    uint32_t keys[SORT_PER];
+    const int64_t t0 = (int64_t)j * TILE;
+    uint32_t keys[PER];
     unsigned mine = 0; // bit r: this thread's item of round r stays
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
+    for (int r = 0; r < PER; r++) {
         const int64_t i = t0 + r * SORT_NT + tid;
         keys[r] = i < sb.n ? knew[i] : 0u;
         if (i < sb.n && ((sb.stay_bits[i >> 5] >> lane) & 1u)) mine |= 1u << r; // i % 32 == lane: rounds and warps start at multiples of 32
@@ -488,14 +487,14 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
         if (c) pk = max(pk, mk + 1);
     }
     if (aborted_cta(st)) return;
-    if (bc > (uint32_t)SORT_MAXM) { // the whole CTA: the substep is repeated with a full sort
+    if (bc > (uint32_t)MAXM) { // the whole CTA: the substep is repeated with a full sort
         if (tid == 0) raise_flag(st, FLAG_SORT);
         return;
     }
     const int nm = (int)bc;
     for (int q = tid; q < nm; q += SORT_NT) {
-        m_key[q] = sb.b_key[(size_t)j * SORT_MAXM + q];
-        m_idx[q] = sb.b_idx[(size_t)j * SORT_MAXM + q];
+        m_key[q] = sb.b_key[(size_t)j * MAXM + q];
+        m_idx[q] = sb.b_idx[(size_t)j * MAXM + q];
     }
     for (int o = 16; o > 0; o >>= 1) {
         below += __shfl_down_sync(0xffffffffu, below, o);
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
     }
     // the tile's stayers, compacted in storage order
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
+    for (int r = 0; r < PER; r++) {
         const unsigned b = __ballot_sync(0xffffffffu, (mine >> r) & 1u);
         if (lane == 0) s_wcnt[r][w] = __popc(b);
     }
@@ -528,10 +527,10 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
         if (lane == 0) *total = carry;
     };
     __syncthreads();
-    if (w == 0) scan_counts(SORT_PER, &s_ns);
+    if (w == 0) scan_counts(PER, &s_ns);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < SORT_PER; r++) {
+    for (int r = 0; r < PER; r++) {
         const unsigned b = __ballot_sync(0xffffffffu, (mine >> r) & 1u);
         if ((mine >> r) & 1u) {
             const uint32_t pos = s_wcnt[r][w] + __popc(b & ((1u << lane) - 1u));
@@ -565,7 +564,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
         out_keys[pos] = k;
         out_vals[pos] = v;
         o_key[p] = k;
-        if (pos % SORT_TILE == 0) sb.t_first[pos / SORT_TILE] = k; // B of the next substep
+        if (pos % TILE == 0) sb.t_first[pos / TILE] = k; // B of the next substep
     };
     for (int t = tid; t < ns; t += SORT_NT) { // stayer: its rank + the bucket's movers with a smaller key
         const uint32_t k = s_key[t];
@@ -682,7 +681,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_merge(StepArgs<T> a, const uin
 constexpr uint64_t LB_AGG = 1ull << 62, LB_PREFIX = 2ull << 62, LB_VALUE = (1ull << 62) - 1;
 
 static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* keys, int64_t n, KeyLayout kl, uint64_t* status, uint32_t* counter,
-    uint32_t* g_start, uint32_t cap, uint32_t* t_first, DevStatus* st)
+    uint32_t* g_start, uint32_t cap, uint32_t* t_first, int first_tile, DevStatus* st)
 {
     __shared__ uint32_t s_w[SORT_PER][SORT_NT / 32];
     __shared__ int s_tile;
@@ -692,7 +691,8 @@ static __global__ void __launch_bounds__(SORT_NT) k_group_heads(const uint64_t* 
     __syncthreads();
     const int j = s_tile;
     const int64_t t0 = (int64_t)j * SORT_TILE;
-    if (tid == 0) t_first[j] = (uint32_t)kl.at(keys, (uint32_t)t0); // B of the next substep's incremental sort (32-bit keys)
+    // B of the next substep's incremental sort (32-bit keys), whose tiles are first_tile items long
+    for (int64_t i = t0 + (int64_t)tid * first_tile; i < min(n, t0 + SORT_TILE); i += (int64_t)SORT_NT * first_tile) t_first[i / first_tile] = (uint32_t)kl.at(keys, (uint32_t)i);
     unsigned mine = 0;
 #pragma unroll
     for (int r = 0; r < SORT_PER; r++) {
@@ -2289,10 +2289,13 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
     }
     const uint32_t G = a.st->n_items;
     const KeyLayout kl = a.kl;
-    for (;;) {
-        if (threadIdx.x == 0) s_g = (int)atomicAdd(&a.st->work_g2p, 1u);
-        __syncthreads();
-        const int g = s_g;
+    for (bool first = true;; first = false) {
+        int g = blockIdx.x; // the first item is the CTA's own number (claims count from the grid's size)
+        if (!first) {
+            if (threadIdx.x == 0) s_g = (int)(gridDim.x + atomicAdd(&a.st->work_g2p, 1u));
+            __syncthreads();
+            g = s_g;
+        }
         if (g >= (int)G) break;
         const uint4 it = a.item[g];
         const uint32_t start = it.x, end = it.y;
