@@ -1222,115 +1222,77 @@ struct OffsetTiles {
     }
 };
 
-// The same sums where several lanes hold pieces of one cell (see CellSplit). FP32 spreads a cell over both warps of an
-// offset, so it adds with shared-memory atomics (8.5 lane-operations per clock and SM against 15.6 for the plain form); in
-// FP64 one warp holds all cells of an offset, so the pieces of a cell take turns (`parts` of them at most) and the plain
-// form stays. Every lane of the warp must call it.
+// The same sums where several lanes hold pieces of one cell (split_cells): the pieces of a cell take turns, `parts` of them at
+// most. Every lane of the warp must call it.
 template <class T, class L>
 __device__ __forceinline__ void add_pieces_to_offset_tile(const NodeAcc<T>& acc, T* tiles, int cell, int ii, int nf, bool used, int part, int parts)
 {
     using OT = OffsetTiles<L>;
     T* base = tiles + ii * NACC * OT::TS + OT::corner(cell);
-    if constexpr (L::nodes > 32) {
-        (void)part;
-        (void)parts;
-        if (!used) return;
+    for (int turn = 0; turn < parts; turn++) {
 #pragma unroll
         for (int jj = 0; jj < 3; jj++)
 #pragma unroll
             for (int kk = 0; kk < 3; kk++) {
                 T* t = base + jj * OT::TZ + kk;
+                if (used && part == turn) {
 #pragma unroll
-                for (int f = 0; f < NACC; f++)
-                    if (f < nf) atomicAdd(t + f * OT::TS, acc.field(jj * 3 + kk, f));
+                    for (int f = 0; f < NACC; f++)
+                        if (f < nf) t[f * OT::TS] += acc.field(jj * 3 + kk, f);
+                }
+                __syncwarp();
             }
     }
-    else
-        for (int turn = 0; turn < parts; turn++) {
-#pragma unroll
-            for (int jj = 0; jj < 3; jj++)
-#pragma unroll
-                for (int kk = 0; kk < 3; kk++) {
-                    T* t = base + jj * OT::TZ + kk;
-                    if (used && part == turn) {
-#pragma unroll
-                        for (int f = 0; f < NACC; f++)
-                            if (f < nf) t[f * OT::TS] += acc.field(jj * 3 + kk, f);
-                    }
-                    __syncwarp();
-                }
-        }
 }
 
-// Work of the accumulation's (cell, x-offset) threads where cells hold unequal numbers of particles. A chunk takes as long as
-// its fullest cell, and a cell without particles leaves its threads idle: so the cells are cut into pieces of at most R
-// particles, one piece per thread of an offset, R the smallest count for which the pieces fit.
-// FP32 does so where cells are crowded: a chunk of 512 particles holds 64 cells at 8 per cell, but 19 at 27 per cell and a
-// handful in a dense cluster. It pays from cells well above both SPLIT_MIN (16: at 8 per cell the threads are taken anyway)
-// and R. FP64 does so in every chunk: there an instruction occupies the FP64 pipe for 16 clocks whatever its active lanes, and
-// on the 425,984-particle slab (a warp's 32 cells hold 5.8 particles on average, the fullest about 12) 61% of the lanes the
-// pipe was issued were active.
-constexpr int SPLIT_MIN = 16;
-template <class L>
-struct CellSplit {
-    static constexpr int NC = L::nodes;
-    uint16_t n[NC], first[NC]; // per cell: particles, first particle of the chunk
-    uint16_t q0[NC], q1[NC]; // per piece: its particles of the chunk
-    uint8_t cell[NC], part[NC]; // per piece: its cell (0xff: unused), its number in the cell
-    int parts; // most pieces of a cell; 0: not split
-};
-
-// Every thread of the CTA calls it, with its cell's range [qa, qb) of the chunk's cnt particles; only the threads of
-// offset 0 (first) fill the table, which is complete after the call.
-template <class L>
-__device__ __forceinline__ void split_cells(CellSplit<L>& cs, bool first, int c, int qa, int qb, int cnt, int tid)
+// Work of the accumulation's (cell, x-offset) threads where cells hold unequal numbers of particles. A warp's 32 cells take as
+// long as the fullest of them, and a cell without particles leaves its lane idle: so the cells are cut into pieces of at
+// most R particles, a piece per lane, R the smallest count for which the pieces fit (but not so small that the turns of a
+// cell's pieces in the tile take longer than they save). It all happens inside the warp: the cells of an x-offset's two warps
+// (FP32) cover disjoint x of the tile, so no warp touches another's nodes. (Pieces dealt over both warps need shared-memory
+// atomics in the tile: on chunks of 19 crowded cells, 27 particles per cell, that made P2G 198 us, no pieces at all 171, these
+// 142. At 8 per cell they change P2G by less than 1%: 53.4 against 53.5 us at 425,984 particles, 307 against 307 at 3,407,872.)
+// [qa, qb): in the particles of the lane's cell c, out those of its piece. Returns the piece: cell (PIECE_NONE: no piece) | number
+// in the cell << 8 | most pieces of a cell << 20 (0: nothing was cut, the piece is the cell).
+constexpr uint32_t PIECE_NONE = 0xff;
+template <class T>
+__device__ __forceinline__ uint32_t split_cells(int c, int& qa, int& qb)
 {
-    constexpr int NC = L::nodes, PER = NC / 32;
-    if (first) {
-        cs.n[c] = (uint16_t)(qb - qa);
-        cs.first[c] = (uint16_t)qa;
-        cs.cell[c] = 0xff;
-        cs.q0[c] = cs.q1[c] = 0;
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, n = qb - qa;
+    const unsigned occupied = __ballot_sync(all, n > 0);
+    if (occupied == all || occupied == 0) return (uint32_t)c; // no lane to give a piece to
+    const int most = __reduce_max_sync(all, n), cnt = __reduce_add_sync(all, n);
+    if (most <= 2) return (uint32_t)c;
+    int R = max((cnt + 31) / 32, (int)sqrtf((float)most)), p;
+    for (;; R++) { // (R = most always fits: at most one piece per cell)
+        p = (int)(((float)(n + R - 1) + 0.5f) * (1.0f / (float)R)); // ceil(n / R), exact for these sizes
+        if (__reduce_add_sync(all, p) <= 32) break;
     }
-    __syncthreads();
-    if (tid < 32) {
-        int n[PER], cells = 0, most = 0;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-            n[k] = cs.n[tid * PER + k];
-            cells += __popc(__ballot_sync(0xffffffffu, n[k] > 0));
-            most = max(most, n[k]);
-        }
-        most = __reduce_max_sync(0xffffffffu, most);
-        int R = (cnt + NC - 1) / NC, p = 0;
-        for (; cells > 0; R++) { // (R = most always fits: at most one piece per cell)
-            p = 0;
-#pragma unroll
-            for (int k = 0; k < PER; k++) p += (n[k] + R - 1) / R;
-            if (__reduce_add_sync(0xffffffffu, p) <= NC) break;
-        }
-        // FP64's pieces of a cell take turns in the tile, a turn costs about half a particle's accumulation
-        const int parts = cells ? (most + R - 1) / R : 1;
-        const bool split = PER > 1 ? 2 * most > 3 * R : 2 * most > 2 * R + parts - 1;
-        if (!split) p = 0;
-        int x = p;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (tid >= o) x += y;
-        }
-        int s = x - p;
-        if (split)
-#pragma unroll
-            for (int k = 0; k < PER; k++)
-                for (int i = 0, q = cs.first[tid * PER + k]; i * R < n[k] && s < NC; i++, s++) { // (s < NC: by the choice of R)
-                    cs.cell[s] = (uint8_t)(tid * PER + k);
-                    cs.part[s] = (uint8_t)i;
-                    cs.q0[s] = (uint16_t)(q + i * R);
-                    cs.q1[s] = (uint16_t)(q + min(n[k], (i + 1) * R));
-                }
-        if (tid == 0) cs.parts = split ? parts : 0;
+    const int parts = (most + R - 1) / R;
+    // a turn in the tile takes about half a particle's accumulation in FP64 and one in FP32
+    if (sizeof(T) == 8 ? 2 * most <= 2 * R + parts - 1 : most < R + parts + 1) return (uint32_t)c;
+    int x = p; // exclusive offsets of the cells' pieces
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(all, x, o);
+        if (lane >= o) x += y;
     }
-    __syncthreads();
+    const int total = __shfl_sync(all, x, 31);
+    x -= p;
+    int l = 0; // the cell (lane) of piece `lane`: the last one whose pieces start at or before it
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int y = __shfl_sync(all, x, l + o);
+        if (y <= lane) l += o;
+    }
+    const int part = lane - __shfl_sync(all, x, l), q0 = __shfl_sync(all, qa, l), q1 = __shfl_sync(all, qb, l);
+    qa = min(q0 + part * R, q1);
+    qb = min(qa + R, q1);
+    if (lane >= total) {
+        qa = qb = q0;
+        return PIECE_NONE | (uint32_t)parts << 20;
+    }
+    return (uint32_t)((c & ~31) + l) | (uint32_t)part << 8 | (uint32_t)parts << 20;
 }
 
 template <class T, class L>
@@ -1650,7 +1612,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
     T* pay = reinterpret_cast<T*>(fused_dyn);
     __shared__ T tile[OffsetTiles<L>::ELEMS]; // one node tile per stencil x-offset
     __shared__ uint8_t cellof[CHUNK];
-    __shared__ CellSplit<L> s_split;
+    __shared__ uint32_t s_piece[NT];
     // the set-up of the current group (buffer b) and of the next one (b ^ 1): group, scene, a bad neighbour slot,
     // the grid slots of the block and its +1 neighbours, the block origin, the sorted range
     __shared__ int s_g[2], s_scene[2], s_bad[2];
@@ -1732,14 +1694,6 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
             uint32_t js[PER];
 #pragma unroll
             for (int k = 0; k < PER; k++) js[k] = tid + k * NT < cnt ? a.vals_sorted[c0 + tid + k * NT] : 0u;
-            // a cell holds particles q and q + SPLIT_MIN of the chunk for some multiple q of SPLIT_MIN: the cells are crowded
-            // (a cell of 2 SPLIT_MIN particles is always found, one of fewer often)
-            static_assert(CHUNK <= 32 * SPLIT_MIN, "one warp probes the chunk");
-            bool crowded = sizeof(T) == 8;
-            if (sizeof(T) == 4 && tid < 32) {
-                const uint64_t k0 = tid * SPLIT_MIN < cnt ? a.kl.at(a.keys_sorted, c0 + tid * SPLIT_MIN) : ~(uint64_t)tid;
-                crowded = __shfl_down_sync(0xffffffffu, (unsigned long long)k0, 1) == k0 && tid < 31;
-            }
 #pragma unroll
             for (int k = 0; k < PER; k++) {
                 const int q = tid + k * NT;
@@ -1751,7 +1705,7 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 if (!inside) raise_flag(a.st, FLAG_CAPACITY); // keys and positions disagree: abort the substep
                 cellof[q] = inside ? (uint8_t)L::element(l0, l1, l2) : (uint8_t)0xff;
             }
-            bool split = __syncthreads_or(crowded) != 0;
+            __syncthreads();
             if (tid == 0 && c0 == start && claimed < (int)G) cp_async<16>(&s_next, a.item + claimed);
             // ---- phases 2 and 3. Particles of one cell are contiguous and the cells ascend (sorted by cell inside
             // the block): the cell's range by two binary searches over the chunk's cells, no pass or barrier of its
@@ -1766,23 +1720,17 @@ __global__ void __launch_bounds__(FusedShape<T, CH>::NT, MINB) k_p2g_fused(StepA
                 return lo;
             };
             int qa = cell_lower(c), qb = cell_lower(c + 1);
-            if (split) { // crowded cells: pieces of them (the whole CTA decides alike)
-                split_cells<L>(s_split, ii == 0, c, qa, qb, cnt, tid);
-                split = s_split.parts > 0;
-                if (split) {
-                    qa = s_split.q0[c];
-                    qb = s_split.q1[c];
-                }
-            }
+            s_piece[tid] = split_cells<T>(c, qa, qb); // (read back after the accumulation: it holds no register through it)
             NodeAcc<T> acc;
             acc.zero();
             if (nf == NACC)
                 for (int q = qa; q < qb; q++) accumulate_particle<T, CPAD, true>(acc, pay + (q + (q >> 3)), ii);
             else
                 for (int q = qa; q < qb; q++) accumulate_particle<T, CPAD, false>(acc, pay + (q + (q >> 3)), ii);
-            if (split) {
-                const int cell = s_split.cell[c];
-                add_pieces_to_offset_tile<T, L>(acc, tile, cell & (NC - 1), ii, nf, cell < NC, s_split.part[c], s_split.parts);
+            const uint32_t piece = s_piece[tid], parts = piece >> 20; // (parts: the same for the whole warp)
+            if (parts) {
+                const int cell = piece & 0xff;
+                add_pieces_to_offset_tile<T, L>(acc, tile, cell & (NC - 1), ii, nf, cell < NC, (piece >> 8) & 0xfff, (int)parts);
             }
             else
                 add_to_offset_tile<T, L>(acc, tile, c, ii, nf); // all lanes (an empty cell adds zeros)
