@@ -843,7 +843,7 @@ private:
     DevStatus* hst_ = nullptr;
     void *sort_tmp_ = nullptr, *stage_ = nullptr;
     size_t sort_bytes_ = 0, stage_bytes_ = 0;
-    int occ_stress_[4] = { 1, 1, 1, 1 }, occ_scatter_[3] = { 1, 1, 1 }, occ_g2p_[4][3] = { { 1, 1, 1 }, { 1, 1, 1 }, { 1, 1, 1 }, { 1, 1, 1 } };
+    int occ_stress_[4] = { 1, 1, 1, 1 }, occ_scatter_[3] = { 1, 1, 1 }, occ_g2p_[4][3][3] = {}; // [variant][threads][damage], set up at the start
     int occ_fused_[2][4] = { { 1, 1, 1, 1 }, { 1, 1, 1, 1 } }; // [fused variant][model set]
     int occ_ws_[4] = { 1, 1, 1, 1 }; // warp-specialised P2G, per model set
     int occ_grid_ = 1; // grid update CTAs per SM
@@ -1129,8 +1129,6 @@ private:
         g2p_setup<3, 2>();
         for (int& o : occ_scatter_) o = std::max(1, o);
         for (int& o : occ_stress_) o = std::max(1, o);
-        for (auto& row : occ_g2p_)
-            for (int& o : row) o = std::max(1, o);
         sched_.scatter_ctas_per_sm = occ_scatter_[0];
         sched_.tuned = 0;
         if (const char* e = std::getenv("ZR_AUTOTUNE")) autotune_mode_ = std::atoi(e);
@@ -1578,23 +1576,42 @@ private:
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_scatter_[V], k, S::NT, S::dyn_bytes);
     }
-    // G2P variant R = g2p_tight: bit 0 the register budget (G2P_RES), bit 1 the halo staged by bulk copies
+    // G2P variant R = g2p_tight: bit 0 the register budget (G2P_RES), bit 1 the halo staged by bulk copies; per damage D the
+    // batch can have (DRIVE_*; the bulk-copy variants are compiled for any)
+    template <int R, int N, int D>
+    static auto g2p_kernel()
+    {
+        return k_g2p<T, G2P_NT[N], G2P_RES[R & 1], (R >> 1) != 0, (R >> 1) != 0 ? DRIVE_ANY : D>;
+    }
     template <int R, int N>
     void g2p_setup()
     {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N], k_g2p<T, G2P_NT[N], G2P_RES[R & 1], (R >> 1) != 0>, G2P_NT[N], 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_NONE], g2p_kernel<R, N, DRIVE_NONE>(), G2P_NT[N], 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_BORDEN], g2p_kernel<R, N, DRIVE_BORDEN>(), G2P_NT[N], 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_ANY], g2p_kernel<R, N, DRIVE_ANY>(), G2P_NT[N], 0);
+        for (int& o : occ_g2p_[R][N]) o = std::max(1, o);
+    }
+    int drive() const { return !any_damage_ ? DRIVE_NONE : ((models_ & (1 << MODEL_QR_STABLE_NEOHOOKEAN)) ? DRIVE_ANY : DRIVE_BORDEN); }
+    template <int R, int N>
+    void launch_g2p_n(const StepArgs<T>& a)
+    {
+        const int d = drive(), ctas = nsm_ * occ_g2p_[R][N][d];
+        if (d == DRIVE_NONE)
+            g2p_kernel<R, N, DRIVE_NONE>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
+        else if (d == DRIVE_BORDEN)
+            g2p_kernel<R, N, DRIVE_BORDEN>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
+        else
+            g2p_kernel<R, N, DRIVE_ANY>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
     }
     template <int R>
     void launch_g2p(const StepArgs<T>& a, int gi)
     {
-        constexpr int RES = G2P_RES[R & 1];
-        constexpr bool BULK = (R >> 1) != 0;
         if (gi == 0)
-            k_g2p<T, G2P_NT[0], RES, BULK><<<nsm_ * occ_g2p_[R][0], G2P_NT[0], 0, stream_>>>(a);
+            launch_g2p_n<R, 0>(a);
         else if (gi == 1)
-            k_g2p<T, G2P_NT[1], RES, BULK><<<nsm_ * occ_g2p_[R][1], G2P_NT[1], 0, stream_>>>(a);
+            launch_g2p_n<R, 1>(a);
         else
-            k_g2p<T, G2P_NT[2], RES, BULK><<<nsm_ * occ_g2p_[R][2], G2P_NT[2], 0, stream_>>>(a);
+            launch_g2p_n<R, 2>(a);
     }
     template <int M, int V>
     void fused_setup(int slot)

@@ -2203,9 +2203,13 @@ __device__ __forceinline__ void gather(const Quad<T>* tv, const Quad<T>* te, con
 // BULK: the 8 neighbouring blocks' velocities reach shared memory by bulk asynchronous copies (one 4-field block of
 // NVEL * nodes values per copy, completing on an mbarrier) and the node tile is built from there; otherwise each
 // thread loads its tile nodes from global memory
-template <class T, int NT, int RESIDENT, bool BULK = false>
+// DRIVE: the damage the batch's scenes can have: none, on the Borden model only, any (the drive of the QR-stable model brings a
+// QR factorisation and a polar decomposition into the kernel)
+enum { DRIVE_NONE = 0, DRIVE_BORDEN = 1, DRIVE_ANY = 2 };
+template <class T, int NT, int RESIDENT, bool BULK = false, int DRIVE = DRIVE_ANY>
 __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
 {
+    constexpr bool QR = DRIVE == DRIVE_ANY;
     using L = typename LayoutOf<T>::type;
     using GS = G2pStage<T, NT>;
     constexpr int BLK = NVEL * L::nodes; // values of one block's velocity fields (1 KB in both precisions)
@@ -2261,7 +2265,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         }
         __syncthreads();
         const SceneParams<T>& sp = a.scenes[s_scene];
-        const bool damage = sp.damage != 0;
+        const bool damage = DRIVE != DRIVE_NONE && sp.damage != 0;
         const Pool<T>& P = a.pin;
         const Pool<T>& Q = a.pout;
         const uint32_t i0 = start + threadIdx.x;
@@ -2333,7 +2337,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
         const T dx2 = dx * dx, half_cfl2 = dx2 * (T)0.25 * (sp.cfl * sp.cfl);
         // scene constants in registers: read through sp inside the loop they would be re-read after every store
         const int key_cells = sp.domain_cells - 3, n_mat = sp.n_materials;
-        const bool implicit = sp.implicit != 0;
+        const bool implicit = DRIVE != DRIVE_NONE && sp.implicit != 0;
         uint32_t flags = 0;
         // storage slots run one particle ahead of the state: with staging the next particle's state is copied
         // while this one computes; without, its slot is known when its loads issue (one latency, not two)
@@ -2389,7 +2393,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
             {
                 const int col = l[0] * TY + l[1];
                 const Quad<T>*pv0 = tv + col * Z1 + l[2], *pe0 = te + col * Z2 + l[2];
-                if (sizeof(T) == 4 || damage) // FP32 carries the phase field in the fourth lane anyway (zero without damage)
+                if ((sizeof(T) == 4 && DRIVE != DRIVE_NONE) || damage) // FP32 carries the phase field in the fourth lane anyway (zero without damage)
                     gather<T, L, true>(pv0, pe0, w, dw, fr[2], gt);
                 else
                     gather<T, L, false>(pv0, pe0, w, dw, fr[2], gt);
@@ -2483,12 +2487,12 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
 #pragma unroll
                         for (int c = 0; c < 9; c++) Fn[c] = Q.f[(P_F + c) * Q.stride + i];
                         bool fb = false;
-                        Q.f[P_DRV * Q.stride + i] = damage_drive(mt, Fn, sc, fb);
+                        Q.f[P_DRV * Q.stride + i] = damage_drive<T, QR>(mt, Fn, sc, fb);
                         if (fb) atomicAdd(&a.st->fallback, 1u);
                     }
                     else {
                         bool fb = false;
-                        dd = damage_update(mt, F, dd, lap, sc, dt, fb);
+                        dd = damage_update<T, QR>(mt, F, dd, lap, sc, dt, fb);
                         if (fb) atomicAdd(&a.st->fallback, 1u);
                     }
                     if (nonfinite(dd)) flags |= FLAG_NONFINITE;

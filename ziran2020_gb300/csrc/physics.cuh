@@ -145,22 +145,23 @@ ZR_HD double rcbrt_(double x)
 #endif
 }
 
-ZR_HD void sincos_(float x, float& s, float& c)
+// sine and cosine of pi x (no reduction of large arguments, whose code needs local memory)
+ZR_HD void sincospi_(float x, float& s, float& c)
 {
 #if defined(__CUDA_ARCH__)
-    sincosf(x, &s, &c);
+    sincospif(x, &s, &c);
 #else
-    s = std::sin(x);
-    c = std::cos(x);
+    s = std::sin((float)M_PI * x);
+    c = std::cos((float)M_PI * x);
 #endif
 }
-ZR_HD void sincos_(double x, double& s, double& c)
+ZR_HD void sincospi_(double x, double& s, double& c)
 {
 #if defined(__CUDA_ARCH__)
-    sincos(x, &s, &c);
+    sincospi(x, &s, &c);
 #else
-    s = std::sin(x);
-    c = std::cos(x);
+    s = std::sin(M_PI * x);
+    c = std::cos(M_PI * x);
 #endif
 }
 
@@ -440,10 +441,9 @@ ZR_HD void tension_part(const T* S, T* Sp)
         const T B00 = a * ip, B11 = b * ip, B22 = c * ip, B01 = s01 * ip, B02 = s02 * ip, B12 = s12 * ip;
         T r = (T)0.5 * (B00 * (B11 * B22 - B12 * B12) - B01 * (B01 * B22 - B12 * B02) + B02 * (B01 * B12 - B11 * B02));
         r = r < (T)-1 ? (T)-1 : (r > (T)1 ? (T)1 : r);
-        const T phi = acos(r) * ((T)1 / (T)3);
-        // cos(phi + 2 pi / 3) = -cos(phi) / 2 - sqrt(3) / 2 sin(phi)
+        // phi = acos(r) / 3, and cos(phi + 2 pi / 3) = -cos(phi) / 2 - sqrt(3) / 2 sin(phi)
         T sphi, cphi;
-        sincos_(phi, sphi, cphi);
+        sincospi_(acos(r) * (T)0.10610329539459689, sphi, cphi);
         l1 = q + (T)2 * p * cphi;
         l3 = q - p * (cphi + (T)1.7320508075688772935 * sphi);
         l2 = (T)3 * q - l1 - l3;
@@ -636,11 +636,12 @@ ZR_HD T degradation(T d, T k)
 // R^T A R = I + alpha e1 e1^T = diag(w) with w = (1 + alpha, 1, 1). So phi sigma_c^2 = sum_ij w_i w_j (sigma~+_ij)^2.
 // This is the same quantity with different rounding. The QR-stable model's fibre term makes its stress
 // anisotropic, so it keeps the polar rotation.
-template <class T>
+// QR = false: no material of the scenes has the QR-stable model (its stress and the polar rotation drop out of the code).
+template <class T, bool QR = true>
 ZR_HD T damage_drive(const Material<T>& mt, const T* F, T sigma_c, bool& fallback)
 {
     T tau[9], invJ;
-    const bool qr = mt.model == MODEL_QR_STABLE_NEOHOOKEAN;
+    const bool qr = QR && mt.model == MODEL_QR_STABLE_NEOHOOKEAN;
     if (qr) {
         invJ = (T)1 / tau_qrnh(mt, F, (T)1, tau, true); // cauchy = P F^T / J with J from the QR (QRStableNeoHookean.h:86-96)
     }
@@ -689,7 +690,7 @@ ZR_HD T damage_drive(const Material<T>& mt, const T* F, T sigma_c, bool& fallbac
 
 // Explicit AnisoMPM damage update of one particle (AnisoFractureSimulation.h:210-283, :365-391) with one
 // structural director a0 = e1 rotated by the polar R of F. Returns the new damage.
-template <class T>
+template <class T, bool QR = true>
 ZR_HD T damage_update(const Material<T>& mt, const T* F, T d, T lap, T sigma_c, T dt, bool& fallback)
 {
     // fully damaged: d + (dt/eta) <...> >= d >= 1 and the update is capped at 1, whatever the drive is
@@ -698,7 +699,7 @@ ZR_HD T damage_update(const Material<T>& mt, const T* F, T d, T lap, T sigma_c, 
         return (T)1;
     }
     T geo = d - mt.l0 * mt.l0 * lap;
-    T dtilde = damage_drive(mt, F, sigma_c, fallback);
+    T dtilde = damage_drive<T, QR>(mt, F, sigma_c, fallback);
     T diff = ((T)1 - d) * dtilde - geo;
     T nd = d + (dt / mt.eta) * (diff > (T)0 ? diff : (T)0);
     return nd < (T)1 ? nd : (T)1;
