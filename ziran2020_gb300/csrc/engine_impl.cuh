@@ -838,8 +838,8 @@ __global__ void k_nbr(StepArgs<T> a)
 // Payload storage: field k of sorted particle q at pay[k * pstride + q + q/8]. The gap after every 8
 // particles carries over into shared memory with the copy and staggers the shared-memory banks of the
 // consumer lanes (one lane per cell, ~8 particles per cell).
-// The Kirchhoff stress of every model here is symmetric (the energies are frame-indifferent), so K keeps its
-// upper triangle, each off-diagonal entry the mean of the two that were computed: six fields instead of nine,
+// The Kirchhoff stress of every model here is symmetric (the energies are frame-indifferent), so K is
+// its upper triangle: six fields instead of nine,
 // three shared-memory loads fewer per particle and stencil x-offset in the accumulation.
 // ---------------------------------------------------------------------------------------------------
 //
@@ -904,8 +904,8 @@ __device__ __forceinline__ void particle_payload(const Pool<T>& P, uint32_t j, c
         fr[e] = xs - (T)b[e];
     }
     using Y = Pay<T>;
-    const T kf = -dt * V0 * inv_dx, hk = (T)0.5 * kf;
-    const T K[6] = { kf * tau[0], hk * (tau[1] + tau[3]), hk * (tau[2] + tau[6]), kf * tau[4], hk * (tau[5] + tau[7]), kf * tau[8] };
+    const T kf = -dt * V0 * inv_dx;
+    const T K[6] = { kf * tau[0], kf * tau[1], kf * tau[2], kf * tau[4], kf * tau[5], kf * tau[8] };
     y[Y::M * S] = mass;
     y[Y::D * S] = dd;
     if constexpr (sizeof(T) == 4) {

@@ -128,6 +128,13 @@ ZR_HD void mul3_bt(const T* A, const T* B, T* R) // A B^T
         for (int c = 0; c < 3; c++) R[3 * r + c] = A[3 * r] * B[3 * c] + A[3 * r + 1] * B[3 * c + 1] + A[3 * r + 2] * B[3 * c + 2];
 }
 
+template <class T>
+ZR_HD void sym3_bt(const T* A, const T* B, T* R) // A B^T where it is symmetric: the upper triangle, mirrored
+{
+    for (int r = 0; r < 3; r++)
+        for (int c = r; c < 3; c++) R[3 * r + c] = R[3 * c + r] = A[3 * r] * B[3 * c] + A[3 * r + 1] * B[3 * c + 1] + A[3 * r + 2] * B[3 * c + 2];
+}
+
 ZR_HD float rcbrt_(float x)
 {
 #if defined(__CUDA_ARCH__)
@@ -478,13 +485,16 @@ ZR_HD void tension_part(const T* S, T* Sp)
 template <class T>
 ZR_HD bool tau_corotated(const Material<T>& mt, const T* F, T* tau)
 {
-    T R[9], Cf[9], P[9];
+    T R[9];
     bool fb = polar_rotation(F, R);
-    cofactor3(F, Cf);
     T J = det3(F);
-    T a = (T)2 * mt.mu, b = mt.lambda * (J - (T)1);
-    for (int i = 0; i < 9; i++) P[i] = a * (F[i] - R[i]) + b * Cf[i];
-    mul3_bt(P, F, tau);
+    // J F^{-T} F^T = J, and (F - R) F^T is symmetric (R S = F): six products with the small difference F - R
+    T a = (T)2 * mt.mu, b = mt.lambda * (J - (T)1) * J;
+    for (int i = 0; i < 9; i++) R[i] = a * (F[i] - R[i]);
+    sym3_bt(R, F, tau);
+    tau[0] += b;
+    tau[4] += b;
+    tau[8] += b;
     return fb;
 }
 
@@ -614,7 +624,7 @@ ZR_HD T tau_qrnh(const Material<T>& mt, const T* F, T g, T* tau, bool effective 
         }
     T QA[9];
     mul3(Q, A, QA);
-    mul3_bt(QA, Q, tau);
+    sym3_bt(QA, Q, tau);
     return J;
 }
 
