@@ -1295,7 +1295,8 @@ double scene_bytes(int precision, int64_t n)
 {
     const double s = precision == ZR_F64 ? 8 : 4, nodes = precision == ZR_F64 ? 32 : 64;
     // two pool copies (30 fields and the id), keys (in, sorted), sort values, iota, group starts, the P2G payload
-    // (27 fields at 9/8 density) and the incremental sort's six index and key lists
+    // (27 fields at 9/8 density: room for FP32's 24; FP64 keeps 4 unless a schedule asks for a split P2G form) and the
+    // incremental sort's lists (movers' keys and indices by bucket; 24 B a particle leaves room for its per-tile words)
     const double per_particle = 2 * (30 * s + 4) + 8 + 8 + 4 + 4 + 4 + 27 * s * 9 / 8 + 6 * 4;
     const double groups = (double)n / (nodes * 4) + 64;
     return n * per_particle + 8 * groups * (10 * nodes * s + 64);

@@ -148,15 +148,16 @@ public:
             pid_[1] = grown_pid[1];
             cap_ = (uint64_t)cap;
             pay_ = nullptr;
+            pay_fields_ = payload_fields();
             sort_aux_ = nullptr;
             inc_bkey_ = inc_bidx_ = nullptr;
-            // P2G payload: Pay<T>::N fields of sorted particles at q + q/8, plus the copy granularity at the end
+            // P2G payload: fields of sorted particles at q + q/8, plus the copy granularity at the end
             pstride_ = (int64_t)((pay_pos((uint64_t)cap) + 64 + 63) & ~(uint64_t)63);
             if (alloc((void**)&keys_in_, 8 * cap) || alloc((void**)&keys_sorted_, 8 * cap) || alloc((void**)&iota_, 4 * cap)
-                || alloc((void**)&vals_sorted_, 4 * cap) || alloc((void**)&g_start_, 4 * cap) || alloc((void**)&pay_, sizeof(T) * Pay<T>::N * (size_t)pstride_)
+                || alloc((void**)&vals_sorted_, 4 * cap) || alloc((void**)&g_start_, 4 * cap) || alloc((void**)&pay_, sizeof(T) * pay_fields_ * (size_t)pstride_)
                 || alloc((void**)&sort_aux_, sort_aux_bytes(cap)) || alloc((void**)&inc_bkey_, 4 * bucket_slots(cap)) || alloc((void**)&inc_bidx_, 4 * bucket_slots(cap)))
                 return ZR_ERR_CUDA_;
-            ZR_CUDA(cudaMemsetAsync(pay_, 0, sizeof(T) * Pay<T>::N * (size_t)pstride_, stream_));
+            ZR_CUDA(cudaMemsetAsync(pay_, 0, sizeof(T) * pay_fields_ * (size_t)pstride_, stream_));
             ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes(cap), stream_));
             k_iota<T><<<nsm_ * 4, 256, 0, stream_>>>(iota_, (uint32_t)cap);
             size_t sb = 0, sb32 = 0;
@@ -275,6 +276,7 @@ public:
     // An aborted substep is retried after growing the grid (capacity) or reported with the state left at its start.
     int run_steps(int nsteps, StepReport& r, int& done)
     {
+        if (int rc = ensure_payload()) return rc;
         if (int rc = refresh_drive()) return rc;
         const int target = done + nsteps;
         int grow_rounds = 0;
@@ -867,6 +869,7 @@ private:
     uint64_t inv_cap_ = 0;
     T* pay_ = nullptr;
     int64_t pstride_ = 0;
+    size_t pay_fields_ = 0; // fields pay_ has room for
     Schedule sched_{ 0, VAR_CHUNK[0], VAR_NBUF[0], 2, 128, 0, 0 };
     int autotune_mode_ = 1; // 0 off (defaults), 1 on (cached), 2 always re-tune on a new batch
     bool tuned_ = false;
@@ -1129,8 +1132,7 @@ private:
         g2p_setup<3, 2>();
         for (int& o : occ_scatter_) o = std::max(1, o);
         for (int& o : occ_stress_) o = std::max(1, o);
-        sched_.scatter_ctas_per_sm = occ_scatter_[0];
-        sched_.tuned = 0;
+        sched_ = default_schedule();
         if (const char* e = std::getenv("ZR_AUTOTUNE")) autotune_mode_ = std::atoi(e);
         if (const char* e = std::getenv("ZR_SORT")) inc_sort_on_ = std::string(e) != "full";
         if (const char* e = std::getenv("ZR_PREFETCH")) prefetch_ = std::atoi(e) != 0;
@@ -1328,7 +1330,8 @@ private:
             ZR_CUDA(bin_incremental(n, a));
             if (ev) ZR_CUDA(cudaEventRecord(ev[1], stream_)); // the merge also activates the blocks: both in the first phase
         }
-        if (sched_.fused == 0 || sched_.fused == 3) // these P2G forms read grid slots; the fused one translates its groups' entries
+        if (reads_payload() && pay_fields_ < (size_t)Pay<T>::N) return fail(ZR_ERR_STATE_, "P2G payload not allocated");
+        if (reads_payload()) // these P2G forms read grid slots; the fused one translates its groups' entries
             k_nbr<T><<<nsm_ * 4, 256, 0, stream_>>>(a);
         if (ev) ZR_CUDA(cudaEventRecord(ev[2], stream_));
         if (sched_.fused == 3)
@@ -1745,7 +1748,33 @@ private:
         return false;
     }
 
-    Schedule default_schedule() const { return Schedule{ 0, VAR_CHUNK[0], VAR_NBUF[0], occ_scatter_[0], G2P_NT[1], 0, 0 }; }
+    // In FP64 only an explicit schedule takes a split P2G form: its payload in HBM is 41 fields, 369 B a particle on top of the
+    // ~530 of everything else, for a kernel the FP64 pipe bounds either way (the tuned 426k slab's pass the same without the split
+    // candidates: 1.002x).
+    static constexpr bool SPLIT_TRIED = sizeof(T) == 4;
+    Schedule default_schedule() const
+    {
+        if (!SPLIT_TRIED) return Schedule{ fused_code(1), FUSED_CH[1], 0, occ_fused_[1][models_slot()], G2P_NT[1], 0, 0 };
+        return Schedule{ 0, VAR_CHUNK[0], VAR_NBUF[0], occ_scatter_[0], G2P_NT[1], 0, 0 };
+    }
+    bool reads_payload() const { return sched_.fused == 0 || sched_.fused == 3; }
+    // the implicit damage solve's scratch, or the payload of a schedule that reads it
+    size_t payload_fields() const { return SPLIT_TRIED || reads_payload() ? Pay<T>::N : DS_NF; }
+    // before a run: the schedule may have been set since the buffer was made
+    int ensure_payload()
+    {
+        if (!cap_ || pay_fields_ >= payload_fields()) return 0;
+        drop_graphs();
+        void* p = pay_;
+        dfree(p);
+        pay_ = nullptr;
+        pay_fields_ = 0;
+        const size_t bytes = sizeof(T) * payload_fields() * (size_t)pstride_;
+        if (alloc((void**)&pay_, bytes)) return ZR_ERR_CUDA_;
+        ZR_CUDA(cudaMemsetAsync(pay_, 0, bytes, stream_));
+        pay_fields_ = payload_fields();
+        return 0;
+    }
 
     int autotune_trials()
     {
@@ -1760,14 +1789,14 @@ private:
         ZR_CUDA(cudaMemcpyAsync(scenes_backup_, d_scenes_, sb, cudaMemcpyDeviceToDevice, stream_));
         // P2G candidates with the default G2P, then G2P candidates with the chosen P2G
         std::vector<Schedule> p2g_c;
-        for (int vi = 0; vi < 3; vi++)
+        for (int vi = 0; SPLIT_TRIED && vi < 3; vi++)
             for (int c = occ_scatter_[vi]; c >= std::max(1, occ_scatter_[vi] - 1); c--)
                 p2g_c.push_back(Schedule{ 0, VAR_CHUNK[vi], VAR_NBUF[vi], c, G2P_NT[1], 0, 1 });
         for (int fv = 0; fv < 2; fv++) {
             const int of = occ_fused_[fv][models_slot()];
             for (int c = of; c >= std::max(1, of - 1); c--) p2g_c.push_back(Schedule{ fused_code(fv), FUSED_CH[fv], 0, c, G2P_NT[1], 0, 1 });
         }
-        {
+        if (SPLIT_TRIED) {
             const int ow = occ_ws_[models_slot()];
             for (int c = ow; c >= std::max(1, ow - 1); c--) p2g_c.push_back(Schedule{ 3, WsShape<T>::CHUNK, WsShape<T>::NSTAGE, c, G2P_NT[1], 0, 1 });
         }
@@ -1868,6 +1897,7 @@ private:
         sort_tmp_ = stage_ = nullptr;
         stage_bytes_ = 0;
         pay_ = nullptr;
+        pay_fields_ = 0;
         pstride_ = 0;
         cg_ = nullptr;
         cgs_ = nullptr;

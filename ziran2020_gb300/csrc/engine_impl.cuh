@@ -2542,7 +2542,7 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
 // batch runs the iterations it would run alone. G2P then adds sum_i w_ip (x_i - pf_i) to the damage.
 // ---------------------------------------------------------------------------------------------------
 enum { CG_SA = 0, CG_SV, CG_DIAG, CG_X, CG_R, CG_Z, CG_P, CG_AP, CG_NF }; // node vectors
-enum { DS_F = 0, DS_E = 3 }; // particle scratch fields in the payload buffer: fractional position, e_p
+enum { DS_F = 0, DS_E = 3, DS_NF = 4 }; // particle scratch fields in the payload buffer: fractional position, e_p
 constexpr int CG_MAX_ITERATIONS = 100;
 
 template <class T>
