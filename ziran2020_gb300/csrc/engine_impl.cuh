@@ -2666,7 +2666,10 @@ struct DmgShape {
     static constexpr int NT = 3 * L::nodes;
     static constexpr int CHUNK = 512;
     static constexpr int NS = 6; // staged values per particle
-    static constexpr int MINB = 4; // CTAs per SM the registers are cut for: these kernels wait on memory
+    // CTAs per SM the registers are cut for. These kernels wait on memory (loads 5.5 of 13 cycles per issued instruction in
+    // k_dmg_rhs), and in FP32 4 / 5 / 6 CTAs cost 79 / 64 / 56 registers with 0 / 8 / 12 bytes of spill (7: 184): per substep
+    // 3,407,872 particles 1057 / 1013 / 995 us, 425,984 215.8 / 208.5 / 209.7. FP64 waits on its pipe: 956 / - / 955.
+    static constexpr int MINB = sizeof(T) == 4 ? 6 : 4;
 };
 
 // v[i] by selects (an index that varies at run time puts the array into local memory)
