@@ -327,11 +327,17 @@ __device__ __forceinline__ float newton_step<float>(float* X, float* Cf, float a
 }
 #endif
 
+// The Newton step's scale 1 / cbrt(det X), which only speeds convergence up: on an X whose singular values are 1 / g to
+// within e it returns R (I + e^2 / 2). In FP64 it comes from FP32, whose root is off by up to 1.2e-7 (e^2 / 2 = 7e-15, tens of
+// FP64 units), so the steps whose result is returned take no scale: the last one moves X by less than polar_tol = 1e-8, so
+// det X rounds to one in FP32 and its root is one but for its own error, less than 4e-7. (The errors of earlier steps are
+// squared by the later ones.)
 ZR_HD float newton_scale(float J) { return rcbrt_(J); }
 ZR_HD double newton_scale(double J)
 {
-    // det F within the condition bound, but beyond FP32's range: the FP64 root
-    return J > 1e-30 && J < 1e30 ? (double)rcbrt_((float)J) : rcbrt_(J);
+    if (!(J > 1e-30 && J < 1e30)) return rcbrt_(J); // det F within the condition bound, but beyond FP32's range: the FP64 root
+    const float g = rcbrt_((float)J);
+    return fabsf(g - 1.0f) < 4e-7f ? 1.0 : (double)g;
 }
 
 // The FP64 path of polar_rotation, kept out of line: it is rare, and inlining it into every kernel that
@@ -363,7 +369,6 @@ ZR_HD bool polar_rotation(const T* F, T* R)
         // Frobenius condition number ||F|| ||F^-1|| = sqrt(nf nc) / J
         if (J > 0 && nf * nc < (Eps<T>::polar_kappa * Eps<T>::polar_kappa) * (J * J)) {
             for (int it = 0; it < Eps<T>::polar_iters; it++) {
-                // the scaling only speeds convergence up, so FP64 takes it from FP32 (any g that enters both terms alike serves)
                 const T g = newton_scale(J);
                 T a = (T)0.5 * g, b = (T)0.5 / (g * J);
                 const T diff = newton_step(X, Cf, a, b);
