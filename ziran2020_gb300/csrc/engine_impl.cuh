@@ -2931,7 +2931,7 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_appl
                         g2 += w[0][i] * sC;
                     }
                     const T sgc = ev * inv_dx * inv_dx; // both gradients carry 1/dx
-                    energy += (double)(sgc * (g0 * g0 + g1 * g1 + g2 * g2));
+                    energy += gradient_share(sgc, g0, g1, g2);
                     g0 *= sgc;
                     g1 *= sgc;
                     g2 *= sgc;
@@ -3084,7 +3084,7 @@ __global__ void __launch_bounds__(CG_NT) k_cg_nodes(StepArgs<T> a, cudaGraphCond
                     *p = zz;
                     *Ap = 0;
                     acc = (double)rhs * (double)zz;
-                    dsum = on ? (double)(diag * zz) * (double)zz : 0.0;
+                    dsum = on ? diagonal_share(diag, zz) : 0.0;
                 }
                 else if (STAGE == CG_STEP) {
                     const T alpha = (T)cs.alpha;
@@ -3099,7 +3099,7 @@ __global__ void __launch_bounds__(CG_NT) k_cg_nodes(StepArgs<T> a, cudaGraphCond
                 else if (STAGE == CG_DIR) {
                     const T pn = zv + (T)cs.beta * pv;
                     *p = pn;
-                    dsum = on ? (double)(diag * pn) * (double)pn : 0.0;
+                    dsum = on ? diagonal_share(diag, pn) : 0.0;
                 }
                 else {
                     *pf = on ? xv - pfv : (T)0;

@@ -393,6 +393,16 @@ ZR_HD bool polar_rotation(const T* F, T* R)
     return true;
 }
 
+// Shares of p . A p in the implicit damage solve's step length: a particle's s |g|^2 (g: the direction's gradient there) and
+// a node's diagonal term. Every product is taken in FP64, as FP32 ones would round before the sum.
+template <class T>
+ZR_HD double gradient_share(T s, T g0, T g1, T g2)
+{
+    return (double)s * ((double)g0 * (double)g0 + (double)g1 * (double)g1 + (double)g2 * (double)g2);
+}
+template <class T>
+ZR_HD double diagonal_share(T diag, T p) { return (double)diag * (double)p * (double)p; }
+
 // Tensile part sigma+ = sum_i <lambda_i>_+ q_i q_i^T of a symmetric 3x3 matrix (the quantity
 // AnisoFractureSimulation.h:240-254 builds from an eigen-decomposition). Eigenvalues come from the
 // trigonometric closed form; at most one eigenvector is needed: with one positive eigenvalue
