@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <unordered_map>
 
 #define ZR_CUDA(call)                                                                                      \
     do {                                                                                                   \
@@ -138,19 +139,14 @@ public:
                 ZR_CUDA(cudaMemcpyAsync(grown_pid[0] + np[q].first, old_pid + src_first[q], 4 * np[q].count, cudaMemcpyDeviceToDevice, stream_));
             }
             ZR_CUDA(cudaStreamSynchronize(stream_));
-            void* olds[] = { pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, sort_tmp_, pay_,
-                sort_aux_, inc_bkey_, inc_bidx_ };
-            for (void* p : olds)
-                if (p) cudaFree(p);
+            dfree(pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, sort_tmp_, pay_, sort_aux_, inc_bkey_,
+                inc_bidx_);
             pool_[0] = grown_pool[0];
             pool_[1] = grown_pool[1];
             pid_[0] = grown_pid[0];
             pid_[1] = grown_pid[1];
             cap_ = (uint64_t)cap;
-            pay_ = nullptr;
             pay_fields_ = payload_fields();
-            sort_aux_ = nullptr;
-            inc_bkey_ = inc_bidx_ = nullptr;
             // P2G payload: fields of sorted particles at q + q/8, plus the copy granularity at the end
             pstride_ = (int64_t)((pay_pos((uint64_t)cap) + 64 + 63) & ~(uint64_t)63);
             if (alloc((void**)&keys_in_, 8 * cap) || alloc((void**)&keys_sorted_, 8 * cap) || alloc((void**)&iota_, 4 * cap)
@@ -179,15 +175,7 @@ public:
         }
         // per-scene device arrays
         if (np.size() > scene_cap_) {
-            void* p1 = d_scenes_;
-            dfree(p1);
-            void* p2 = grid_mass_;
-            dfree(p2);
-            void* p3 = cgs_;
-            dfree(p3);
-            d_scenes_ = nullptr;
-            grid_mass_ = nullptr;
-            cgs_ = nullptr;
+            dfree(d_scenes_, grid_mass_, cgs_);
             scene_cap_ = std::max<size_t>(np.size(), 2 * scene_cap_);
             if (alloc((void**)&d_scenes_, sizeof(SceneParams<T>) * scene_cap_) || alloc((void**)&grid_mass_, 8 * scene_cap_)
                 || alloc((void**)&cgs_, sizeof(CgScalars) * scene_cap_))
@@ -222,14 +210,11 @@ public:
         for (size_t q = 0; q < add.size(); q++) {
             int rc = upload_scene(*add[q], h_scenes_[first_new + q].first, dst, d_mat, buf);
             if (rc) {
-                cudaFree(d_mat);
+                dfree(d_mat);
                 return rc;
             }
         }
-        if (d_mat) {
-            cudaFree(d_mat);
-            dev_bytes_ -= (int64_t)max_add;
-        }
+        dfree(d_mat);
         // keys, and a first binning pass that sizes the grid (every group activates at most 8 blocks)
         k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, nullptr);
         ZR_CUDA(sort_keys((int64_t)N_));
@@ -347,9 +332,7 @@ public:
     int fill_inv(int s)
     {
         if (!inv_ || inv_cap_ < cap_) {
-            void* old = inv_;
-            dfree(old);
-            inv_ = nullptr;
+            dfree(inv_);
             inv_cap_ = 0;
             if (alloc((void**)&inv_, 4 * (size_t)cap_)) return ZR_ERR_CUDA_;
             inv_cap_ = cap_;
@@ -603,9 +586,7 @@ public:
     void free_io()
     {
         for (int b = 0; b < 2; b++) {
-            dfree(io_in_[b]);
-            dfree(io_out_[b]);
-            io_in_[b] = io_out_[b] = nullptr;
+            dfree(io_in_[b], io_out_[b]);
         }
         io_bytes_ = 0;
     }
@@ -647,9 +628,7 @@ public:
         if (!N_) return fail(ZR_ERR_STATE_, "no scenes loaded");
         const size_t pool_b = sizeof(T) * P_NF * (size_t)cap_, pid_b = 4 * (size_t)cap_, sc_b = sizeof(SceneParams<T>) * h_scenes_.size();
         if (!ck_pool_ || ck_cap_ != cap_ || ck_scenes_n_ < h_scenes_.size()) {
-            dfree(ck_pool_);
-            dfree(ck_pid_);
-            dfree(ck_scenes_);
+            dfree(ck_pool_, ck_pid_, ck_scenes_);
             if (alloc(&ck_pool_, pool_b) || alloc(&ck_pid_, pid_b) || alloc(&ck_scenes_, sc_b)) return ZR_ERR_CUDA_;
             ck_cap_ = cap_;
             ck_scenes_n_ = h_scenes_.size();
@@ -897,7 +876,8 @@ private:
     std::vector<cudaEvent_t> ev_;
     cudaEvent_t t0_ = nullptr, t1_ = nullptr;
     KernelTimes kt_;
-    int64_t dev_bytes_ = 0;
+    int64_t dev_bytes_ = 0; // held by the allocations listed in alloc_bytes_
+    std::unordered_map<void*, size_t> alloc_bytes_;
 
     Pool<T> pool(int which) const { return Pool<T>{ pool_[which], pid_[which], (int64_t)cap_ }; }
 
@@ -1148,6 +1128,7 @@ private:
             return ZR_ERR_CUDA_;
         }
         dev_bytes_ += (int64_t)bytes;
+        alloc_bytes_[*p] = bytes;
         return 0;
     }
     int cuda_fail(cudaError_t e)
@@ -1155,45 +1136,26 @@ private:
         err_ = std::string("CUDA error: ") + cudaGetErrorString(e);
         return ZR_ERR_CUDA_;
     }
-    void dfree(void*& p)
+    template <class... P>
+    void dfree(P*&... p)
     {
-        if (p) cudaFree(p);
-        p = nullptr;
+        (free_one(p), ...);
+        ((p = nullptr), ...);
+    }
+    void free_one(void* p)
+    {
+        if (!p) return;
+        cudaFree(p);
+        const auto it = alloc_bytes_.find(p);
+        if (it == alloc_bytes_.end()) return;
+        dev_bytes_ -= (int64_t)it->second;
+        alloc_bytes_.erase(it);
     }
 
     int alloc_grid(uint32_t cap)
     {
         drop_graphs();
-        void* p;
-        p = g_nbr_;
-        dfree(p);
-        p = b_key_;
-        dfree(p);
-        p = acc_;
-        dfree(p);
-        p = vel_;
-        dfree(p);
-        p = h_keys_;
-        dfree(p);
-        p = h_vals_;
-        dfree(p);
-        p = item_;
-        dfree(p);
-        p = i_slot_;
-        dfree(p);
-        p = open_;
-        dfree(p);
-        p = cg_;
-        dfree(p);
-        cg_ = nullptr;
-        item_ = nullptr;
-        open_ = nullptr;
-        i_slot_ = nullptr;
-        g_nbr_ = nullptr;
-        b_key_ = nullptr;
-        acc_ = vel_ = nullptr;
-        h_keys_ = nullptr;
-        h_vals_ = nullptr;
+        dfree(g_nbr_, b_key_, acc_, vel_, h_keys_, h_vals_, item_, i_slot_, open_, cg_);
         b_cap_ = cap;
         uint32_t hs = 1;
         while (hs < 4 * cap) hs <<= 1;
@@ -1765,9 +1727,7 @@ private:
     {
         if (!cap_ || pay_fields_ >= payload_fields()) return 0;
         drop_graphs();
-        void* p = pay_;
-        dfree(p);
-        pay_ = nullptr;
+        dfree(pay_);
         pay_fields_ = 0;
         const size_t bytes = sizeof(T) * payload_fields() * (size_t)pstride_;
         if (alloc((void**)&pay_, bytes)) return ZR_ERR_CUDA_;
@@ -1877,42 +1837,16 @@ private:
         if (h2d_) cudaStreamSynchronize(h2d_);
         if (d2h_) cudaStreamSynchronize(d2h_);
         free_io();
-        void* ps[] = { pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, g_nbr_, b_key_, acc_, vel_, h_keys_, h_vals_,
-            d_scenes_, grid_mass_, st_, sort_tmp_, stage_, pay_, scenes_backup_, ck_pool_, ck_pid_, ck_scenes_, cg_, cgs_,
-            sort_aux_, inc_bkey_, inc_bidx_, inv_, item_, i_slot_, open_ };
-        for (void* p : ps)
-            if (p) cudaFree(p);
-        pool_[0] = pool_[1] = nullptr;
-        pid_[0] = pid_[1] = nullptr;
-        keys_in_ = keys_sorted_ = nullptr;
-        iota_ = vals_sorted_ = g_start_ = nullptr;
-        g_nbr_ = nullptr;
-        b_key_ = nullptr;
-        acc_ = vel_ = nullptr;
-        h_keys_ = nullptr;
-        h_vals_ = nullptr;
-        d_scenes_ = nullptr;
-        grid_mass_ = nullptr;
-        st_ = nullptr;
-        sort_tmp_ = stage_ = nullptr;
+        dfree(pool_[0], pool_[1], pid_[0], pid_[1], keys_in_, keys_sorted_, iota_, vals_sorted_, g_start_, g_nbr_, b_key_, acc_, vel_, h_keys_, h_vals_,
+            d_scenes_, grid_mass_, st_, sort_tmp_, stage_, pay_, scenes_backup_, ck_pool_, ck_pid_, ck_scenes_, cg_, cgs_, sort_aux_, inc_bkey_,
+            inc_bidx_, inv_, item_, i_slot_, open_);
         stage_bytes_ = 0;
-        pay_ = nullptr;
         pay_fields_ = 0;
         pstride_ = 0;
-        cg_ = nullptr;
-        cgs_ = nullptr;
         implicit_ = false;
-        sort_aux_ = nullptr;
-        inc_bkey_ = inc_bidx_ = nullptr;
-        item_ = nullptr;
-        open_ = nullptr;
-        i_slot_ = nullptr;
-        inv_ = nullptr;
         inv_cap_ = 0;
         sort_base_stale_ = true;
-        scenes_backup_ = nullptr;
         scenes_backup_bytes_ = 0;
-        ck_pool_ = ck_pid_ = ck_scenes_ = nullptr;
         ck_cap_ = 0;
         ck_scenes_n_ = 0;
         ck_valid_ = false;
@@ -1921,7 +1855,6 @@ private:
         cap_ = 0;
         scene_cap_ = 0;
         b_cap_ = 0;
-        dev_bytes_ = 0;
         h_scenes_.clear();
     }
 
