@@ -146,7 +146,7 @@ public:
             pid_[0] = grown_pid[0];
             pid_[1] = grown_pid[1];
             cap_ = (uint64_t)cap;
-            pay_fields_ = payload_fields();
+            pay_fields_ = payload_fields(sched_);
             // P2G payload: fields of sorted particles at q + q/8, plus the copy granularity at the end
             pstride_ = (int64_t)((pay_pos((uint64_t)cap) + 64 + 63) & ~(uint64_t)63);
             if (alloc((void**)&keys_in_, 8 * cap) || alloc((void**)&keys_sorted_, 8 * cap) || alloc((void**)&iota_, 4 * cap)
@@ -261,7 +261,6 @@ public:
     // An aborted substep is retried after growing the grid (capacity) or reported with the state left at its start.
     int run_steps(int nsteps, StepReport& r, int& done)
     {
-        if (int rc = ensure_payload()) return rc;
         if (int rc = refresh_drive()) return rc;
         const int target = done + nsteps;
         int grow_rounds = 0;
@@ -783,6 +782,9 @@ public:
         if (sc.fused < 0 || sc.fused > 3 || (!sc.fused && variant_index(sc.chunk, sc.buffers) < 0) || g2p_index(sc.g2p_threads) < 0
             || sc.scatter_ctas_per_sm < 1 || sc.scatter_ctas_per_sm > 8 || sc.g2p_tight < 0 || sc.g2p_tight > 3)
             return arg("schedule: unknown P2G form, (chunk, buffers) pair or G2P width, or CTAs per SM outside [1, 8]");
+        // a form that reads the payload from HBM: its buffer now, so that running out of memory is this call's error and not a
+        // later step's, and leaves the schedule as it was
+        if (int rc = ensure_payload(payload_fields(sc))) return rc;
         sched_ = sc;
         if (sc.fused) {
             sched_.chunk = sc.fused == 3 ? WsShape<T>::CHUNK : FUSED_CH[fused_variant(sc.fused)];
@@ -1292,8 +1294,8 @@ private:
             ZR_CUDA(bin_incremental(n, a));
             if (ev) ZR_CUDA(cudaEventRecord(ev[1], stream_)); // the merge also activates the blocks: both in the first phase
         }
-        if (reads_payload() && pay_fields_ < (size_t)Pay<T>::N) return fail(ZR_ERR_STATE_, "P2G payload not allocated");
-        if (reads_payload()) // these P2G forms read grid slots; the fused one translates its groups' entries
+        if (reads_payload(sched_) && pay_fields_ < (size_t)Pay<T>::N) return fail(ZR_ERR_STATE_, "P2G payload not allocated");
+        if (reads_payload(sched_)) // these P2G forms read grid slots; the fused one translates its groups' entries
             k_nbr<T><<<nsm_ * 4, 256, 0, stream_>>>(a);
         if (ev) ZR_CUDA(cudaEventRecord(ev[2], stream_));
         if (sched_.fused == 3)
@@ -1719,20 +1721,21 @@ private:
         if (!SPLIT_TRIED) return Schedule{ fused_code(1), FUSED_CH[1], 0, occ_fused_[1][models_slot()], G2P_NT[1], 0, 0 };
         return Schedule{ 0, VAR_CHUNK[0], VAR_NBUF[0], occ_scatter_[0], G2P_NT[1], 0, 0 };
     }
-    bool reads_payload() const { return sched_.fused == 0 || sched_.fused == 3; }
+    static bool reads_payload(const Schedule& sc) { return sc.fused == 0 || sc.fused == 3; }
     // the implicit damage solve's scratch, or the payload of a schedule that reads it
-    size_t payload_fields() const { return SPLIT_TRIED || reads_payload() ? Pay<T>::N : DS_NF; }
-    // before a run: the schedule may have been set since the buffer was made
-    int ensure_payload()
+    static size_t payload_fields(const Schedule& sc) { return SPLIT_TRIED || reads_payload(sc) ? Pay<T>::N : DS_NF; }
+    // room for so many payload fields; the buffer is kept where it is large enough
+    int ensure_payload(size_t fields)
     {
-        if (!cap_ || pay_fields_ >= payload_fields()) return 0;
+        if (!cap_ || pay_fields_ >= fields) return 0;
+        T* grown = nullptr;
+        const size_t bytes = sizeof(T) * fields * (size_t)pstride_;
+        if (alloc((void**)&grown, bytes)) return ZR_ERR_CUDA_;
+        ZR_CUDA(cudaMemsetAsync(grown, 0, bytes, stream_));
         drop_graphs();
-        dfree(pay_);
-        pay_fields_ = 0;
-        const size_t bytes = sizeof(T) * payload_fields() * (size_t)pstride_;
-        if (alloc((void**)&pay_, bytes)) return ZR_ERR_CUDA_;
-        ZR_CUDA(cudaMemsetAsync(pay_, 0, bytes, stream_));
-        pay_fields_ = payload_fields();
+        dfree(pay_); // (waits for what is in flight)
+        pay_ = grown;
+        pay_fields_ = fields;
         return 0;
     }
 
