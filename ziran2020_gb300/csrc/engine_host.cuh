@@ -1550,13 +1550,21 @@ private:
     {
         return k_g2p<T, G2P_NT[N], G2P_RES[R & 1], (R >> 1) != 0, (R >> 1) != 0 ? DRIVE_ANY : D>;
     }
+    static constexpr size_t g2p_dyn(int variant) { return (variant >> 1) != 0 ? G2P_HALO : 0; }
+    template <int R, int N, int D>
+    void g2p_setup_one()
+    {
+        const auto k = g2p_kernel<R, N, D>();
+        if (g2p_dyn(R)) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g2p_dyn(R));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][D], k, G2P_NT[N], g2p_dyn(R));
+        occ_g2p_[R][N][D] = std::max(1, occ_g2p_[R][N][D]);
+    }
     template <int R, int N>
     void g2p_setup()
     {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_NONE], g2p_kernel<R, N, DRIVE_NONE>(), G2P_NT[N], 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_BORDEN], g2p_kernel<R, N, DRIVE_BORDEN>(), G2P_NT[N], 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g2p_[R][N][DRIVE_ANY], g2p_kernel<R, N, DRIVE_ANY>(), G2P_NT[N], 0);
-        for (int& o : occ_g2p_[R][N]) o = std::max(1, o);
+        g2p_setup_one<R, N, DRIVE_NONE>();
+        g2p_setup_one<R, N, DRIVE_BORDEN>();
+        g2p_setup_one<R, N, DRIVE_ANY>();
     }
     int drive() const { return !any_damage_ ? DRIVE_NONE : ((models_ & (1 << MODEL_QR_STABLE_NEOHOOKEAN)) ? DRIVE_ANY : DRIVE_BORDEN); }
     template <int R, int N>
@@ -1564,11 +1572,11 @@ private:
     {
         const int d = drive(), ctas = nsm_ * occ_g2p_[R][N][d];
         if (d == DRIVE_NONE)
-            g2p_kernel<R, N, DRIVE_NONE>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
+            g2p_kernel<R, N, DRIVE_NONE>()<<<ctas, G2P_NT[N], g2p_dyn(R), stream_>>>(a);
         else if (d == DRIVE_BORDEN)
-            g2p_kernel<R, N, DRIVE_BORDEN>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
+            g2p_kernel<R, N, DRIVE_BORDEN>()<<<ctas, G2P_NT[N], g2p_dyn(R), stream_>>>(a);
         else
-            g2p_kernel<R, N, DRIVE_ANY>()<<<ctas, G2P_NT[N], 0, stream_>>>(a);
+            g2p_kernel<R, N, DRIVE_ANY>()<<<ctas, G2P_NT[N], g2p_dyn(R), stream_>>>(a);
     }
     template <int R>
     void launch_g2p(const StepArgs<T>& a, int gi)

@@ -2074,6 +2074,7 @@ __global__ void __launch_bounds__(GRID_NT) k_grid(StepArgs<T> a)
 // NT threads per CTA; RESIDENT: threads per SM the register budget is cut for
 // G2P's staged particle state: x, F, m, V0, d, sigma_c (fields G2P_SF) and the pid, per thread and buffer
 enum { GS_X = 0, GS_F = 3, GS_M = 12, GS_V0 = 13, GS_D = 14, GS_SC = 15, G2P_SF = 16 };
+constexpr size_t G2P_HALO = 8 * 1024; // dynamic shared memory of the variants that stage the 8 blocks' velocities
 template <class T, int NT>
 struct G2pStage {
     // double-buffered per-thread slots, field-major so a warp's accesses are consecutive words; off where the
@@ -2202,7 +2203,8 @@ __device__ __forceinline__ void gather(const Quad<T>* tv, const Quad<T>* te, con
 
 // BULK: the 8 neighbouring blocks' velocities reach shared memory by bulk asynchronous copies (one 4-field block of
 // NVEL * nodes values per copy, completing on an mbarrier) and the node tile is built from there; otherwise each
-// thread loads its tile nodes from global memory
+// thread loads its tile nodes from global memory. The copies land in dynamic shared memory (G2P_HALO bytes): beside the tiles and
+// the staged state, FP32 at 256 threads and FP64 at 128 would pass the 48 KB a kernel's static shared memory may have.
 // DRIVE: the damage the batch's scenes can have: none, on the Borden model only, any (the drive of the QR-stable model brings a
 // QR factorisation and a polar decomposition into the kernel)
 enum { DRIVE_NONE = 0, DRIVE_BORDEN = 1, DRIVE_ANY = 2 };
@@ -2213,7 +2215,9 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
     using L = typename LayoutOf<T>::type;
     using GS = G2pStage<T, NT>;
     constexpr int BLK = NVEL * L::nodes; // values of one block's velocity fields (1 KB in both precisions)
-    __shared__ __align__(128) T s_halo[BULK ? 8 * BLK : 1];
+    static_assert(8 * BLK * sizeof(T) == G2P_HALO, "eight blocks");
+    extern __shared__ __align__(128) unsigned char g2p_dyn[];
+    T* s_halo = reinterpret_cast<T*>(g2p_dyn); // (BULK)
     __shared__ __align__(8) uint64_t s_hbar;
     uint32_t hphase = 0;
     // the grid velocities around the group's block as one dense node tile (the block plus 2 nodes on the
@@ -2229,6 +2233,8 @@ __global__ void __launch_bounds__(NT, RESIDENT / NT) k_g2p(StepArgs<T> a)
     __shared__ uint32_t s_pid[GS::NP];
     __shared__ int s_g, s_last, s_nbr[8], s_scene, s_org[3];
     __shared__ uint16_t s_map[TN]; // tile node -> (neighbour block 0-7) << 8 | element in that block
+    static_assert(sizeof(tv) + sizeof(te) + sizeof(s_mat) + sizeof(s_st) + sizeof(s_pid) + sizeof(s_map) + 512 <= 48 * 1024,
+        "static shared memory of a kernel (512 B: the words above and the arrays' alignment)");
     if (aborted_cta(a.st)) return;
     if (BULK && threadIdx.x == 0) {
         mbar_init(&s_hbar, 1);
