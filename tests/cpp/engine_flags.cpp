@@ -1,0 +1,116 @@
+// Scenes that reach (or must not reach) the incremental sort's overflow, run through the engine interface, which reports the
+// substeps' flags. Prints "name value" pairs for the Python test. Each run is compared with one that sorts in full (ZR_SORT=full):
+// the two give the same particle order, so they differ by the order of grid sums alone.
+#include "../../ziran2020_gb300/csrc/engine.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+
+using namespace zr;
+
+constexpr uint32_t SORT_OVERFLOW = 1u << 7; // FLAG_SORT: a bucket of the incremental sort had no room for its movers
+
+struct Rng { // seeded, the same on every machine
+    uint64_t s;
+    double operator()()
+    {
+        s = s * 6364136223846793005ull + 1442695040888963407ull;
+        return (double)(s >> 11) * (1.0 / 9007199254740992.0);
+    }
+};
+
+// nx x ny x nz cells of a stiffness so low that the body moves freely, 8 particles a cell at random places
+static SceneDesc box(int nx, int ny, int nz, int cells, int first, double speed_cells)
+{
+    SceneDesc d;
+    d.dx = 1.0 / cells;
+    d.dt = 1e-4;
+    d.domain_cells = cells + 4;
+    d.materials.push_back({});
+    d.materials[0].E = 1.0;
+    Rng u{ 12345 };
+    for (int i = 0; i < nx; i++)
+        for (int j = 0; j < ny; j++)
+            for (int k = 0; k < nz; k++)
+                for (int q = 0; q < 8; q++) {
+                    d.x.push_back((first + i + u()) * d.dx);
+                    d.x.push_back((first + j + u()) * d.dx);
+                    d.x.push_back((first + k + u()) * d.dx);
+                    for (int c = 0; c < 3; c++) d.v.push_back(speed_cells * d.dx / d.dt);
+                }
+    d.n = (int64_t)d.x.size() / 3;
+    d.m.assign(d.n, 1000 * d.dx * d.dx * d.dx / 8);
+    d.V0.assign(d.n, d.dx * d.dx * d.dx / 8);
+    return d;
+}
+
+static void must(int rc, EngineBase& e)
+{
+    if (!rc) return;
+    std::fprintf(stderr, "error %d: %s\n", rc, e.last_error().c_str());
+    std::exit(1);
+}
+
+static std::unique_ptr<EngineBase> engine(int precision, const SceneDesc& d, bool full_sort)
+{
+    if (full_sort) setenv("ZR_SORT", "full", 1); // read when the engine is made
+    auto e = precision == 8 ? make_engine_f64() : make_engine_f32();
+    unsetenv("ZR_SORT");
+    e->set_autotune(0);
+    must(e->load({ &d }), *e);
+    return e;
+}
+
+// largest difference of two states: positions and F as they are, velocities in units of the speed, C of the speed over dx
+static double difference(const std::vector<double>& a, const std::vector<double>& b, const SceneDesc& d)
+{
+    double speed = 0, m = 0;
+    for (double v : d.v) speed = std::max(speed, std::fabs(v));
+    for (size_t i = 0; i < a.size(); i++) {
+        const int f = (int)(i % 25);
+        const double unit = f < 3 ? 1.0 : (f < 6 ? speed : (f < 15 ? speed / d.dx : 1.0));
+        m = std::isfinite(a[i]) && std::isfinite(b[i]) ? std::max(m, std::fabs(a[i] - b[i]) / unit) : 1e30;
+    }
+    return m;
+}
+
+// A written state in which a few percent of the particles moved, all into one place: more than a bucket holds, in all far
+// fewer than a quarter.
+static void concentrated(SceneDesc& d, std::vector<double>& state)
+{
+    const int64_t part = 3000;
+    for (int64_t p = 0; p < part; p++) // the first layers, beside the box's far end
+        for (int c = 0; c < 3; c++) state[25 * p + c] = d.x[3 * p + c] + (c == 0 ? 20 * d.dx : 0.0);
+}
+
+int main(int argc, char** argv)
+{
+    const std::string mode = argc > 1 ? argv[1] : "";
+    const int precision = argc > 2 ? std::atoi(argv[2]) : 8;
+    if (mode == "written") {
+        SceneDesc d = box(16, 16, 16, 64, 8, 0.005);
+        std::vector<double> out[2];
+        uint32_t flags = 0;
+        for (int full = 0; full < 2; full++) {
+            auto e = engine(precision, d, full != 0);
+            StepReport r;
+            must(e->step(4, &r), *e);
+            out[full].resize(25 * d.n);
+            must(e->get_state(0, out[full].data(), 0), *e);
+            concentrated(d, out[full]);
+            must(e->set_state(0, out[full].data(), 0), *e);
+            StepReport r2;
+            must(e->step(3, &r2), *e);
+            must(e->get_state(0, out[full].data(), 0), *e);
+            if (!full) flags = r2.flags;
+        }
+        std::printf("particles %lld overflow %d difference %.3e\n", (long long)d.n, (flags & SORT_OVERFLOW) != 0, difference(out[0], out[1], d));
+        return 0;
+    }
+    return 2;
+}

@@ -1,0 +1,33 @@
+"""GPU: the incremental sort where a tile's bucket has no room for its movers, through the engine interface (tests/cpp/engine_flags.cpp),
+whose report says whether a substep overflowed and was repeated."""
+import os
+import subprocess
+
+import pytest
+
+import ziran2020_gb300 as zr
+
+pytestmark = pytest.mark.gpu
+SRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp", "engine_flags.cpp")
+TOL = {8: 1e-12, 4: 1e-5}  # a few substeps of sums of ~100 terms in another order, in units of each field
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    lib = zr.library_path()
+    exe = str(tmp_path_factory.mktemp("flags") / "engine_flags")
+    subprocess.check_call(["g++", "-std=c++17", "-O2", SRC, "-o", exe, lib, "-Wl,-rpath," + os.path.dirname(lib)])
+
+    def call(mode, precision):
+        words = subprocess.check_output([exe, mode, str(precision)], text=True, timeout=300).split()
+        return {k: float(v) for k, v in zip(words[::2], words[1::2])}
+
+    return call
+
+
+@pytest.mark.parametrize("precision", [8, 4])
+def test_a_written_state_that_would_overflow_one_bucket_is_sorted_in_full(run, precision):
+    """a twelfth of the particles moved into one place: nothing aborts, the next substep sorts in full"""
+    r = run("written", precision)
+    assert r["particles"] == 32768 and r["overflow"] == 0
+    assert r["difference"] < TOL[precision]

@@ -136,6 +136,7 @@ struct DevStatus {
     uint32_t cg_loops; // iterations of the damage solve's loop in this substep (any scene)
     uint32_t g2p_done; // CTAs of the substep's G2P that have finished
     uint32_t max_movers; // particles that left the key their slot was sorted by (counted when a state is written)
+    uint32_t full_bucket; // a sort bucket would not hold its movers (counted when a state is written)
 };
 
 constexpr int MAX_OBJECTS = 8;

@@ -919,13 +919,10 @@ private:
     uint32_t* tile_first() const { return reinterpret_cast<uint32_t*>(sort_aux_) + sort_zero_bytes((int64_t)cap_) / 4 + (cap_ + 31) / 32; }
     bool inc_sort_usable() const { return inc_sort_on_ && !kl_.wide && kl_.total() <= 31; }
 
-    // The sorted keys and storage indices of keys_in_ from the previous substep's sorted keys (keys_sorted_), the groups
-    // and their blocks, by the hand-written kernels of the incremental sort (stayers in place, movers bucketed by stayer
-    // tile and merged).
-    cudaError_t bin_incremental(int64_t n, const StepArgs<T>& a)
+    SortBufs sort_bufs()
     {
         SortBufs sb;
-        const int64_t tiles = sort_tiles(n, sort_per()), tcap = max_tiles((int64_t)cap_);
+        const int64_t tcap = max_tiles((int64_t)cap_);
         sb.b_cnt = reinterpret_cast<uint32_t*>(sort_aux_);
         sb.b_max = sb.b_cnt + tcap;
         sb.stay_bits = sb.b_max + tcap;
@@ -934,8 +931,18 @@ private:
         sb.t_last = sb.t_stay + tcap;
         sb.b_key = inc_bkey_;
         sb.b_idx = inc_bidx_;
-        sb.n = n;
-        sb.tiles = (int)tiles;
+        sb.n = (int64_t)N_;
+        sb.tiles = (int)sort_tiles((int64_t)N_, sort_per());
+        return sb;
+    }
+
+    // The sorted keys and storage indices of keys_in_ from the previous substep's sorted keys (keys_sorted_), the groups
+    // and their blocks, by the hand-written kernels of the incremental sort (stayers in place, movers bucketed by stayer
+    // tile and merged).
+    cudaError_t bin_incremental(const StepArgs<T>& a)
+    {
+        const SortBufs sb = sort_bufs();
+        const int tiles = sb.tiles;
         const uint32_t* nk = (const uint32_t*)keys_in_;
         if (sort_per() == 2) {
             k_sort_tiles<2><<<(unsigned)tiles, SORT_NT, 0, stream_>>>(nk, (const uint32_t*)keys_sorted_, sb, st_);
@@ -1198,17 +1205,33 @@ private:
     {
         sorted_storage_ = false; // new positions: the storage order may no longer follow the cells
         // The sort base (keys_sorted_) stays a sorted array of the same keys' layout, which is all the incremental sort
-        // needs to be correct: particles whose key matches it at their slot form a sorted subsequence. When more than a
-        // quarter of the particles left their slot's key, the next substep sorts in full: a tile's bucket takes half as many
-        // movers as the tile has particles, and an overflow found out in that substep aborts it and the launches already
-        // queued behind it run empty.
+        // needs to be correct: particles whose key matches it at their slot form a sorted subsequence. Where a tile's bucket
+        // would not hold its movers, the next substep sorts in full: found out in that substep, the overflow aborts it and the
+        // launches already queued behind it run empty. So it does where more than a quarter of all particles left their slot's
+        // key (a bucket has room for half a tile's worth, or a whole one in small scenes): nothing is counted by bucket then,
+        // nor where there are fewer movers than a bucket has slots.
         const bool based = inc_sort_usable() && !sort_base_stale_;
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, based ? (const uint32_t*)keys_sorted_ : nullptr);
         ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
-        if (based && (uint64_t)hst_->max_movers * 4 > (uint64_t)N_) sort_base_stale_ = true;
-        if (hst_->flags & FLAG_OUT_OF_DOMAIN) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
+        const bool outside = (hst_->flags & FLAG_OUT_OF_DOMAIN) != 0;
+        const int64_t movers = based ? (int64_t)hst_->max_movers : 0;
+        if (movers * 4 > (int64_t)N_)
+            sort_base_stale_ = true;
+        else if (movers > (sort_per() == 2 ? SortTile<2>::MAXM : SortTile<SORT_PER>::MAXM)) {
+            const uint32_t *nk = (const uint32_t*)keys_in_, *ok = (const uint32_t*)keys_sorted_;
+            if (sort_per() == 2)
+                k_sort_probe<2><<<nsm_ * 4, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
+            else
+                k_sort_probe<SORT_PER><<<nsm_ * 4, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
+            ZR_CUDA(cudaGetLastError());
+            ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_));
+            ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
+            ZR_CUDA(cudaStreamSynchronize(stream_));
+            if (hst_->full_bucket) sort_base_stale_ = true;
+        }
+        if (outside) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
         return 0;
     }
 
@@ -1291,7 +1314,7 @@ private:
             k_activate<T><<<nsm_ * 4, 256, 0, stream_>>>(a);
         }
         else {
-            ZR_CUDA(bin_incremental(n, a));
+            ZR_CUDA(bin_incremental(a));
             if (ev) ZR_CUDA(cudaEventRecord(ev[1], stream_)); // the merge also activates the blocks: both in the first phase
         }
         if (reads_payload(sched_) && pay_fields_ < (size_t)Pay<T>::N) return fail(ZR_ERR_STATE_, "P2G payload not allocated");

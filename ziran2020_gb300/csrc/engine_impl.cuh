@@ -281,6 +281,30 @@ struct SortBufs {
 };
 constexpr int SORT_FIRST = 4096; // tiles whose first keys a CTA copies to shared memory for its searches
 
+// bucket of mover key k: the last tile whose first old key is not above it
+__device__ __forceinline__ uint32_t bucket_of(const uint32_t* B, int tiles, uint32_t k)
+{
+    int lo = 0, hi = tiles; // first q with B[q] > k
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (B[mid] <= k) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo > 0 ? (uint32_t)(lo - 1) : 0u;
+}
+
+// After a state write: would a bucket of the next substep's sort hold more movers than its slots? Its movers counted by bucket
+// (b_cnt, which the host clears again) with the keys, the base and the tiles that k_sort_tiles will see.
+template <int PER>
+__global__ void __launch_bounds__(SORT_NT) k_sort_probe(const uint32_t* knew, const uint32_t* kold, SortBufs sb, DevStatus* st)
+{
+    for (int64_t i = blockIdx.x * (int64_t)SORT_NT + threadIdx.x; i < sb.n; i += (int64_t)gridDim.x * SORT_NT) {
+        const uint32_t k = knew[i];
+        if (k == kold[i]) continue;
+        if (atomicAdd(&sb.b_cnt[bucket_of(sb.t_first, sb.tiles, k)], 1u) == (uint32_t)SortTile<PER>::MAXM) st->full_bucket = 1;
+    }
+}
+
 template <int PER>
 __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, const uint32_t* kold, SortBufs sb, const DevStatus* st)
 {
@@ -332,13 +356,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_tiles(const uint32_t* knew, co
     for (int r = 0; r < PER; r++) {
         if (!((moves >> r) & 1u)) continue;
         const uint32_t k = kn[r];
-        int lo = 0, hi = T; // first q with B[q] > k
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (B[mid] <= k) lo = mid + 1;
-            else hi = mid;
-        }
-        const uint32_t b = lo > 0 ? (uint32_t)(lo - 1) : 0u;
+        const uint32_t b = bucket_of(B, T, k);
         const uint32_t t = atomicAdd(&sb.b_cnt[b], 1u);
         atomicMax(&sb.b_max[b], k);
         if (t < (uint32_t)MAXM) { // a fuller bucket makes the merge raise FLAG_SORT
