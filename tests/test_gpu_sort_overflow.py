@@ -31,3 +31,14 @@ def test_a_written_state_that_would_overflow_one_bucket_is_sorted_in_full(run, p
     r = run("written", precision)
     assert r["particles"] == 32768 and r["overflow"] == 0
     assert r["difference"] < TOL[precision]
+
+
+@pytest.mark.parametrize("precision", [8, 4])
+def test_a_body_that_overflows_in_every_substep_launches_few_empty_ones(run, precision):
+    """681,472 particles (tiles of 2,048 storage indices) that move 0.25 cells along each axis per substep: every incremental sort
+    overflows. The substeps launched stay within four times those asked for (they were n (n + 1) / 2), and the run equals the
+    one that sorts in full."""
+    r = run("fast", precision)
+    assert r["particles"] == 681472 and r["overflow"] == 1 and r["done"] == 40
+    assert r["launched"] <= 4 * 40
+    assert r["difference"] < TOL[precision]

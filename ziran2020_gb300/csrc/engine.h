@@ -58,7 +58,26 @@ struct StepReport {
     double device_ms = 0; // device time of the substeps, CUDA events on the engine's stream
     uint32_t flags = 0;
     int32_t steps_done = 0;
+    int32_t launched = 0; // substeps enqueued, those that ran empty behind an aborted one among them
     uint32_t n_groups = 0, n_blocks = 0, fallback = 0;
+};
+
+// How a run goes on after a substep that overflowed the incremental sort (it is repeated with a full sort). The substeps queued
+// behind it ran empty, so what is launched next is bounded: as many substeps as `full` sort in full, twice as many each time the
+// first incremental one behind them overflows again, and no more than `limit` go out at once, which doubles while all goes well.
+// So a run of n substeps launches O(n), whichever of them overflow.
+struct SortBackoff {
+    int full = 0, limit = 0x40000000;
+    void overflowed(int done_before) // substeps of the launch that were finished
+    {
+        full = done_before <= full && full ? 2 * full : 1;
+        limit = 2 * full > 8 ? 2 * full : 8;
+    }
+    void finished()
+    {
+        full = 0;
+        if (limit < 0x40000000) limit *= 2;
+    }
 };
 
 // Launch schedule of the substep (what the autotuner picks). None of these changes the arithmetic beyond

@@ -264,16 +264,19 @@ public:
         if (int rc = refresh_drive()) return rc;
         const int target = done + nsteps;
         int grow_rounds = 0;
+        SortBackoff backoff;
         while (done < target) {
             ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
             const int cur0 = cur_;
-            int todo = target - done;
+            const int todo = std::min(target - done, backoff.limit);
+            const int full = std::min(todo, std::max(backoff.full, sort_base_stale_ ? 1 : 0));
             if (!timing_ && graphs_on_) {
-                int rcg = prepare_graphs(todo - (sort_base_stale_ ? 1 : 0));
+                int rcg = prepare_graphs(todo - full);
                 if (rcg) return rcg;
             }
             ZR_CUDA(cudaEventRecord(t0_, stream_));
-            int rc = launch_steps(todo);
+            int rc = launch_steps(todo, full);
+            r.launched += todo;
             if (rc) return rc;
             ZR_CUDA(cudaEventRecord(t1_, stream_));
             ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
@@ -291,7 +294,8 @@ public:
                 done += todo;
                 sorted_storage_ = true;
                 sort_base_stale_ = false;
-                break;
+                backoff.finished();
+                continue;
             }
             sort_base_stale_ = true; // the aborted substep's sort overwrote the base
             const int k = hst_->abort_step;
@@ -307,6 +311,7 @@ public:
             if ((f & FLAG_SORT) && !(f & (FLAG_CFL | FLAG_NONFINITE | FLAG_OUT_OF_DOMAIN | FLAG_TIMEOUT | FLAG_CHECK | FLAG_CAPACITY))) {
                 // a bucket beyond the merge's shared memory: the substep is repeated with a full sort (it cannot raise
                 // FLAG_SORT, so every retry makes progress)
+                backoff.overflowed(k);
                 continue;
             }
             if ((f & FLAG_CAPACITY) && !(f & (FLAG_CFL | FLAG_NONFINITE | FLAG_OUT_OF_DOMAIN | FLAG_TIMEOUT | FLAG_CHECK)) && grow_rounds < 6) {
@@ -1498,21 +1503,18 @@ private:
         }
     }
 
-    // Substeps from buffer cur_. The first one sorts in full when the sort base is stale; the others (and the
-    // captured graphs) sort incrementally.
-    int launch_steps(int nsteps)
+    // Substeps from buffer cur_. The first `full` sort in full (at least one where the sort base is stale); the others (and
+    // the captured graphs) sort incrementally.
+    int launch_steps(int nsteps, int full)
     {
         if (timing_ && (int)ev_.size() < 6 * nsteps) {
             size_t old = ev_.size();
             ev_.resize(6 * (size_t)nsteps);
             for (size_t i = old; i < ev_.size(); i++) ZR_CUDA(cudaEventCreate(&ev_[i]));
         }
-        int s0 = 0;
-        if (nsteps > 0 && sort_base_stale_) {
-            int rc = enqueue_step(cur_ & 1, timing_ ? &ev_[0] : nullptr, true);
-            if (rc) return rc;
-            s0 = 1;
-        }
+        const int s0 = full;
+        for (int s = 0; s < full; s++)
+            if (int rc = enqueue_step((cur_ + s) & 1, timing_ ? &ev_[6 * (size_t)s] : nullptr, true)) return rc;
         if (timing_ || !graphs_on_) {
             for (int s = s0; s < nsteps; s++) {
                 int rc = enqueue_step((cur_ + s) & 1, timing_ ? &ev_[6 * (size_t)s] : nullptr);
