@@ -1298,8 +1298,11 @@ double scene_bytes(int precision, int64_t n)
     // (27 fields at 9/8 density: room for FP32's 24; FP64 keeps 4 unless a schedule asks for a split P2G form) and the
     // incremental sort's lists (movers' keys and indices by bucket; 24 B a particle leaves room for its per-tile words)
     const double per_particle = 2 * (30 * s + 4) + 8 + 8 + 4 + 4 + 4 + 27 * s * 9 / 8 + 6 * 4;
+    // per block slot: the node fields; neighbour lists (groups', items'), items and the block key; 8 hash entries at most
+    // (the hash is a power of two of at least 4 per slot) of a key, a value and an open range
+    const double per_slot = 10 * nodes * s + (32 + 32 + 16 + 8) + 8 * (8 + 4 + 8);
     const double groups = (double)n / (nodes * 4) + 64;
-    return n * per_particle + 8 * groups * (10 * nodes * s + 64);
+    return n * per_particle + 8 * groups * per_slot;
 }
 } // namespace
 
