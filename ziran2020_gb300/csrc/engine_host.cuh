@@ -224,7 +224,10 @@ public:
         ZR_CUDA(cudaStreamSynchronize(stream_));
         if (hs.flags & FLAG_OUT_OF_DOMAIN) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
-        const uint32_t need = std::max<uint32_t>(4096, 8 * hs.n_groups + 1024);
+        // the block slots also number the items: one per group and one per item_size particles at most, which is more than eight
+        // per group where cells are crowded (a first substep that ran out of them would abort and be repeated)
+        const uint64_t items = (uint64_t)hs.n_groups + N_ / item_size();
+        const uint32_t need = (uint32_t)std::max<uint64_t>({ 4096, 8 * (uint64_t)hs.n_groups + 1024, items + items / 8 });
         if (need > b_cap_) {
             int rc = alloc_grid(std::max(need, b_cap_ * 2));
             if (rc) return rc;
