@@ -1294,10 +1294,11 @@ namespace {
 double scene_bytes(int precision, int64_t n)
 {
     const double s = precision == ZR_F64 ? 8 : 4, nodes = precision == ZR_F64 ? 32 : 64;
-    // two pool copies (30 fields and the id), keys (in, sorted), sort values, iota, group starts, the P2G payload
-    // (27 fields at 9/8 density: room for FP32's 24; FP64 keeps 4 unless a schedule asks for a split P2G form) and the
+    // two pool copies (30 fields and the id), keys (in, sorted), sort values, iota, group starts, the P2G payload at 9/8
+    // density (FP32 27 fields, room for its 24; FP64 the 41 of the split form, which the autotuner may choose) and the
     // incremental sort's lists (movers' keys and indices by bucket; 24 B a particle leaves room for its per-tile words)
-    const double per_particle = 2 * (30 * s + 4) + 8 + 8 + 4 + 4 + 4 + 27 * s * 9 / 8 + 6 * 4;
+    const double pay = precision == ZR_F64 ? 41 : 27;
+    const double per_particle = 2 * (30 * s + 4) + 8 + 8 + 4 + 4 + 4 + pay * s * 9 / 8 + 6 * 4;
     // per block slot: the node fields; neighbour lists (groups', items'), items and the block key; 8 hash entries at most
     // (the hash is a power of two of at least 4 per slot) of a key, a value and an open range
     const double per_slot = 10 * nodes * s + (32 + 32 + 16 + 8) + 8 * (8 + 4 + 8);

@@ -226,6 +226,7 @@ public:
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         // the block slots also number the items: one per group and one per item_size particles at most, which is more than eight
         // per group where cells are crowded (a first substep that ran out of them would abort and be repeated)
+        load_groups_ = hs.n_groups;
         const uint64_t items = (uint64_t)hs.n_groups + N_ / item_size();
         const uint32_t need = (uint32_t)std::max<uint64_t>({ 4096, 8 * (uint64_t)hs.n_groups + 1024, items + items / 8 });
         if (need > b_cap_) {
@@ -249,7 +250,7 @@ public:
         int done = 0;
         StepReport r;
         int rc = 0;
-        if (nsteps > 0 && !tuned_ && !fixed_schedule_ && !autotune_cached()) {
+        if (nsteps > 0 && !tuned_ && !fixed_schedule_ && !autotune_cached(rc)) {
             // the trials must see the particles in sorted storage order, which one substep of G2P produces
             if (!sorted_storage_) rc = run_steps(1, r, done);
             if (!rc && done < nsteps) rc = autotune_trials();
@@ -811,7 +812,7 @@ private:
     std::string err_;
     std::vector<SceneParams<T>> h_scenes_;
     SceneParams<T>* d_scenes_ = nullptr;
-    uint32_t N_ = 0;
+    uint32_t N_ = 0, load_groups_ = 0; // particles; occupied blocks when the batch was formed
     uint64_t cap_ = 0; // particle capacity of the buffers (the pool's field stride)
     size_t scene_cap_ = 0;
     KeyLayout kl_{};
@@ -1691,7 +1692,7 @@ private:
     }
     uint64_t tune_key() const
     {
-        return (uint64_t)sizeof(T) | ((uint64_t)models_ << 4) | ((uint64_t)any_damage_ << 6) | ((uint64_t)bitlen(N_) << 8)
+        return (uint64_t)sizeof(T) | ((uint64_t)(!SPLIT_TRIED && sparse()) << 1) | ((uint64_t)models_ << 4) | ((uint64_t)any_damage_ << 6) | ((uint64_t)bitlen(N_) << 8)
             | ((uint64_t)bitlen((uint64_t)n_scenes()) << 16) | ((uint64_t)nsm_ << 24);
     }
 
@@ -1727,31 +1728,31 @@ private:
     }
 
     // A schedule without measuring: the fixed default (mode 0) or a cached choice (mode 1). False when trials are needed.
-    bool autotune_cached()
+    bool autotune_cached(int& rc)
     {
-        if (autotune_mode_ == 0) {
-            sched_ = default_schedule();
-            tuned_ = true;
-            drop_graphs();
-            return true;
-        }
+        Schedule sc = default_schedule();
         if (autotune_mode_ == 1) {
             std::lock_guard<std::mutex> lk(tune_mutex());
             auto it = tune_cache().find(tune_key());
-            if (it != tune_cache().end()) {
-                sched_ = it->second;
-                tuned_ = true;
-                drop_graphs();
-                return true;
-            }
+            if (it == tune_cache().end()) return false;
+            sc = it->second;
         }
-        return false;
+        else if (autotune_mode_ != 0)
+            return false;
+        tuned_ = true;
+        rc = adopt(sc);
+        return true;
     }
 
-    // In FP64 only an explicit schedule takes a split P2G form: its payload in HBM is 41 fields, 369 B a particle on top of the
-    // ~530 of everything else, for a kernel the FP64 pipe bounds either way (the tuned 426k slab's pass the same without the split
-    // candidates: 1.002x).
+    // The forms that read a payload from HBM. FP32 always has the buffer and tries them all. FP64's payload is 41 fields, 369 B a
+    // particle on top of the ~530 of everything else, and the FP64 pipe bounds the kernel either way: it has the buffer only for a
+    // schedule that reads it, and tries the split form with one staging buffer in sparse scenes. P2G split / fused: 1 particle per
+    // cell 269 / 338 us (box, 64,000 particles), 764 / 843 (slab, 200,000), 1588 / 1773 (thinned 1/256 slab, 426,421); thinned to 2
+    // 0.97-1.11 of the fused form, to 4 0.94-1.05, to 6 0.96-1.07; 8 per cell 789 / 745 (425,984), 27 1434 / 647. The other split and the
+    // warp-specialised forms were never ahead of the better of these two (11 scenes of 4,096 to 1,068,903 particles).
     static constexpr bool SPLIT_TRIED = sizeof(T) == 4;
+    bool split_tried_here() const { return SPLIT_TRIED || sparse(); }
+    bool sparse() const { return (uint64_t)N_ < 5 * (uint64_t)L::nodes * load_groups_; } // fewer than 5 particles per cell of the occupied blocks
     Schedule default_schedule() const
     {
         if (!SPLIT_TRIED) return Schedule{ fused_code(1), FUSED_CH[1], 0, occ_fused_[1][models_slot()], G2P_NT[1], 0, 0 };
@@ -1775,6 +1776,24 @@ private:
         return 0;
     }
 
+    // gives back a payload buffer that only trials needed
+    int trim_payload()
+    {
+        const size_t fields = payload_fields(sched_);
+        if (pay_fields_ <= fields) return 0;
+        drop_graphs();
+        dfree(pay_);
+        pay_fields_ = 0;
+        return ensure_payload(fields);
+    }
+    // a measured schedule; the default one where there is no room for its payload
+    int adopt(const Schedule& sc)
+    {
+        sched_ = ensure_payload(payload_fields(sc)) ? default_schedule() : sc;
+        drop_graphs();
+        return trim_payload();
+    }
+
     int autotune_trials()
     {
         tuned_ = true;
@@ -1788,7 +1807,8 @@ private:
         ZR_CUDA(cudaMemcpyAsync(scenes_backup_, d_scenes_, sb, cudaMemcpyDeviceToDevice, stream_));
         // P2G candidates with the default G2P, then G2P candidates with the chosen P2G
         std::vector<Schedule> p2g_c;
-        for (int vi = 0; SPLIT_TRIED && vi < 3; vi++)
+        const int splits = SPLIT_TRIED ? 3 : (split_tried_here() && !ensure_payload(Pay<T>::N) ? 1 : 0); // (no room: not tried)
+        for (int vi = 0; vi < splits; vi++)
             for (int c = occ_scatter_[vi]; c >= std::max(1, occ_scatter_[vi] - 1); c--)
                 p2g_c.push_back(Schedule{ 0, VAR_CHUNK[vi], VAR_NBUF[vi], c, G2P_NT[1], 0, 1 });
         for (int fv = 0; fv < 2; fv++) {
@@ -1809,11 +1829,7 @@ private:
                 bool ab = false;
                 int rc = trial(sc, p, g, ab);
                 if (rc) return rc;
-                if (ab) { // the state cannot step (CFL, out of domain, capacity): keep defaults, the step reports it
-                    sched_ = default_schedule();
-                    drop_graphs();
-                    return 0;
-                }
+                if (ab) return adopt(default_schedule()); // the state cannot step (CFL, out of domain, capacity): the step reports it
                 mp = std::min(mp, p);
             }
             if (mp < best_p2g) {
@@ -1835,11 +1851,7 @@ private:
                 bool ab = false;
                 int rc = trial(sc, p, g, ab);
                 if (rc) return rc;
-                if (ab) {
-                    sched_ = default_schedule();
-                    drop_graphs();
-                    return 0;
-                }
+                if (ab) return adopt(default_schedule());
                 mg = std::min(mg, g);
             }
             if (mg < best_g2p) {
@@ -1849,8 +1861,7 @@ private:
             }
         }
         best.tuned = 1;
-        sched_ = best;
-        drop_graphs();
+        if (int rc = adopt(best)) return rc;
         std::lock_guard<std::mutex> lk(tune_mutex());
         tune_cache()[tune_key()] = best;
         return 0;
