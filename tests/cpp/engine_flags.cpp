@@ -127,5 +127,58 @@ int main(int argc, char** argv)
             (r[0].flags & SORT_OVERFLOW) != 0, r[0].launched, r[0].steps_done, difference(out[0], out[1], d), r[0].device_ms, r[1].device_ms);
         return 0;
     }
+    if (mode == "tiles") { // the first n particles of a box that moves 0.04 cells along each axis per substep: no sort overflows
+        const int64_t n = std::atoll(argv[3]);
+        int side = 1;
+        while ((int64_t)side * side * side * 8 < n) side++;
+        SceneDesc d = box(side, side, side, 256, 8, 0.04);
+        d.n = n;
+        d.x.resize(3 * n);
+        d.v.resize(3 * n);
+        d.m.resize(n);
+        d.V0.resize(n);
+        std::vector<double> out[2];
+        StepReport r[2];
+        for (int full = 0; full < 2; full++) {
+            auto e = engine(precision, d, full != 0);
+            must(e->step(5, &r[full]), *e);
+            out[full].resize(25 * d.n);
+            must(e->get_state(0, out[full].data(), 0), *e);
+        }
+        std::printf("particles %lld overflow %d difference %.3e groups %u full_groups %u blocks %u full_blocks %u\n", (long long)d.n,
+            (r[0].flags & SORT_OVERFLOW) != 0, difference(out[0], out[1], d), r[0].n_groups, r[1].n_groups, r[0].n_blocks, r[1].n_blocks);
+        return 0;
+    }
+    if (mode == "stream") { // pipelined one-substep jobs, some of whose states would overflow a bucket of the job before
+        SceneDesc d = box(16, 16, 16, 64, 8, 0.005);
+        auto e = engine(precision, d, false);
+        std::vector<double> plain(25 * d.n);
+        must(e->get_state(0, plain.data(), 0), *e);
+        std::vector<double> moved = plain;
+        concentrated(d, moved);
+        const std::vector<double>* jobs[] = { &plain, &plain, &moved, &plain, &moved, &moved, &plain };
+        constexpr int J = 7;
+        std::vector<double> out[J], want[J];
+        const void* in[J];
+        void* to[J];
+        for (int j = 0; j < J; j++) {
+            out[j].resize(25 * d.n);
+            in[j] = jobs[j]->data();
+            to[j] = out[j].data();
+        }
+        must(e->stream_steps(0, J, in, to, 0), *e);
+        auto f = engine(precision, d, true);
+        double m = 0;
+        for (int j = 0; j < J; j++) {
+            want[j].resize(25 * d.n);
+            StepReport r;
+            must(f->set_state(0, in[j], 0), *f);
+            must(f->step(1, &r), *f);
+            must(f->get_state(0, want[j].data(), 0), *f);
+            m = std::max(m, difference(out[j], want[j], d));
+        }
+        std::printf("particles %lld reruns %lld difference %.3e\n", (long long)d.n, (long long)e->stream_reruns(), m);
+        return 0;
+    }
     return 2;
 }

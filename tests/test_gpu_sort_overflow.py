@@ -18,8 +18,8 @@ def run(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("flags") / "engine_flags")
     subprocess.check_call(["g++", "-std=c++17", "-O2", SRC, "-o", exe, lib, "-Wl,-rpath," + os.path.dirname(lib)])
 
-    def call(mode, precision):
-        words = subprocess.check_output([exe, mode, str(precision)], text=True, timeout=300).split()
+    def call(mode, precision, *more):
+        words = subprocess.check_output([exe, mode, str(precision)] + [str(m) for m in more], text=True, timeout=300).split()
         return {k: float(v) for k, v in zip(words[::2], words[1::2])}
 
     return call
@@ -42,3 +42,30 @@ def test_a_body_that_overflows_in_every_substep_launches_few_empty_ones(run, pre
     assert r["particles"] == 681472 and r["overflow"] == 1 and r["done"] == 40
     assert r["launched"] <= 4 * 40
     assert r["difference"] < TOL[precision]
+
+
+@pytest.mark.parametrize("precision", [8, 4])
+def test_pipelined_jobs_run_again_after_an_overflow(run, precision):
+    """the pipeline does not count movers; the job whose sort overflows and those behind it run the safe way"""
+    r = run("stream", precision)
+    assert 0 < r["reruns"] <= 6
+    assert r["difference"] < TOL[precision]
+
+
+@pytest.mark.parametrize("n", [599_999, 600_000, 600_001, 614_399, 614_400, 614_401])
+@pytest.mark.parametrize("precision", [8, 4])
+def test_large_tiles_at_their_edges(run, precision, n):
+    """512-index tiles up to 600,000 particles, 2,048 above (614,400 = 300 whole ones): incremental against full sort"""
+    r = run("tiles", precision, n)
+    assert r["particles"] == n and r["overflow"] == 0
+    assert (r["groups"], r["blocks"]) == (r["full_groups"], r["full_blocks"])
+    assert r["difference"] < TOL[precision]
+
+
+@pytest.mark.parametrize("n", [2048 * 4096, 2048 * 4096 + 1])
+def test_more_tiles_than_a_block_copies(run, n):
+    """beyond 4,096 tiles the first keys are searched in global memory"""
+    r = run("tiles", 4, n)
+    assert r["particles"] == n and r["overflow"] == 0
+    assert (r["groups"], r["blocks"]) == (r["full_groups"], r["full_blocks"])
+    assert r["difference"] < TOL[4]
