@@ -1218,29 +1218,29 @@ private:
         // would not hold its movers, the next substep sorts in full: found out in that substep, the overflow aborts it and the
         // launches already queued behind it run empty. So it does where more than a quarter of all particles left their slot's
         // key (a bucket has room for half a tile's worth, or a whole one in small scenes): nothing is counted by bucket then,
-        // nor where there are fewer movers than a bucket has slots.
+        // nor where there are fewer movers than a bucket has slots (sort_counted).
         const bool based = inc_sort_usable() && !sort_base_stale_;
         ZR_CUDA(cudaMemsetAsync(st_, 0, sizeof(DevStatus), stream_));
         k_keys<T><<<nsm_ * 4, 256, 0, stream_>>>(pool(cur_), d_scenes_, n_scenes(), keys_in_, N_, kl_, st_, based ? (const uint32_t*)keys_sorted_ : nullptr);
+        const bool small = sort_per() == 2;
+        if (based) {
+            const uint32_t *nk = (const uint32_t*)keys_in_, *ok = (const uint32_t*)keys_sorted_;
+            const int grid = (int)std::min<int64_t>(nsm_ * 4, ((int64_t)N_ + SORT_NT - 1) / SORT_NT);
+            if (small)
+                k_sort_probe<2><<<grid, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
+            else
+                k_sort_probe<SORT_PER><<<grid, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
+            ZR_CUDA(cudaGetLastError());
+        }
         ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
-        const bool outside = (hst_->flags & FLAG_OUT_OF_DOMAIN) != 0;
-        const int64_t movers = based ? (int64_t)hst_->max_movers : 0;
-        if (movers * 4 > (int64_t)N_)
-            sort_base_stale_ = true;
-        else if (movers > (sort_per() == 2 ? SortTile<2>::MAXM : SortTile<SORT_PER>::MAXM)) {
-            const uint32_t *nk = (const uint32_t*)keys_in_, *ok = (const uint32_t*)keys_sorted_;
-            if (sort_per() == 2)
-                k_sort_probe<2><<<nsm_ * 4, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
-            else
-                k_sort_probe<SORT_PER><<<nsm_ * 4, SORT_NT, 0, stream_>>>(nk, ok, sort_bufs(), st_);
-            ZR_CUDA(cudaGetLastError());
-            ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_));
-            ZR_CUDA(cudaMemcpyAsync(hst_, st_, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
-            ZR_CUDA(cudaStreamSynchronize(stream_));
-            if (hst_->full_bucket) sort_base_stale_ = true;
+        if (based) {
+            const int64_t movers = (int64_t)hst_->max_movers;
+            if (movers * 4 > (int64_t)N_ || hst_->full_bucket) sort_base_stale_ = true;
+            if (small ? sort_counted<2>(movers, N_) : sort_counted<SORT_PER>(movers, N_))
+                ZR_CUDA(cudaMemsetAsync(sort_aux_, 0, sort_zero_bytes((int64_t)cap_), stream_));
         }
-        if (outside) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
+        if (hst_->flags & FLAG_OUT_OF_DOMAIN) return fail(ZR_ERR_OUT_OF_DOMAIN_, "a particle lies outside its scene's domain");
         return 0;
     }
 

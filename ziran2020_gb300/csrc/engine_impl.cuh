@@ -294,14 +294,32 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t* B, int tiles, uint
 }
 
 // After a state write: would a bucket of the next substep's sort hold more movers than its slots? Its movers counted by bucket
-// (b_cnt, which the host clears again) with the keys, the base and the tiles that k_sort_tiles will see.
+// (b_cnt, which the host clears again) with the keys, the base and the tiles that k_sort_tiles will see. Launched behind k_keys,
+// whose count of movers says whether there is a question (sort_counted), so that both answers come back with one copy. One
+// atomic per bucket and warp: neighbours in storage mostly go to one bucket.
+template <int PER>
+__host__ __device__ __forceinline__ bool sort_counted(int64_t movers, int64_t n) { return movers > SortTile<PER>::MAXM && 4 * movers <= n; }
 template <int PER>
 __global__ void __launch_bounds__(SORT_NT) k_sort_probe(const uint32_t* knew, const uint32_t* kold, SortBufs sb, DevStatus* st)
 {
-    for (int64_t i = blockIdx.x * (int64_t)SORT_NT + threadIdx.x; i < sb.n; i += (int64_t)gridDim.x * SORT_NT) {
-        const uint32_t k = knew[i];
-        if (k == kold[i]) continue;
-        if (atomicAdd(&sb.b_cnt[bucket_of(sb.t_first, sb.tiles, k)], 1u) == (uint32_t)SortTile<PER>::MAXM) st->full_bucket = 1;
+    constexpr uint32_t MAXM = SortTile<PER>::MAXM;
+    __shared__ uint32_t s_first[SORT_FIRST];
+    if (!sort_counted<PER>(st->max_movers, sb.n)) return;
+    const int T = sb.tiles, lane = threadIdx.x & 31;
+    if (T <= SORT_FIRST)
+        for (int q = threadIdx.x; q < T; q += SORT_NT) s_first[q] = sb.t_first[q];
+    __syncthreads();
+    const uint32_t* B = T <= SORT_FIRST ? s_first : sb.t_first;
+    for (int64_t i0 = blockIdx.x * (int64_t)SORT_NT + (threadIdx.x & ~31); i0 < sb.n; i0 += (int64_t)gridDim.x * SORT_NT) {
+        const int64_t i = i0 + lane;
+        const uint32_t k = i < sb.n ? knew[i] : 0u;
+        const bool move = i < sb.n && k != kold[i];
+        if (!__any_sync(0xffffffffu, move)) continue;
+        const uint32_t b = move ? bucket_of(B, T, k) : SORT_NOKEY;
+        const unsigned same = __match_any_sync(0xffffffffu, b);
+        if (!move || lane != __ffs(same) - 1) continue;
+        const uint32_t add = (uint32_t)__popc(same);
+        if (atomicAdd(&sb.b_cnt[b], add) + add > MAXM) st->full_bucket = 1;
     }
 }
 
