@@ -683,8 +683,8 @@ def run_ours(args, world, rank):
     cfg["particle_groups"] = int(groups)
     cfg["schedule"] = schedule
     if over.get("implicit_damage"):
-        # the CG loop runs as a conditional node of the substep graph: 5 kernels per iteration, not counted in
-        # kernels_per_substep; the phase "grid" includes the whole damage solve
+        # the solve's first iteration is part of kernels_per_substep; further ones run in a conditional node of the substep
+        # graph, 3 kernels each, not counted there; the phase "grid" includes the whole damage solve
         cfg["damage_solve"] = {"cg_iterations_last_substep": cg_iterations, "kernels_per_cg_iteration": 3}
     line = {"metric": "particle-substeps/sec", "value": value, "unit": "particle-substeps/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

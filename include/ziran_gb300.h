@@ -204,7 +204,8 @@ int zr_scene_get_timing(zr_scene* s, double out5[5], int64_t* steps);
  * counterpart: Ziran's CPU loops are scheduled by TBB (MpmSimulationBase.cpp:669-855, 1269-1515).
  * mode 0 = a fixed default schedule, 1 = autotuned: measured with trial substeps on the scene's own state
  * when it first steps (the trials are rolled back) and cached per workload class in the process,
- * 2 = autotuned, re-measured per batch. Schedules differ only in the order of floating-point sums.
+ * 2 = autotuned, re-measured per batch. The trials want the particles in the order a substep leaves: a call that
+ * sets the state and steps once, or a job of zr_scene_step_stream, takes a cached choice or the default. Schedules differ only in the order of floating-point sums.
  * get: out7 = fused, chunk, buffers, CTAs per SM, G2P threads, G2P register cut, 1 if measured.
  * set: in6 = fused (0 split, 1 fused, 2 fused with registers cut for one more CTA per SM),
  * (chunk, buffers) one of (512, 1), (512, 2), (256, 2) in FP32 or (256, 1), (256, 2), (128, 2) in FP64

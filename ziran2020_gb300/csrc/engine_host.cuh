@@ -472,8 +472,8 @@ public:
         return rekey();
     }
 
-    // Pipelined jobs. Job 0 runs the safe way (set_state, step, get_state: it tunes the schedule, builds the one-substep
-    // graphs and leaves a valid sort base). Jobs 1.. run without a host check between them: input i is copied host ->
+    // Pipelined jobs. Job 0 runs the safe way (set_state, step, get_state: it builds the one-substep graphs and leaves a valid
+    // sort base; it takes a cached schedule, but its one substep leaves none over for trials). Jobs 1.. run without a host check between them: input i is copied host ->
     // device (copy engine, stream h2d_) into one of two device slots two jobs ahead, imported by a kernel, keyed, stepped
     // by the one-substep graph, exported into one of two output slots and copied device -> host (stream d2h_) while the
     // next jobs compute. The status is read once at the end; the status flags accumulate, so after the first aborted
@@ -1309,8 +1309,9 @@ private:
         return std::min<uint32_t>(P2G_CHUNK<T>, std::max<uint32_t>(least, even));
     }
 
-    // Enqueue one substep reading buffer `parity`. With ev != nullptr, events are recorded between the
-    // phases (sort | group heads, activate, neighbour slots | p2g | grid | g2p+end).
+    // Enqueue one substep reading buffer `parity`. With ev != nullptr, events are recorded between the phases (sort, groups,
+    // items and activation | neighbour slots, for the P2G forms that read them | p2g | grid with the damage solve | g2p); a full
+    // sort's group heads and activation count to the second.
     int enqueue_step(int parity, cudaEvent_t* ev, bool full_sort = false)
     {
         StepArgs<T> a = args(parity);
@@ -1380,7 +1381,8 @@ private:
 
     // Implicit damage solve of the substep (AnisoFractureSimulation.h:437-626): D~ history, coefficients, right-hand side
     // and preconditioner sums, CG initialisation, the first iteration, a conditional loop with the others, the nodal change
-    // for G2P. Every solve runs one iteration (r.z is only below the tolerance at the start where it is zero); more are rare.
+    // for G2P. A scene whose
+    // residual starts at or below 1e-6 is done before the first iteration (CG_INIT); the others rarely need a second one.
     int enqueue_damage_solve(const StepArgs<T>& a)
     {
         const int ng = cg_ctas();

@@ -8,14 +8,14 @@
 //   2. groups    the sorted range of every (scene, SPGrid page)
 //   3. activate  every group inserts its page and the 7 pages at +1 block into a hash table; new
 //                entries get a grid slot (MpmGrid::pollute, MpmGrid.h:153-193); in one kernel with the merge
-//   4. p2g       one CTA per group: stress V0*tau(F, g(d)) + APIC scatter of m, m v + m C (x_i - x_p),
+//   4. p2g       one CTA per work item (a group, or a piece of a large one): stress V0*tau(F, g(d)) + APIC scatter of m, m v + m C (x_i - x_p),
 //                -V0 tau grad w and the phase-field pair (d w, w) into a shared node tile, then
 //                vector atomics into the 8 neighbouring grid blocks (MpmSimulationBase.cpp:669-855,
 //                FBasedMpmForceHelper.cpp:43-63, AnisoFractureSimulation.h:161-176)
 //   5. grid      v = m v / m, v += g dt + f dt / m, half-space BCs, phase field normalised; clears the
 //                accumulators and the hash table for the next substep (MpmSimulationBase.cpp:655-666,
 //                1179-1228, AnisoFractureSimulation.h:177-179)
-//   6. g2p       one CTA per group: gather v, C (APIC/RPIC blend), grad v and the damage Laplacian,
+//   6. g2p       one CTA per work item: gather v, C (APIC/RPIC blend), grad v and the damage Laplacian,
 //                damage update with the old F, F <- (I + dt grad v) F, x += dt v, CFL / finiteness /
 //                domain checks, next key; writes the particle to its sorted slot of the other buffer
 //                (MpmSimulationBase.cpp:1269-1515, FBasedMpmForceHelper.cpp:95-108,
@@ -236,8 +236,8 @@ struct GroupHead {
 // particles whose cell did not change ("stayers") are already sorted; only the particles that changed cell
 // ("movers", ~2% per substep at the slab's speeds) need placing.
 //
-// Storage is cut into tiles (SortTile: 2,048 indices, or 512 in small scenes, see the host's sort_per). B[j] = the first old key of tile j (the old keys ascend with the
-// storage index). Mover key k belongs to bucket b(k) = the largest j with B[j] <= k (0 when there is none): every
+// Storage is cut into tiles (SortTile: 2,048 indices, or 512 in small scenes, see the host's sort_per). B[j] = the first old
+// key of tile j (the old keys ascend with the storage index). Mover key k belongs to bucket b(k) = the largest j with B[j] <= k (0 when there is none): every
 // element of bucket j (its movers) and tile j (its stayers) lies in [B[j], B[j+1]] and comes after every element of
 // lower tiles and buckets, so tile j's merged output starts at (stayers in tiles < j) + (movers in buckets < j). Inside
 // it, in the order (key, stayers first, storage index), a stayer goes to its rank among the tile's stayers plus the
@@ -258,7 +258,9 @@ struct GroupHead {
 // a third kernel behind the merge, for the head counts of the lower tiles): as five nodes (a memset
 // and four kernels) the substep took 57.0 us on 32,768 particles and 125.6 us on 425,984, with two 49.3 and 118.8 us.
 //
-// A bucket larger than its slots (SortTile::MAXM) raises FLAG_SORT: the host repeats the substep with a full radix sort.
+// A bucket larger than its slots (SortTile::MAXM) raises FLAG_SORT: the host repeats the substep with a full radix sort, and sorts
+// in full for longer each time that the sort behind it overflows again (SortBackoff). After a state write k_sort_probe tells
+// beforehand.
 // ---------------------------------------------------------------------------------------------------
 constexpr int SORT_NT = 256, SORT_PER = 8, SORT_TILE = SORT_NT * SORT_PER; // the group-head pass, and tiles of large scenes
 template <int PER>
@@ -864,7 +866,7 @@ __global__ void k_nbr(StepArgs<T> a)
 // directly (m v + dt f), which the grid update turns into v + f dt/m + g dt as the reference's
 // gridVelocityExplicitUpdate does (MpmSimulationBase.cpp:1197-1226).
 //
-// k_scatter (CTA per group, persistent): a producer warp streams each chunk of a group's payload from
+// k_scatter (a CTA per work item, persistent): a producer warp streams each chunk of an item's payload from
 // HBM into shared memory with bulk asynchronous copies (double-buffered, mbarrier-synchronised); the
 // consumer threads, one per (cell, stencil x-offset), accumulate the 9 nodes x 6 fields of their cell's
 // particles in registers (all particles of a cell share the same 27 nodes), add them into a shared
@@ -2742,7 +2744,7 @@ __global__ void __launch_bounds__(DmgShape<T>::NT, DmgShape<T>::MINB) k_dmg_rhs(
 {
     using L = typename LayoutOf<T>::type;
     using D = DmgShape<T>;
-    constexpr int NC = L::nodes, NT = D::NT, CHUNK = D::CHUNK, TY = L::sy + 2, TZ = L::sz + 2, TN = (L::sx + 2) * TY * TZ;
+    constexpr int NC = L::nodes, NT = D::NT, CHUNK = D::CHUNK;
     constexpr int TE = 3 * 3 * OffsetTiles<L>::TS; // per-offset tiles of the 3 node vectors
     __shared__ T tile[TE];
     __shared__ T st[D::NS][CHUNK]; // fr x3, vol D~ dt/eta, vol, c
