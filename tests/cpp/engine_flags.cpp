@@ -1,5 +1,5 @@
 // Scenes that reach (or must not reach) the incremental sort's overflow, run through the engine interface, which reports the
-// substeps' flags. Prints "name value" pairs for the Python test. Each run is compared with one that sorts in full (ZR_SORT=full):
+// substeps' flags, and checkpoints, which it takes. Prints "name value" pairs for the Python test. Each run is compared with one that sorts in full (ZR_SORT=full):
 // the two give the same particle order, so they differ by the order of grid sums alone.
 #include "../../ziran2020_gb300/csrc/engine.h"
 
@@ -147,6 +147,39 @@ int main(int argc, char** argv)
         }
         std::printf("particles %lld overflow %d difference %.3e groups %u full_groups %u blocks %u full_blocks %u\n", (long long)d.n,
             (r[0].flags & SORT_OVERFLOW) != 0, difference(out[0], out[1], d), r[0].n_groups, r[1].n_groups, r[0].n_blocks, r[1].n_blocks);
+        return 0;
+    }
+    if (mode == "restore") { // a checkpoint of a written state, before its damage drives were formed: a run, the checkpoint, the run again
+        SceneDesc d = box(8, 8, 8, 64, 20, 0.0);
+        d.implicit_damage = 1;
+        auto& m = d.materials[0];
+        m.model = 1;
+        m.E = 5e4;
+        m.nu = 0.25;
+        m.damage = 1;
+        m.alpha = -1;
+        m.l0 = 0.5 * d.dx;
+        m.eta = 0.1;
+        m.residual = 0.01;
+        d.sigma_c.assign(d.n, 100.0);
+        d.F.resize(9 * d.n);
+        for (int64_t p = 0; p < d.n; p++)
+            for (int c = 0; c < 9; c++) d.F[9 * p + c] = c == 0 ? 1.05 : (c % 4 ? 0.0 : 1.0);
+        auto e = engine(precision, d, false);
+        std::vector<double> first(25 * d.n), again(25 * d.n);
+        StepReport r;
+        must(e->checkpoint_save(), *e);
+        must(e->step(4, &r), *e);
+        must(e->get_state(0, first.data(), 0), *e);
+        must(e->checkpoint_restore(), *e);
+        must(e->step(4, &r), *e);
+        must(e->get_state(0, again.data(), 0), *e);
+        double damage = 0, m2 = 0;
+        for (int64_t p = 0; p < d.n; p++) {
+            damage = std::max(damage, first[25 * p + 24]);
+            m2 = std::max(m2, std::fabs(first[25 * p + 24] - again[25 * p + 24]));
+        }
+        std::printf("particles %lld damage %.6f difference %.3e\n", (long long)d.n, damage, m2);
         return 0;
     }
     if (mode == "stream") { // pipelined one-substep jobs, some of whose states would overflow a bucket of the job before

@@ -646,6 +646,7 @@ public:
         ZR_CUDA(cudaMemcpyAsync(ck_scenes_, d_scenes_, sc_b, cudaMemcpyDeviceToDevice, stream_));
         ZR_CUDA(cudaStreamSynchronize(stream_));
         ck_host_scenes_ = h_scenes_;
+        ck_drive_stale_ = drive_stale_; // the saved drives (P_DRV) are as fresh as the current ones
         ck_valid_ = true;
         return 0;
     }
@@ -685,6 +686,7 @@ public:
         ZR_CUDA(cudaMemcpyAsync(pid_[cur_], ck_pid_, pid_b, cudaMemcpyDeviceToDevice, stream_));
         ZR_CUDA(cudaMemcpyAsync(d_scenes_, ck_scenes_, sc_b, cudaMemcpyDeviceToDevice, stream_));
         h_scenes_ = ck_host_scenes_;
+        drive_stale_ = ck_drive_stale_;
         // a clean grid and the keys of the restored positions
         ZR_CUDA(clean_substep());
         return rekey();
@@ -877,7 +879,7 @@ private:
     void *ck_pool_ = nullptr, *ck_pid_ = nullptr, *ck_scenes_ = nullptr; // device checkpoint
     uint64_t ck_cap_ = 0;
     size_t ck_scenes_n_ = 0;
-    bool ck_valid_ = false;
+    bool ck_valid_ = false, ck_drive_stale_ = true;
     std::vector<SceneParams<T>> ck_host_scenes_;
     void* scenes_backup_ = nullptr;
     size_t scenes_backup_bytes_ = 0;
