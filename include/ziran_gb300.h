@@ -210,7 +210,9 @@ int zr_scene_get_timing(zr_scene* s, double out5[5], int64_t* steps);
  * set: in6 = fused (0 split, 1 fused, 2 fused with registers cut for one more CTA per SM),
  * (chunk, buffers) one of (512, 1), (512, 2), (256, 2) in FP32 or (256, 1), (256, 2), (128, 2) in FP64
  * (ignored when fused), CTAs per SM, G2P threads (64, 128 or 256), G2P register cut (0 or 1: more
- * resident threads per SM); an explicit schedule disables the autotuner for the scene. */
+ * resident threads per SM); an explicit schedule disables the autotuner for the scene. In FP64 a split form gets
+ * its payload buffer (369 B a particle) in this call, or with the scene when set before its first use; without
+ * room for it the call returns ZR_ERR_CUDA and the schedule stays as it was. */
 int zr_scene_set_autotune(zr_scene* s, int mode);
 int zr_scene_set_schedule(zr_scene* s, const int32_t in6[6]);
 int zr_scene_get_schedule(zr_scene* s, int32_t out7[7]);
