@@ -1144,6 +1144,7 @@ private:
         cudaError_t e = cudaMalloc(p, bytes);
         if (e != cudaSuccess) {
             *p = nullptr;
+            cudaGetLastError(); // reported here: a later launch check is not to find it
             err_ = std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e);
             return ZR_ERR_CUDA_;
         }
@@ -1765,37 +1766,27 @@ private:
     static bool reads_payload(const Schedule& sc) { return sc.fused == 0 || sc.fused == 3; }
     // the implicit damage solve's scratch, or the payload of a schedule that reads it
     static size_t payload_fields(const Schedule& sc) { return SPLIT_TRIED || reads_payload(sc) ? Pay<T>::N : DS_NF; }
-    // room for so many payload fields; the buffer is kept where it is large enough
-    int ensure_payload(size_t fields)
+    // room for so many payload fields; the buffer is kept where it is large enough, and where there is no memory for another
+    int ensure_payload(size_t fields) { return !cap_ || pay_fields_ >= fields ? 0 : replace_payload(fields); }
+    int replace_payload(size_t fields)
     {
-        if (!cap_ || pay_fields_ >= fields) return 0;
-        T* grown = nullptr;
+        T* fresh = nullptr;
         const size_t bytes = sizeof(T) * fields * (size_t)pstride_;
-        if (alloc((void**)&grown, bytes)) return ZR_ERR_CUDA_;
-        ZR_CUDA(cudaMemsetAsync(grown, 0, bytes, stream_));
+        if (alloc((void**)&fresh, bytes)) return ZR_ERR_CUDA_;
         drop_graphs();
         dfree(pay_); // (waits for what is in flight)
-        pay_ = grown;
+        pay_ = fresh;
         pay_fields_ = fields;
+        ZR_CUDA(cudaMemsetAsync(pay_, 0, bytes, stream_));
         return 0;
-    }
-
-    // gives back a payload buffer that only trials needed
-    int trim_payload()
-    {
-        const size_t fields = payload_fields(sched_);
-        if (pay_fields_ <= fields) return 0;
-        drop_graphs();
-        dfree(pay_);
-        pay_fields_ = 0;
-        return ensure_payload(fields);
     }
     // a measured schedule; the default one where there is no room for its payload
     int adopt(const Schedule& sc)
     {
         sched_ = ensure_payload(payload_fields(sc)) ? default_schedule() : sc;
         drop_graphs();
-        return trim_payload();
+        if (pay_fields_ > payload_fields(sched_)) replace_payload(payload_fields(sched_)); // a buffer that only trials needed
+        return 0;
     }
 
     int autotune_trials()
