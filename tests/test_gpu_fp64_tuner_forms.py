@@ -37,7 +37,7 @@ def payload_bytes(n):
 
 @pytest.mark.parametrize("mode", [1, 2])
 def test_the_form_follows_the_density(mode):
-    sparse, dense = lattice(40, 1), lattice(14, 27)  # 64,000 and 74,088 particles: one size class
+    sparse, dense = lattice(41, 1), lattice(14, 27)  # 68,921 and 74,088 particles: one size class (17 bits)
     a, b = run(sparse, mode), run(dense, mode)
     fixed_a, fixed_b = run(sparse, 0), run(dense, 0)
     assert a.schedule()["tuned"] and a.schedule()["fused"] == 0
@@ -46,6 +46,6 @@ def test_the_form_follows_the_density(mode):
         e = scenes.errors(scenes.gpu_state(s), scenes.gpu_state(f))
         assert e["x"][0] < 1e-12 and e["v"][0] < 1e-9, e
     held = lambda s, f: s.stats()["device_bytes"] - f.stats()["device_bytes"]
-    assert payload_bytes(64000) <= held(a, fixed_a) < payload_bytes(64000) + 65536  # (the trials' copy of the scene parameters)
+    assert payload_bytes(a.count) <= held(a, fixed_a) < payload_bytes(a.count) + 65536  # (the trials' copy of the scene parameters)
     assert 0 <= held(b, fixed_b) < 65536
     assert run(sparse, mode).schedule()["fused"] == 0  # mode 1: from the cache, with its payload
